@@ -6,13 +6,17 @@
 
 namespace lgb {
 
-#define LGB_COL_SIZES(X) \
-  X(48) X(64) X(128) X(256) X(288) X(512) X(576) X(1024) X(2048) X(2880) X(3072) X(3840) X(4096) X(5760)
+#define LGB_COL_TAB_SIZES(X) X(48) X(128)
 
 bool supported_col(int H) {
   switch (H) {
+    case 64:
+    case 256:
+    case 288:
+    case 512:
 #define X(n) case n:
-    LGB_COL_SIZES(X)
+    LGB_COL_TAB_SIZES(X)
+    LGB_COL_REG_SIZES(X)
 #undef X
     return true;
     default:
@@ -89,8 +93,6 @@ int launch_colpass(int H, const void* A, const void* Ip, int h, int Wcp, int n_c
   if (cpi < 1 || y_rows < 1 || y_rows > H || Wcp % kColGroup) return LGB_ERR_INVALID_ARGUMENT;
   if (norm && (H != 288 || norm_w < 2 || norm_w / 2 + 1 > Wcp || norm_stride < 1)) return LGB_ERR_UNSUPPORTED_SIZE;
   switch (H) {
-    case 4096:
-      return colpass_fused_t<16, 3>(A, Ip, h, Wcp, n_c, cpi, y_rows, waves, Y, s);
     case 512:
       return colpass_fused_t<8, 3>(A, Ip, h, Wcp, n_c, cpi, y_rows, waves, Y, s);
     case 256:
@@ -99,14 +101,15 @@ int launch_colpass(int H, const void* A, const void* Ip, int h, int Wcp, int n_c
       return colpass_fused_t<8, 2>(A, Ip, h, Wcp, n_c, cpi, y_rows, waves, Y, s);
     case 288:
       return colpass_pair_t<16, 18>(A, Ip, h, Wcp, n_c, cpi, y_rows, waves, Y, s, norm, norm_stride, norm_w);
-    default:
-      break;
-  }
-  switch (H) {
+#define X(n) \
+  case n:    \
+    return launch_colpass_##n(A, Ip, h, Wcp, n_c, cpi, y_rows, waves, Y, s);
+    LGB_COL_REG_SIZES(X)
+#undef X
 #define X(n) \
   case n:    \
     return colpass_tab_t<n>(A, Ip, h, Wcp, n_c, cpi, y_rows, waves, Y, s);
-    LGB_COL_SIZES(X)
+    LGB_COL_TAB_SIZES(X)
 #undef X
     default:
       return LGB_ERR_UNSUPPORTED_SIZE;

@@ -1,6 +1,6 @@
 // Register-fused column and row passes of the plain FP32 search.
 //
-// colpass_fused_kernel<R, P>  (H = R^P, one butterfly per thread per pass)
+// colpass_fused_kernel<R, P>  (H = R^P = 64, 256, 512, one butterfly per thread per pass)
 //   The forward FFT's last Stockham pass leaves element j + q*H/R of the
 //   column in thread j, and the inverse FFT's first pass consumes exactly those
 //   elements in the same thread: forward-last -> cross power -> inverse-first
@@ -202,27 +202,24 @@ __global__ void __launch_bounds__(ColFused<R, P>::THREADS, 1)
 }
 
 // ---------------------------------------------------------------------------
-// Column pass for the mixed-radix lengths (those without a uniform R^P plan):
-// the generic Stockham schedule of Plan<HN> with the twiddles of every pass
+// Column pass for the short lengths without a uniform R^P plan: the generic
+// Stockham schedule of Plan<HN> with the twiddles of every pass
 // after the first read from one shared table (filled once per CTA) instead
 // of sincospif per butterfly.  The forward first pass is pruned to the h
-// non-zero inputs.  G columns per CTA (ColGroupOf).
+// non-zero inputs.  G columns per CTA.
 // ---------------------------------------------------------------------------
 template <int HN>
 struct ColTab {
   using RL = typename Plan<HN>::type;
   static constexpr int NT = FftThreads<HN>::value;
-  // 288 (the refinement crops, 18 threads per column): 8 columns per CTA and
-  // up to 4 CTAs per SM measured 3 % faster than 4 columns at one CTA
-  static constexpr int G = HN == 288 ? 8 : ColGroupOf<HN>::value;
-  static constexpr int MIN_BLOCKS = HN == 288 ? 4 : 1;
+  static constexpr int G = kColGroup;
   static constexpr int STRIDE = IdxPad16::pad(HN) + 4;
   static constexpr int TAB = TableSize<1, RL>::value;
   static constexpr size_t SMEM = sizeof(float2) * ((size_t)G * STRIDE + TAB);
 };
 
 template <int HN>
-__global__ void __launch_bounds__(ColTab<HN>::G* ColTab<HN>::NT, ColTab<HN>::MIN_BLOCKS)
+__global__ void __launch_bounds__(ColTab<HN>::G* ColTab<HN>::NT)
     colpass_tab_kernel(const float2* __restrict__ A, const float2* __restrict__ Ip, int h, int Wcp, int n_c,
                        int c_per_block, int c_per_image, int y_rows, float2* __restrict__ Y) {
   using CT = ColTab<HN>;

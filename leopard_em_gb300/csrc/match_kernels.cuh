@@ -11,7 +11,8 @@
 //                     and the zero-padded row rfft of length W          [n_c, d, Wcp]
 //   column pass       per column: pruned FFT along y (length H), cross power
 //                     image * conj(P) with P[0,0]=0, inverse FFT along y
-//                     (colpass_fused_kernel / colpass_tab_kernel)      [n_c, H, Wcp]
+//                     (colpass_reg_kernel and, for short columns,
+//                     colpass_fused / _tab / _pair_kernel)             [n_c, H, Wcp]
 //   rowpass_kernel    per row: c2r of length W (1/(H W)) and the fused
 //                     statistics update (utils.py:191-255): max over the
 //                     batch, strict '>' MIP update, global index, FP64 sums
@@ -669,13 +670,6 @@ __global__ void __launch_bounds__(ROWS* FftThreads<WH>::value, (PadRows<WH, ROWS
     __syncthreads();  // this pass's rows are read before the next ones are staged
   }
 }
-
-// Columns per colpass CTA: kColGroup, or 2 where four transforms of length HN
-// would need more than 1024 threads (HN = 5760).
-template <int HN>
-struct ColGroupOf {
-  static constexpr int value = kColGroup * FftThreads<HN>::value <= 1024 ? kColGroup : 2;
-};
 
 // ---------------------------------------------------------------------------
 // rowpass: row y of every correlogram in the batch: c2r of length W = 2*WH

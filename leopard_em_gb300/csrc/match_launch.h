@@ -45,6 +45,14 @@ int launch_pad_rfft(int W, const float* proj, const double* rowstats, int h, int
 int launch_colpass(int H, const void* A, const void* Ip, int h, int Wcp, int n_c, int c_per_image, int y_rows,
                    int waves, void* Y, cudaStream_t s, const float2* norm = nullptr, int norm_stride = 0,
                    int norm_w = 0);
+// Its lengths in two register passes (match_cols_reg.cuh), one translation unit
+// each so that they compile in parallel.
+#define LGB_COL_REG_SIZES(X) X(576) X(1024) X(2048) X(2880) X(3072) X(3840) X(4096) X(5760)
+#define X(n)                                                                                                  \
+  int launch_colpass_##n(const void* A, const void* Ip, int h, int Wcp, int n_c, int c_per_image, int y_rows, \
+                         int waves, void* Y, cudaStream_t s);
+LGB_COL_REG_SIZES(X)
+#undef X
 // Rows y < y_rows of the H x W correlograms (Y is [n_c][y_rows][Wcp]); global
 // index base o0 + *o0_dev (o0_dev may be null).
 int launch_rowpass(int W, const void* Y, int H, int y_rows, int Wcp, int n_c, int nb, int n_orient, int o0,

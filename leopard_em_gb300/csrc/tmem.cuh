@@ -1,0 +1,86 @@
+// Tensor memory as per-thread storage: a warp reaches its own quarter of the
+// 128 lanes, a thread its own lane, and a 32x32b access moves consecutive
+// 32-bit columns of that lane to or from the thread's registers.  Every lane of
+// the warp takes part.
+#pragma once
+
+#include "common.cuh"
+
+namespace lgb {
+
+__device__ __forceinline__ void tmem_alloc(unsigned* slot, unsigned columns) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(slot);
+  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s), "r"(columns) : "memory");
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc(unsigned base, unsigned columns) {
+  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(columns) : "memory");
+}
+// Orders the allocation (and the last accesses) with the CTA's barrier.
+__device__ __forceinline__ void tmem_barrier() {
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// N complex values, 2 N columns; a load is complete when its statement is.
+__device__ __forceinline__ void tmem_put2(unsigned addr, const float2* v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "f"(v[0].x), "f"(v[0].y), "f"(v[1].x), "f"(v[1].y)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_get2(unsigned addr, float2* v) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];\n tcgen05.wait::ld.sync.aligned;"
+               : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[1].x), "=f"(v[1].y)
+               : "r"(addr)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_put4(unsigned addr, const float2* v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(addr), "f"(v[0].x), "f"(v[0].y), "f"(v[1].x), "f"(v[1].y), "f"(v[2].x), "f"(v[2].y), "f"(v[3].x), "f"(v[3].y)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_get4(unsigned addr, float2* v) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n tcgen05.wait::ld.sync.aligned;"
+               : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[1].x), "=f"(v[1].y), "=f"(v[2].x), "=f"(v[2].y), "=f"(v[3].x), "=f"(v[3].y)
+               : "r"(addr)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_put8(unsigned addr, const float2* v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(addr), "f"(v[0].x), "f"(v[0].y), "f"(v[1].x), "f"(v[1].y), "f"(v[2].x), "f"(v[2].y), "f"(v[3].x), "f"(v[3].y), "f"(v[4].x), "f"(v[4].y), "f"(v[5].x), "f"(v[5].y), "f"(v[6].x), "f"(v[6].y), "f"(v[7].x), "f"(v[7].y)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_get8(unsigned addr, float2* v) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n tcgen05.wait::ld.sync.aligned;"
+               : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[1].x), "=f"(v[1].y), "=f"(v[2].x), "=f"(v[2].y), "=f"(v[3].x), "=f"(v[3].y), "=f"(v[4].x), "=f"(v[4].y), "=f"(v[5].x), "=f"(v[5].y), "=f"(v[6].x), "=f"(v[6].y), "=f"(v[7].x), "=f"(v[7].y)
+               : "r"(addr)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_put16(unsigned addr, const float2* v) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(addr), "f"(v[0].x), "f"(v[0].y), "f"(v[1].x), "f"(v[1].y), "f"(v[2].x), "f"(v[2].y), "f"(v[3].x), "f"(v[3].y), "f"(v[4].x), "f"(v[4].y), "f"(v[5].x), "f"(v[5].y), "f"(v[6].x), "f"(v[6].y), "f"(v[7].x), "f"(v[7].y), "f"(v[8].x), "f"(v[8].y), "f"(v[9].x), "f"(v[9].y), "f"(v[10].x), "f"(v[10].y), "f"(v[11].x), "f"(v[11].y), "f"(v[12].x), "f"(v[12].y), "f"(v[13].x), "f"(v[13].y), "f"(v[14].x), "f"(v[14].y), "f"(v[15].x), "f"(v[15].y)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_get16(unsigned addr, float2* v) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n tcgen05.wait::ld.sync.aligned;"
+               : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[1].x), "=f"(v[1].y), "=f"(v[2].x), "=f"(v[2].y), "=f"(v[3].x), "=f"(v[3].y), "=f"(v[4].x), "=f"(v[4].y), "=f"(v[5].x), "=f"(v[5].y), "=f"(v[6].x), "=f"(v[6].y), "=f"(v[7].x), "=f"(v[7].y), "=f"(v[8].x), "=f"(v[8].y), "=f"(v[9].x), "=f"(v[9].y), "=f"(v[10].x), "=f"(v[10].y), "=f"(v[11].x), "=f"(v[11].y), "=f"(v[12].x), "=f"(v[12].y), "=f"(v[13].x), "=f"(v[13].y), "=f"(v[14].x), "=f"(v[14].y), "=f"(v[15].x), "=f"(v[15].y)
+               : "r"(addr)
+               : "memory");
+}
+
+template <int N>
+__device__ __forceinline__ void tmem_put(unsigned addr, const float2* v) {
+  static_assert(N % 4 == 0, "multiples of four");
+#pragma unroll
+  for (int i = 0; i < N / 16; ++i) tmem_put16(addr + 32 * i, v + 16 * i);
+  if constexpr (N % 16 >= 8) tmem_put8(addr + 32 * (N / 16), v + 16 * (N / 16));
+  if constexpr (N % 8) tmem_put4(addr + 2 * (N - 4), v + N - 4);
+}
+template <int N>
+__device__ __forceinline__ void tmem_get(unsigned addr, float2* v) {
+  static_assert(N == 2 || N == 4 || N == 8 || N == 16, "one access");
+  if constexpr (N == 2) tmem_get2(addr, v);
+  if constexpr (N == 4) tmem_get4(addr, v);
+  if constexpr (N == 8) tmem_get8(addr, v);
+  if constexpr (N == 16) tmem_get16(addr, v);
+}
+
+}  // namespace lgb

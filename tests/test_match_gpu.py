@@ -223,3 +223,33 @@ def test_production_configuration_against_oracle():
     err_f32 = ((f32["mip"].double() - ref["mip"].double()).abs() / scale).max().item()
     print(f"MIP relative error vs FP64: CUDA path {err_gpu:.2e}, FP32 restatement {err_f32:.2e}")
     assert err_gpu < err_f32
+
+
+@pytest.mark.parametrize(
+    "H,W,d,n_df",
+    [
+        # the register column passes: every length, with few and many non-zero rows (the dense
+        # first pass where the template reaches it), and a cut micrograph on the padded grid
+        (576, 80, 48, 1), (576, 256, 256, 1), (1024, 64, 32, 1), (1024, 288, 288, 1), (2048, 64, 48, 2),
+        (2880, 48, 32, 1), (3072, 64, 64, 1), (3072, 512, 512, 1), (3840, 48, 48, 1), (3840, 512, 512, 1),
+        (4096, 64, 64, 3), (4090, 64, 32, 1), (5760, 48, 48, 1), (5701, 64, 64, 1),
+    ],
+)
+def test_register_column_pass_against_oracle(H, W, d, n_df):
+    kw = _small_workload(H, W, d, 16, n_df)
+    gpu = _gpu_search(kw, 5)
+    # 64-bit oracle: the 32-bit one's own rotations drift past the tolerance at 512
+    ref = orc.core_match_template_cpu(**kw, orientation_batch_size=5, track_second_best=True,
+                                      stat_dtype=torch.float64, compute_dtype=torch.float64, device="cuda:0")
+    if (H, W) != _padded(H, W):  # linear instead of circular beyond the valid positions
+        keys = [k for k, v in ref.items() if isinstance(v, torch.Tensor) and v.shape == (H, W)]
+        gpu["best_global_index"] = gpu["best_global_index"][:H, :W]
+        for r in (gpu, ref):
+            r.update({k: r[k][: H - d + 1, : W - d + 1] for k in keys if k in r})
+    _assert_parity(gpu, ref, second=ref["second_best"])
+
+
+def _padded(H, W):
+    from leopard_em_gb300.backend.core_match_template import padded_grid
+
+    return padded_grid(H, W)

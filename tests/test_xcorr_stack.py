@@ -73,3 +73,20 @@ def test_device_argument_errors():
         cross_correlate_particle_stack(ps, t, r[:2], f)
     with pytest.raises(ValueError):
         cross_correlate_particle_stack(ps, t, r, f, mag_matrix=torch.eye(2))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("H,W,d,mode", [(576, 80, 48, "same"), (1024, 64, 32, "valid"), (2048, 48, 48, "same")])
+def test_device_matches_oracle_register_column_lengths(H, W, d, mode):
+    """The register column passes with another image for each correlogram."""
+    from leopard_em_gb300.backend import cross_correlate_particle_stack
+
+    g = torch.Generator().manual_seed(H + d)
+    ps = torch.fft.rfft2(torch.randn((3, H, W), generator=g))
+    vol = torch.fft.fftshift(torch.fft.rfftn(torch.randn((d, d, d), generator=g)), dim=(0, 1))
+    rot = torch.linalg.qr(torch.randn((3, 3, 3), generator=g, dtype=torch.float64))[0].float()
+    rot *= torch.linalg.det(rot)[:, None, None].sign()
+    pf = torch.rand((3, d, d // 2 + 1), generator=g) + 0.5
+    got = cross_correlate_particle_stack(ps, vol, rot, pf, mode=mode)
+    ref = orr.cross_correlate_particle_stack_cpu(ps, vol, rot, pf, mode=mode)
+    _close(got.numpy(), ref.numpy())
