@@ -37,6 +37,17 @@ __device__ __forceinline__ float2 mul_i(float2 a) {
   return DIR > 0 ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
 }
 
+// ---- async copy helpers (16-byte cp.async, completion via wait_group) -------
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+
 // Status codes returned by every C-ABI entry point (see include/leopard_gb300.h).
 #define LGB_CUDA_TRY(expr)                                   \
   do {                                                       \

@@ -1,4 +1,4 @@
-// Register-fused column and row passes of the plain FP32 search.
+// Register-fused column passes of the plain FP32 search.
 //
 // colpass_fused_kernel<R, P>  (H = R^P = 64, 256, 512, one butterfly per thread per pass)
 //   The forward FFT's last Stockham pass leaves element j + q*H/R of the
@@ -11,32 +11,12 @@
 //   per-CTA shared table (built once with sincospif).  Thread layout: lane
 //   bits 0-1 select one of four adjacent columns, so each warp touches 8 rows
 //   x 32 B: whole sectors.
-//
-// rowpass_fused_kernel<WH, NT, Plan>  (W = 2*WH)
-//   The c2r pre-twiddle (X[k], conj X[WH-k] -> Z[k]) is applied while the
-//   first pass loads from the staged row; the last pass's outputs stay in
-//   registers and feed the statistics directly.  Rows are staged with
-//   cp.async double buffering (the next correlogram's row is in flight while
-//   the current one is transformed).  Waits are cp.async.wait_group: no spins.
 #pragma once
-
-#include <type_traits>
 
 #include "fft.cuh"
 #include "match_kernels.cuh"
 
 namespace lgb {
-
-// ---- async copy helpers (16-byte cp.async, completion via wait_group) -------
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
 
 // L2 placement: measured, neither an evict_last policy on the image-spectrum
 // loads nor streaming stores of the intermediate help -- both take L2 away
@@ -388,188 +368,6 @@ __global__ void __launch_bounds__(ColPair<R1, R2>::THREADS, 4)
       }
     }
     __syncthreads();  // before the next correlogram's pass-1 stores
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Fused row pass (c2r of length 2*WH + statistics).
-// ---------------------------------------------------------------------------
-template <int WH, int NT, class RL>
-struct RowFused {
-  static constexpr int R1 = Head<RL>::value;
-  static constexpr int RLAST = Last<RL>::value;
-  static constexpr int NB1 = WH / R1;
-  static constexpr int PER1 = (NB1 + NT - 1) / NT;
-  static constexpr int NBL = WH / RLAST;
-  static constexpr int PERL = NBL / NT;
-  // the 8, 8 middle passes of 2048 = 8 8 8 4 store / load through the 16x2 layout
-  static constexpr bool MID88 = std::is_same<typename Middle<RL>::type, Radices<8, 8>>::value;
-  static constexpr int ZS = (MID88 ? IdxPad16x2::pad(WH) : IdxPad16::pad(WH)) + 2;
-  static constexpr int TAB = TableSize<1, RL>::value;
-  static_assert(NBL % NT == 0, "last pass must give every thread whole butterflies");
-  static_assert(NB1 <= NT * PER1, "first pass coverage");
-  static_assert(16 % (2 * R1) == 0, "pre-twiddle roots exp(i pi q / R1) come from the 16th roots");
-  static size_t smem(int wcp) { return sizeof(float2) * (size_t)(2 * wcp + ZS + TAB); }
-};
-
-template <int WH, int NT, class RL, int MINB = 3>
-__global__ void __launch_bounds__(NT, MINB)
-    rowpass_fused_kernel(const float2* __restrict__ Y, int y_rows, int Wcp, int n_c, int nb, int n_orient, int o0,
-                         const int* __restrict__ o0_dev, float scale, float* __restrict__ mip,
-                         int* __restrict__ best, double* __restrict__ s1, double* __restrict__ s2) {
-  using RF = RowFused<WH, NT, RL>;
-  constexpr int R1 = RF::R1, RLAST = RF::RLAST, NB1 = RF::NB1, PER1 = RF::PER1, NBL = RF::NBL, PERL = RF::PERL;
-  constexpr int OUT = PERL * RLAST;  // complex outputs (pixel pairs) per thread
-  extern __shared__ float2 rsm[];
-  float2* xr0 = rsm;
-  float2* xr1 = rsm + Wcp;
-  float2* z = rsm + 2 * Wcp;
-  float2* tab = z + RF::ZS;
-  const int y = blockIdx.x;
-  const int t = threadIdx.x;
-  const int n16 = Wcp / 2;  // 16-byte chunks per row
-
-  // stage row 0 while the tables are built
-  {
-    const float2* src = Y + (size_t)y * Wcp;
-    for (int i = t; i < n16; i += NT) cp_async16(xr0 + 2 * i, src + 2 * i);
-    cp_async_commit();
-  }
-  FillTables<WH, 1, RL>::run(tab, t, NT);
-  // c2r pre-twiddle exp(+i pi k / WH) at k = j + q*NB1 factors into
-  // exp(+i pi j / WH) (per thread, kept in registers) x exp(+i pi q / R1)
-  float2 prej[PER1];
-#pragma unroll
-  for (int p = 0; p < PER1; ++p) {
-    float sn, cs;
-    sincospif((float)(t + p * NT) / (float)WH, &sn, &cs);
-    prej[p] = make_float2(cs, sn);
-  }
-  const float2* tab_last = tab + TableSize<1, typename DropLast<RL>::type>::value;
-
-  float bmax[2 * OUT], bs[2 * OUT], bss[2 * OUT];
-  unsigned barg[OUT];  // batch index of each pixel pair's maxima: low / high 16 bits
-#pragma unroll
-  for (int i = 0; i < 2 * OUT; ++i) {
-    bmax[i] = -INFINITY;
-    bs[i] = 0.f;
-    bss[i] = 0.f;
-  }
-#pragma unroll
-  for (int i = 0; i < OUT; ++i) barg[i] = 0u;
-
-#pragma unroll 1
-  for (int c = 0; c < n_c; ++c) {
-    const float2* xr = (c & 1) ? xr1 : xr0;
-    if (c + 1 < n_c) {
-      float2* nxt = (c & 1) ? xr0 : xr1;
-      const float2* src = Y + ((size_t)(c + 1) * y_rows + y) * Wcp;
-      for (int i = t; i < n16; i += NT) cp_async16(nxt + 2 * i, src + 2 * i);
-      cp_async_commit();
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    __syncthreads();
-    // ---- pass 1: pre-twiddle while loading, no twiddles (stride 1)
-    {
-      float2 v[PER1][R1];
-#pragma unroll
-      for (int p = 0; p < PER1; ++p) {
-        const int j = t + p * NT;
-        if ((NB1 % NT == 0) || j < NB1) {
-#pragma unroll
-          for (int q = 0; q < R1; ++q) {
-            const int k = j + q * NB1;
-            float2 a = xr[k];
-            float2 b = xr[WH - k];
-            if (k == 0) {
-              a.y = 0.f;
-              b.y = 0.f;
-            }
-            b.y = -b.y;
-            float2 xo = cmul(csub(a, b), prej[p]);
-            if (q) xo = cmulc(xo, kRootsFwd16[q * (16 / (2 * R1))]);
-            v[p][q] = cadd(cadd(a, b), mul_i<1>(xo));
-          }
-          Dft<R1, +1>::run(v[p]);
-        }
-      }
-#pragma unroll
-      for (int p = 0; p < PER1; ++p) {
-        const int j = t + p * NT;
-        if ((NB1 % NT == 0) || j < NB1) {
-#pragma unroll
-          for (int q = 0; q < R1; ++q) z[IdxPad16::f(j * R1 + q)] = v[p][q];
-        }
-      }
-    }
-    __syncthreads();
-    if constexpr (RF::MID88) {
-      // stride-8 radix-8 stores into the 16x2 layout, read back by the
-      // stride-64 pass, which stores the plain padded layout again
-      table_pass_io<WH, 8, R1, NT, +1, IdxPad16, IdxPad16x2>(z, tab, t);
-      table_pass_io<WH, 8, R1 * 8, NT, +1, IdxPad16x2, IdxPad16>(z, tab + R1 * 7, t);
-    } else {
-      TablePasses<WH, NT, +1, IdxPad16, R1, typename Middle<RL>::type>::run(z, tab, t);
-    }
-    // ---- last pass -> registers -> statistics
-#pragma unroll
-    for (int p = 0; p < PERL; ++p) {
-      const int j = t + p * NT;
-      float2 v[RLAST];
-#pragma unroll
-      for (int q = 0; q < RLAST; ++q) v[q] = z[IdxPad16::f(j + q * NBL)];
-      twiddle_from_table<RLAST, +1, NBL>(v, tab_last, j);
-      Dft<RLAST, +1>::run(v);
-#pragma unroll
-      for (int q = 0; q < RLAST; ++q) {
-        const int o = 2 * (p * RLAST + q);
-        const float a = v[q].x * scale, b = v[q].y * scale;
-        const int k = p * RLAST + q;
-        if (a > bmax[o]) { bmax[o] = a; barg[k] = (barg[k] & 0xffff0000u) | (unsigned)c; }
-        if (b > bmax[o + 1]) { bmax[o + 1] = b; barg[k] = (barg[k] & 0xffffu) | ((unsigned)c << 16); }
-        bs[o] += a;
-        bss[o] = fmaf(a, a, bss[o]);
-        bs[o + 1] += b;
-        bss[o + 1] = fmaf(b, b, bss[o + 1]);
-      }
-    }
-    __syncthreads();
-  }
-
-  const size_t W = 2 * (size_t)WH;
-  if (o0_dev) o0 += *o0_dev;
-#pragma unroll
-  for (int p = 0; p < PERL; ++p) {
-#pragma unroll
-    for (int q = 0; q < RLAST; ++q) {
-      const int o = 2 * (p * RLAST + q);
-      const int m = t + p * NT + q * NBL;
-      const size_t idx = (size_t)y * W + 2 * (size_t)m;
-      float2 mm = *reinterpret_cast<float2*>(mip + idx);
-      int2 bi = *reinterpret_cast<int2*>(best + idx);
-      double2 sa = *reinterpret_cast<double2*>(s1 + idx);
-      double2 sq = *reinterpret_cast<double2*>(s2 + idx);
-      if (bmax[o] > mm.x) {
-        mm.x = bmax[o];
-        const int cc = (int)(barg[p * RLAST + q] & 0xffffu);
-        bi.x = (cc / nb) * n_orient + o0 + (cc - (cc / nb) * nb);
-      }
-      if (bmax[o + 1] > mm.y) {
-        mm.y = bmax[o + 1];
-        const int cc = (int)(barg[p * RLAST + q] >> 16);
-        bi.y = (cc / nb) * n_orient + o0 + (cc - (cc / nb) * nb);
-      }
-      sa.x += f2d_bits(bs[o]);
-      sa.y += f2d_bits(bs[o + 1]);
-      sq.x += f2d_bits(bss[o]);
-      sq.y += f2d_bits(bss[o + 1]);
-      *reinterpret_cast<float2*>(mip + idx) = mm;
-      *reinterpret_cast<int2*>(best + idx) = bi;
-      *reinterpret_cast<double2*>(s1 + idx) = sa;
-      *reinterpret_cast<double2*>(s2 + idx) = sq;
-    }
   }
 }
 

@@ -13,7 +13,8 @@
 //                     image * conj(P) with P[0,0]=0, inverse FFT along y
 //                     (colpass_reg_kernel and, for short columns,
 //                     colpass_fused / _tab / _pair_kernel)             [n_c, H, Wcp]
-//   rowpass_kernel    per row: c2r of length W (1/(H W)) and the fused
+//   row pass          per row: c2r of length W (1/(H W)) and the fused
+//                     (rowpass_half_kernel, short rows rowpass_kernel)
 //                     statistics update (utils.py:191-255): max over the
 //                     batch, strict '>' MIP update, global index, FP64 sums
 // Two-register-pass forms for the refinement crops (288^2, d = 256):

@@ -57,6 +57,13 @@ LGB_COL_REG_SIZES(X)
 // index base o0 + *o0_dev (o0_dev may be null).
 int launch_rowpass(int W, const void* Y, int H, int y_rows, int Wcp, int n_c, int nb, int n_orient, int o0,
                    const int* o0_dev, float* mip, int* best, double* s1, double* s2, cudaStream_t s);
+// Its long rows (match_rows_half.cuh).
+#define LGB_ROW_HALF_SIZES(X) X(512) X(1024) X(2048) X(2880) X(3072) X(3840) X(4096) X(5760)
+#define X(n)                                                                                                \
+  int launch_rowpass_##n(const void* Y, int H, int y_rows, int Wcp, int n_c, int nb, int n_orient, int o0,  \
+                         const int* o0_dev, float* mip, int* best, double* s1, double* s2, cudaStream_t s);
+LGB_ROW_HALF_SIZES(X)
+#undef X
 
 // Every argument check of lgb_match_search except the workspace; LGB_OK or
 // the status lgb_match_search would return.  Runs no GPU work.

@@ -1,6 +1,5 @@
 // Launchers: zero-padded projection rfft and the row c2r + statistics pass
 // (image width W).
-#include "match_fused.cuh"
 #include "match_kernels.cuh"
 #include "match_launch.h"
 
@@ -25,6 +24,9 @@ int launch_norm_constants(double* rowstats, int n_c, int h, int norm_h, int norm
   return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
 }
 
+
+// W/2 of the short rows, which the generic row pass takes
+#define LGB_ROW_GENERIC_SIZES(X) X(24) X(32) X(40) X(64) X(128) X(144) X(288)
 
 // W/2 values
 #define LGB_ROW_SIZES(X) \
@@ -110,48 +112,19 @@ int launch_pad_rfft(int W, const float* proj, const double* rowstats, int h, int
   }
 }
 
-template <int WH, int NT, class RL, int MINB = 3>
-static int rowpass_fused_t(const void* Y, int H, int y_rows, int Wcp, int n_c, int nb, int n_orient, int o0,
-                           const int* o0_dev, float* mip, int* best, double* s1, double* s2, cudaStream_t s) {
-  using RF = RowFused<WH, NT, RL>;
-  if (n_c > 0xffff) return LGB_ERR_INVALID_ARGUMENT;  // batch indices are kept in 16 bits
-  const size_t smem = RF::smem(Wcp);
-  if (cudaFuncSetAttribute(rowpass_fused_kernel<WH, NT, RL, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem) != cudaSuccess ||
-      cudaFuncSetAttribute(rowpass_fused_kernel<WH, NT, RL, MINB>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                           cudaSharedmemCarveoutMaxShared) != cudaSuccess)
-    return LGB_ERR_CUDA;
-  const float scale = 1.0f / ((float)H * (float)(2 * WH));
-  rowpass_fused_kernel<WH, NT, RL, MINB><<<y_rows, NT, smem, s>>>(static_cast<const float2*>(Y), y_rows, Wcp, n_c, nb,
-                                                            n_orient, o0, o0_dev, scale, mip, best, s1, s2);
-  return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
-}
-
 int launch_rowpass(int W, const void* Y, int H, int y_rows, int Wcp, int n_c, int nb, int n_orient, int o0,
                    const int* o0_dev, float* mip, int* best, double* s1, double* s2, cudaStream_t s) {
   if (W % 2 || y_rows < 1 || y_rows > H) return LGB_ERR_INVALID_ARGUMENT;
   switch (W / 2) {
-    case 2048:
-      return rowpass_fused_t<2048, 256, Radices<8, 8, 8, 4>>(Y, H, y_rows, Wcp, n_c, nb, n_orient, o0, o0_dev, mip,
-                                                             best, s1, s2, s);
-    case 2880:  // 5760-wide grids (e.g. a 5760 x 4092 micrograph searched transposed): one CTA per SM at
-                // 157 registers without spills (two CTAs at 80 registers spill 324 B and run 9 % slower)
-      return rowpass_fused_t<2880, 360, Radices<8, 9, 5, 8>, 1>(Y, H, y_rows, Wcp, n_c, nb, n_orient, o0, o0_dev,
-                                                                mip, best, s1, s2, s);
-    case 1024:
-      return rowpass_fused_t<1024, 256, Radices<8, 8, 4, 4>>(Y, H, y_rows, Wcp, n_c, nb, n_orient, o0, o0_dev, mip,
-                                                             best, s1, s2, s);
-    case 256:
-      return rowpass_fused_t<256, 64, Radices<8, 8, 4>>(Y, H, y_rows, Wcp, n_c, nb, n_orient, o0, o0_dev, mip, best,
-                                                        s1, s2, s);
-    default:
-      break;
-  }
-  switch (W / 2) {
+#define X(n)        \
+  case n / 2:       \
+    return launch_rowpass_##n(Y, H, y_rows, Wcp, n_c, nb, n_orient, o0, o0_dev, mip, best, s1, s2, s);
+    LGB_ROW_HALF_SIZES(X)
+#undef X
 #define X(n) \
   case n:    \
     return rowpass_t<n>(Y, H, y_rows, Wcp, n_c, nb, n_orient, o0, o0_dev, mip, best, s1, s2, s);
-    LGB_ROW_SIZES(X)
+    LGB_ROW_GENERIC_SIZES(X)
 #undef X
     default:
       return LGB_ERR_UNSUPPORTED_SIZE;

@@ -110,6 +110,48 @@ struct Dft<15, DIR> {
   }
 };
 
+// Prime-factor 2 x 5: input n = (5 n1 + 2 n2) mod 10, output k = (5 k1 + 6 k2) mod 10.
+template <int DIR>
+struct Dft<10, DIR> {
+  static __device__ __forceinline__ void run(float2* v) {
+    float2 a[5], b[5];
+#pragma unroll
+    for (int n2 = 0; n2 < 5; ++n2) {
+      const float2 x0 = v[(2 * n2) % 10], x1 = v[(5 + 2 * n2) % 10];
+      a[n2] = cadd(x0, x1);
+      b[n2] = csub(x0, x1);
+    }
+    Dft<5, DIR>::run(a);
+    Dft<5, DIR>::run(b);
+#pragma unroll
+    for (int k2 = 0; k2 < 5; ++k2) {
+      v[(6 * k2) % 10] = a[k2];
+      v[(5 + 6 * k2) % 10] = b[k2];
+    }
+  }
+};
+
+// Prime-factor 3 x 4: input n = (4 n1 + 3 n2) mod 12, output k = (4 k1 + 9 k2) mod 12.
+template <int DIR>
+struct Dft<12, DIR> {
+  static __device__ __forceinline__ void run(float2* v) {
+    float2 u[3][4];
+#pragma unroll
+    for (int n1 = 0; n1 < 3; ++n1) {
+#pragma unroll
+      for (int n2 = 0; n2 < 4; ++n2) u[n1][n2] = v[(4 * n1 + 3 * n2) % 12];
+      Dft<4, DIR>::run(u[n1]);
+    }
+#pragma unroll
+    for (int k2 = 0; k2 < 4; ++k2) {
+      float2 t[3] = {u[0][k2], u[1][k2], u[2][k2]};
+      Dft<3, DIR>::run(t);
+#pragma unroll
+      for (int k1 = 0; k1 < 3; ++k1) v[(4 * k1 + 9 * k2) % 12] = t[k1];
+    }
+  }
+};
+
 // ---- composite DFT of RA * RB points -----------------------------------------
 // RA-point transforms over qa, roots w^(qb ra), RB-point transforms over qb;
 // output r = ra + RA rb.  NT: input q = qa RB + qb in slot q, output r in slot

@@ -253,3 +253,36 @@ def _padded(H, W):
     from leopard_em_gb300.backend.core_match_template import padded_grid
 
     return padded_grid(H, W)
+
+
+@pytest.mark.parametrize("W", [512, 1024, 2048, 2880, 3072, 3840, 4096, 5760])
+@pytest.mark.parametrize("H,n_o,batch,n_df", [(48, 15, 5, 1), (64, 16, 1, 1), (61, 8, 4, 3)])
+def test_long_row_pass_against_oracle(W, H, n_o, batch, n_df):
+    """Row passes of every long length: several rows per CTA, single correlograms, a cut micrograph height."""
+    kw = _small_workload(H, W, 32, n_o, n_df)
+    gpu = _gpu_search(kw, batch)
+    ref = orc.core_match_template_cpu(**kw, orientation_batch_size=batch, track_second_best=True,
+                                      stat_dtype=torch.float64, compute_dtype=torch.float64, device="cuda:0")
+    if (H, W) != _padded(H, W):
+        keys = [k for k, v in ref.items() if isinstance(v, torch.Tensor) and v.shape == (H, W)]
+        gpu["best_global_index"] = gpu["best_global_index"][:H, :W]
+        for r in (gpu, ref):
+            r.update({k: r[k][: H - 31, : W - 31] for k in keys if k in r})
+    _assert_parity(gpu, ref, second=ref["second_best"])
+
+
+@pytest.mark.parametrize("W", [512, 4096])
+def test_not_finite_correlograms_stay_apart(W):
+    """A filter plane of NaN spoils its own correlograms only: they never win,
+    and the other planes' maxima are those of a search without it."""
+    kw = _small_workload(64, W, 32, 15, 3)
+    good = dict(kw, ctf_filters=kw["ctf_filters"][:, [0, 2]].clone(), defocus_values=kw["defocus_values"][[0, 2]])
+    kw["ctf_filters"] = kw["ctf_filters"].clone()
+    kw["ctf_filters"][:, 1] = float("nan")
+    gpu, ref = _gpu_search(kw, 5), _gpu_search(good, 5)
+    assert torch.allclose(gpu["mip"], ref["mip"], rtol=0, atol=1e-5)
+    assert torch.isnan(gpu["correlation_mean"]).all()
+    plane = gpu["best_global_index"].long() // 15
+    assert (plane != 1).all()
+    same = gpu["best_global_index"].long() - plane.clamp(max=1) * 15 == ref["best_global_index"].long()
+    assert same.float().mean() > 0.999
