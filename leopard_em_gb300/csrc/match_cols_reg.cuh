@@ -113,6 +113,38 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
   float2* x = crsm + g * C::STRIDE;
   float2* tab = crsm + G * C::STRIDE;
   if (warp == 0) tmem_alloc(&tm_slot, C::COLS);
+  const int kx = blockIdx.x * G + g;
+  const bool col_ok = kx < Wcp;
+  const bool act2 = FULL2 || t < R1;  // holds a radix-R2 transform
+  const int c_begin = blockIdx.y * c_per_block;
+  const int c_end = min(n_c, c_begin + c_per_block);
+  // sparse inputs of the coming correlogram, read one correlogram ahead
+  constexpr int NZ = SPARSE ? C::R1B : 1;
+  float2 nx[D1][NZ];
+  auto fetch = [&](int c) {
+    const float2* a = A + (size_t)c * h * Wcp + kx;
+#pragma unroll
+    for (int i = 0; i < D1; ++i) {
+      const int b = t + NT * i;
+#pragma unroll
+      for (int q = 0; q < NZ; ++q)
+        nx[i][q] = (col_ok && (FULL1 || (t < NT && b < R2)) && b + R2 * q < h)
+                       ? __ldg(a + (size_t)(b + R2 * q) * Wcp)
+                       : make_float2(0.f, 0.f);
+    }
+  };
+  if (SPARSE && c_begin < c_end) fetch(c_begin);
+  // the first image's columns come in while the roots are computed
+  int image = c_begin / c_per_image;
+  float2 first[R2];
+  {
+    const float2* ip = Ip + (size_t)image * N * Wcp + kx;
+#pragma unroll
+    for (int s = 0; s < R2; ++s) {
+      const int row = t + R1 * DftNT<C::R2A, C::R2B, -1>::out(s);
+      first[s] = (col_ok && act2 && c_begin < c_end) ? __ldg(ip + (size_t)row * Wcp) : make_float2(0.f, 0.f);
+    }
+  }
   if constexpr (C::TWO) {
     auto fill = [&](float2* dst, int r_hi, int nb) {  // rows 0..7: r, rows 8..: 8 (row - 8)
       for (int e = threadIdx.x; e < (8 + r_hi) * nb; e += C::THREADS) {
@@ -135,31 +167,12 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
   tmem_barrier();
   const unsigned tm_base = tm_slot;
   const unsigned tm = tm_base + ((unsigned)(warp % 4) << 21) + (unsigned)(warp / 4) * C::WORDS;
-  const int kx = blockIdx.x * G + g;
-  const bool col_ok = kx < Wcp;
-  const bool act2 = FULL2 || t < R1;  // holds a radix-R2 transform
-  const int c_begin = blockIdx.y * c_per_block;
-  const int c_end = min(n_c, c_begin + c_per_block);
-  int image = -1;
-  // sparse inputs of the coming correlogram, read one correlogram ahead
-  constexpr int NZ = SPARSE ? C::R1B : 1;
-  float2 nx[D1][NZ];
-  auto fetch = [&](int c) {
-    const float2* a = A + (size_t)c * h * Wcp + kx;
 #pragma unroll
-    for (int i = 0; i < D1; ++i) {
-      const int b = t + NT * i;
-#pragma unroll
-      for (int q = 0; q < NZ; ++q)
-        nx[i][q] = (col_ok && (FULL1 || (t < NT && b < R2)) && b + R2 * q < h)
-                       ? __ldg(a + (size_t)(b + R2 * q) * Wcp)
-                       : make_float2(0.f, 0.f);
-    }
-  };
+  for (int s0 = 0; s0 < R2; s0 += CH) tmem_put<CH>(tm + 2 * s0, first + s0);
+  tmem_wait_st();
   using FO = DftNT<C::R1A, C::R1B, +1>;
   const unsigned y_off = (unsigned)(t * Wcp + kx) * 8u, y_step = (unsigned)(R2 * Wcp) * 8u,
                  y_nt = (unsigned)(NT * Wcp) * 8u;
-  if (SPARSE && c_begin < c_end) fetch(c_begin);
 #pragma unroll 1
   for (int c = c_begin; c < c_end; ++c) {
     // ---- this image's columns -> tensor memory, in the slot order of P
