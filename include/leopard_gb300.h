@@ -206,6 +206,14 @@ int lgb_match_finalize(const lgb_match_problem* problem, long long total_positio
                        float* best_phi, float* best_theta, float* best_psi, float* best_defocus,
                        float* corr_mean, float* corr_std, void* stream);
 
+/* The same for a micrograph searched on a larger grid: every output map, the
+ * maximum included, has the micrograph's size (micrograph_h x micrograph_w). */
+int lgb_match_finalize_micrograph(const lgb_match_problem* problem, long long total_positions, const float* mip,
+                                  const int* best_index, const double* corr_sum, const double* corr_sq_sum,
+                                  const float* euler_angles, const float* defocus_values, float* mip_out,
+                                  float* scaled_mip, float* best_phi, float* best_theta, float* best_psi,
+                                  float* best_defocus, float* corr_mean, float* corr_std, void* stream);
+
 /* ------------------------------------------------------------------------ */
 /* Local-grid refinement (core_refine_template.py:33-202, :555-767)          */
 /* ------------------------------------------------------------------------ */

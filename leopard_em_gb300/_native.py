@@ -129,6 +129,7 @@ _SIGNATURES = {
     "lgb_nn_to_bf16": ([_LL, _P, _P, _P], _I),
     "lgb_nn_make_inputs": ([_I, _I, _I, _P, _P, _I] + [_P] * 4 + [ctypes.POINTER(CtfParams), _I, _I, _P, _P], _I),
     "lgb_nn_gauss_newton": ([_I, _I, _I, _P, _P, _P], _I),
+    "lgb_match_finalize_micrograph": ([_PROB, _LL] + [_P] * 15, _I),
     "lgb_match_finalize": ([_PROB, _LL, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P], _I),
 }
 

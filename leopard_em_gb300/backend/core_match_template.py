@@ -429,7 +429,6 @@ class MatchTemplateSearch:
 
         Maps are H x W (the micrograph), also when the search ran on a padded grid."""
         H, W = self.shape
-        Hp, Wp = self.grid
         dev = self.device
         if self.precision_mode:
             status = int(self.device_status.item())
@@ -437,11 +436,11 @@ class MatchTemplateSearch:
                 check(status, "device-side status of the search")
         with torch.cuda.device(dev):
             s = ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
-            out = {k: torch.empty((Hp, Wp), dtype=torch.float32, device=dev) for k in
-                   ("scaled_mip", "best_phi", "best_theta", "best_psi", "best_defocus",
+            res = {k: torch.empty((H, W), dtype=torch.float32, device=dev) for k in
+                   ("mip", "scaled_mip", "best_phi", "best_theta", "best_psi", "best_defocus",
                     "correlation_mean", "correlation_variance")}
             check(
-                lib().lgb_match_finalize(
+                lib().lgb_match_finalize_micrograph(
                     ctypes.byref(self.problem),
                     self.searched_projections,
                     _ptr(self.mip),
@@ -450,29 +449,18 @@ class MatchTemplateSearch:
                     _ptr(self.corr_sq_sum),
                     _ptr(self.decode_euler if self.transpose else self.euler_angles),
                     _ptr(self.defocus_values),
-                    _ptr(out["scaled_mip"]),
-                    _ptr(out["best_phi"]),
-                    _ptr(out["best_theta"]),
-                    _ptr(out["best_psi"]),
-                    _ptr(out["best_defocus"]),
-                    _ptr(out["correlation_mean"]),
-                    _ptr(out["correlation_variance"]),
+                    _ptr(res["mip"]),
+                    _ptr(res["scaled_mip"]),
+                    _ptr(res["best_phi"]),
+                    _ptr(res["best_theta"]),
+                    _ptr(res["best_psi"]),
+                    _ptr(res["best_defocus"]),
+                    _ptr(res["correlation_mean"]),
+                    _ptr(res["correlation_variance"]),
                     s,
                 ),
-                "lgb_match_finalize",
+                "lgb_match_finalize_micrograph",
             )
-            res = {
-                "mip": self.mip.clone(),
-                "scaled_mip": out["scaled_mip"],
-                "best_phi": out["best_phi"],
-                "best_theta": out["best_theta"],
-                "best_psi": out["best_psi"],
-                "best_defocus": out["best_defocus"],
-                "correlation_mean": out["correlation_mean"],
-                "correlation_variance": out["correlation_variance"],
-            }
-            if (Hp, Wp) != (H, W):
-                res = {k: v[:H, :W].contiguous() for k, v in res.items()}
             if self.transpose:
                 res = {k: v.t().contiguous() for k, v in res.items()}
             if to_cpu:

@@ -35,30 +35,67 @@ __global__ void filters_kernel(const float* __restrict__ ctf, const float* __res
     out[i] = ctf[i] * wf[i % plane];
 }
 
-__global__ void finalize_kernel(long long n, int W, long long total, int n_orient, int n_defocus,
-                                const float* __restrict__ mip, const int* __restrict__ best,
-                                const double* __restrict__ s1, const double* __restrict__ s2,
-                                const float* __restrict__ euler, const float* __restrict__ defocus, float* scaled,
-                                float* phi, float* theta, float* psi, float* dfo, float* mean_out, float* std_out) {
-  const long long stride_cs = (long long)n_orient * n_defocus;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const double mean = s1[i] / (double)total;
-    double var = s2[i] / (double)total - mean * mean;
-    const double sd = sqrt(var > 0.0 ? var : 0.0);
-    const float m = mip[i];
-    scaled[i] = sd != 0.0 ? (float)(((double)m - mean) / sd) : 0.0f;
-    mean_out[i] = (float)mean;
-    std_out[i] = (float)sd;
-    // python-style modulo: -1 (never updated) maps to the last index
-    long long g = best[i];
-    long long rem = g % stride_cs;
-    if (rem < 0) rem += stride_cs;
-    const int df = (int)(rem / n_orient);
-    const int o = (int)(rem % n_orient);
-    phi[i] = euler[3 * (size_t)o];
-    theta[i] = euler[3 * (size_t)o + 1];
-    psi[i] = euler[3 * (size_t)o + 2];
-    dfo[i] = defocus[df];
+// Rows and columns of the micrograph only (out_h x out_w of a grid W wide).
+// What bounds it: the maps' traffic (56 B a pixel), now that the FP64 pipe (one
+// operation per SM per clock) is left with the mean and the variance: the
+// standard deviation and z are carried in pairs of floats (48 bits), split from
+// the doubles by integer operations.  24 M pixels: 1,731 us with FP64 division
+// and square root, 793 us with an FP64 Newton step, 365 us now.
+__global__ void __launch_bounds__(256)
+    finalize_kernel(int out_h, int out_w, int W, double inv_total, unsigned stride_cs, unsigned n_orient,
+                    const float* __restrict__ mip, const int* __restrict__ best, const double* __restrict__ s1,
+                    const double* __restrict__ s2, const float* __restrict__ euler, const float* __restrict__ defocus,
+                    float* __restrict__ mip_out, float* __restrict__ scaled, float* __restrict__ phi,
+                    float* __restrict__ theta, float* __restrict__ psi, float* __restrict__ dfo,
+                    float* __restrict__ mean_out, float* __restrict__ std_out) {
+  for (int y = blockIdx.y; y < out_h; y += gridDim.y) {
+    for (int x = blockIdx.x * blockDim.x + threadIdx.x; x < out_w; x += gridDim.x * blockDim.x) {
+      const size_t i = (size_t)y * W + x, o = (size_t)y * out_w + x;
+      const float m = mip[i];
+      const int g = best[i];
+      const double mean = s1[i] * inv_total;
+      const double var = fma(-mean, mean, s2[i] * inv_total);
+      float z = 0.f, sd = 0.f;  // also where var is not a number
+      if (var > 0.0) {
+        if (var > 1e-20 && var < 1e20 && fabs(mean) < 1e20 && fabsf(m) < 1e20f) {
+          const float2 v = d2f_split(var), mu = d2f_split(mean);
+          // 1/sd = y + dy: a float reciprocal square root and its first-order
+          // correction from the exact residual e = 1 - var y^2 (e^2 is below 48 bits)
+          const float y = rsqrtf(v.x);
+          const float p = y * y, pe = fmaf(y, y, -p);
+          const float e = fmaf(-v.x, p, 1.f) - fmaf(v.x, pe, v.y * p);
+          const float dy = 0.5f * y * e;
+          const float s = v.x * y;
+          sd = s + (fmaf(v.x, y, -s) + fmaf(v.y, y, v.x * dy));
+          // m - mean as a sum of two floats
+          const float d = m - mu.x, back = m - d;
+          const float dl = ((m - (d + back)) + (back - mu.x)) - mu.y;
+          const float q = d * y;
+          z = q + (fmaf(d, y, -q) + fmaf(dl, y, d * dy));
+        } else {
+          const double s = sqrt(var);
+          sd = (float)s;
+          z = (float)(((double)m - mean) / s);
+        }
+      }
+      if (mip_out) mip_out[o] = m;
+      scaled[o] = z;
+      mean_out[o] = d2f_bits(mean);
+      std_out[o] = sd;
+      // python-style modulo: -1 (never updated) maps to the last index
+      unsigned rem;
+      if (g >= 0) {
+        rem = (unsigned)g % stride_cs;
+      } else {
+        const long long r = (long long)g % (long long)stride_cs;
+        rem = (unsigned)(r < 0 ? r + stride_cs : r);
+      }
+      const unsigned df = rem / n_orient, k = rem - df * n_orient;
+      phi[o] = euler[3 * (size_t)k];
+      theta[o] = euler[3 * (size_t)k + 1];
+      psi[o] = euler[3 * (size_t)k + 2];
+      dfo[o] = defocus[df];
+    }
   }
 }
 
@@ -362,20 +399,46 @@ int lgb_match_search_graph(const lgb_match_problem* p, const void* template_dft,
   return LGB_OK;
 }
 
+// The maps' first out_h rows and out_w columns; mip_out may be null.
+static int finalize_maps(const lgb_match_problem* p, int out_h, int out_w, long long total_positions, const float* mip,
+                         const int* best_index, const double* corr_sum, const double* corr_sq_sum,
+                         const float* euler_angles, const float* defocus_values, float* mip_out, float* scaled_mip,
+                         float* best_phi, float* best_theta, float* best_psi, float* best_defocus, float* corr_mean,
+                         float* corr_std, void* stream) {
+  if (!valid_problem(p) || total_positions <= 0 || !mip || !best_index || !corr_sum || !corr_sq_sum ||
+      !euler_angles || !defocus_values || !scaled_mip || !best_phi || !best_theta || !best_psi || !best_defocus ||
+      !corr_mean || !corr_std)
+    return LGB_ERR_INVALID_ARGUMENT;
+  // a stride beyond the indices' range leaves every index as it is
+  const long long stride = (long long)p->n_orientations * p->n_defocus;
+  const unsigned stride_cs = stride > 0xffffffffLL ? 0xffffffffu : (unsigned)stride;
+  const int gx = (out_w + 255) / 256, gy = out_h < 65535 ? out_h : 65535;
+  finalize_kernel<<<dim3(gx, gy), 256, 0, (cudaStream_t)stream>>>(
+      out_h, out_w, p->image_w, 1.0 / (double)total_positions, stride_cs, (unsigned)p->n_orientations, mip, best_index,
+      corr_sum, corr_sq_sum, euler_angles, defocus_values, mip_out, scaled_mip, best_phi, best_theta, best_psi,
+      best_defocus, corr_mean, corr_std);
+  return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
+}
+
 int lgb_match_finalize(const lgb_match_problem* p, long long total_positions, const float* mip,
                        const int* best_index, const double* corr_sum, const double* corr_sq_sum,
                        const float* euler_angles, const float* defocus_values, float* scaled_mip, float* best_phi,
                        float* best_theta, float* best_psi, float* best_defocus, float* corr_mean, float* corr_std,
                        void* stream) {
-  if (!valid_problem(p) || total_positions <= 0 || !mip || !best_index || !corr_sum || !corr_sq_sum ||
-      !euler_angles || !defocus_values || !scaled_mip || !best_phi || !best_theta || !best_psi || !best_defocus ||
-      !corr_mean || !corr_std)
-    return LGB_ERR_INVALID_ARGUMENT;
-  const long long n = (long long)p->image_h * p->image_w;
-  finalize_kernel<<<grid_for(n), 256, 0, (cudaStream_t)stream>>>(
-      n, p->image_w, total_positions, p->n_orientations, p->n_defocus, mip, best_index, corr_sum, corr_sq_sum,
-      euler_angles, defocus_values, scaled_mip, best_phi, best_theta, best_psi, best_defocus, corr_mean, corr_std);
-  return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
+  return finalize_maps(p, p ? p->image_h : 0, p ? p->image_w : 0, total_positions, mip, best_index, corr_sum,
+                       corr_sq_sum, euler_angles, defocus_values, nullptr, scaled_mip, best_phi, best_theta, best_psi,
+                       best_defocus, corr_mean, corr_std, stream);
+}
+
+int lgb_match_finalize_micrograph(const lgb_match_problem* p, long long total_positions, const float* mip,
+                                  const int* best_index, const double* corr_sum, const double* corr_sq_sum,
+                                  const float* euler_angles, const float* defocus_values, float* mip_out,
+                                  float* scaled_mip, float* best_phi, float* best_theta, float* best_psi,
+                                  float* best_defocus, float* corr_mean, float* corr_std, void* stream) {
+  if (!mip_out) return LGB_ERR_INVALID_ARGUMENT;
+  return finalize_maps(p, p ? mic_h(p) : 0, p ? mic_w(p) : 0, total_positions, mip, best_index, corr_sum, corr_sq_sum,
+                       euler_angles, defocus_values, mip_out, scaled_mip, best_phi, best_theta, best_psi, best_defocus,
+                       corr_mean, corr_std, stream);
 }
 
 }  // extern "C"

@@ -30,6 +30,30 @@ __device__ __forceinline__ double f2d_bits(float f) {
   const unsigned hi = (u & 0x80000000u) | ((ex + 896u) << 20) | ((u & 0x7fffffu) >> 3);
   return __hiloint2double((int)hi, (int)(u << 29));
 }
+// double -> float rounded to nearest even with integer operations, for values
+// in the range of normal floats; the others go through the converter.
+__device__ __forceinline__ float d2f_bits(double d) {
+  const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
+  const unsigned ex = (hi >> 20) & 0x7ffu;
+  if (ex < 897u || ex > 1149u) return (float)d;
+  const unsigned f = ((ex - 896u) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29);
+  const unsigned rest = lo << 3;  // the 29 bits below the float's mantissa
+  const unsigned up = rest > 0x80000000u || (rest == 0x80000000u && (f & 1u));
+  return __uint_as_float((hi & 0x80000000u) | (f + up));
+}
+// d = x + y to 48 bits with integer operations: x the leading 24 bits
+// (truncated), y the rest.  For |d| < 2^128; below 2^-74 y is dropped, below
+// 2^-126 both are zero.
+__device__ __forceinline__ float2 d2f_split(double d) {
+  const unsigned hi = (unsigned)__double2hiint(d), lo = (unsigned)__double2loint(d);
+  const int ex = (int)((hi >> 20) & 0x7ffu);
+  const unsigned sign = hi & 0x80000000u;
+  if (ex < 897) return make_float2(0.f, 0.f);
+  const float x = __uint_as_float(sign | ((unsigned)(ex - 896) << 23) | ((hi & 0xfffffu) << 3) | (lo >> 29));
+  const int ey = ex - 948;  // biased exponent of 2^(ex - 1023 - 52)
+  const float unit = ey > 0 ? __uint_as_float(sign | ((unsigned)ey << 23)) : 0.f;
+  return make_float2(x, (float)(lo & 0x1fffffffu) * unit);
+}
 __device__ __forceinline__ float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
 // multiply by DIR*i  (DIR = +1: i, DIR = -1: -i)
 template <int DIR>

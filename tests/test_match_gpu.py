@@ -286,3 +286,40 @@ def test_not_finite_correlograms_stay_apart(W):
     assert (plane != 1).all()
     same = gpu["best_global_index"].long() - plane.clamp(max=1) * 15 == ref["best_global_index"].long()
     assert same.float().mean() > 0.999
+
+
+@pytest.mark.parametrize("H,W", [(50, 60), (64, 64), (48, 258)])
+def test_finalize_against_64_bits(H, W):
+    """Mean, std and z of given maps (their edge values among them) against
+    float64 torch; outputs are rounded once to float32, so 1e-6 relative holds them."""
+    kw = _small_workload(H, W, 32, 12, 3)
+    s = MatchTemplateSearch(**kw, device=torch.device("cuda:0"), orientation_batch_size=4)
+    g = torch.Generator().manual_seed(H)
+    shape = s.mip.shape
+    mip = torch.randn(shape, generator=g) * 3
+    mean = torch.randn(shape, generator=g, dtype=torch.float64) * 0.3
+    sd = torch.rand(shape, generator=g, dtype=torch.float64) * 2 + 1e-3
+    sd[0, :8] = torch.tensor([0.0, 1e-20, 1e-9, 1e3, 1e20, 1.0, 1.0, 1.0], dtype=torch.float64)
+    mean[0, 5], mip[0, 6] = float("nan"), -float("inf")
+    best = torch.randint(-1, 36, shape, generator=g, dtype=torch.int32)
+    n = s.total_projections
+    maps = {"mip": mip, "best_global_index": best, "correlation_sum": mean * n,
+            "correlation_squared_sum": (sd**2 + mean**2) * n}
+    s.load_maps({k: v.cuda() for k, v in maps.items()})
+    res = s.result()
+    m = maps["correlation_sum"] / n
+    var = maps["correlation_squared_sum"] / n - m * m
+    ref_sd = torch.where(var > 0, var, torch.zeros_like(var)).sqrt()
+    z = torch.where(ref_sd != 0, (mip.double() - m) / ref_sd, torch.zeros_like(m))
+    idx = best.long() % 36
+    assert res["mip"].shape == (H, W) and torch.equal(res["mip"], mip[:H, :W])
+    # cancellation in var: its float64 rounding error bounds sd and z where sd is small against the mean
+    ok = (var > 1e-9 * (m * m + 1e-300)) & torch.isfinite(m) & torch.isfinite(mip)
+    ok[0, 6:8] = True
+    for key, ref in (("correlation_mean", m), ("correlation_variance", ref_sd), ("scaled_mip", z)):
+        got, want, use = res[key].double(), ref[:H, :W], ok[:H, :W]
+        same = (got == want) | ((got - want).abs() <= 1e-6 * want.abs())
+        assert same[use].all(), key
+    assert torch.isnan(res["correlation_mean"][0, 5]) and res["scaled_mip"][0, 5] == 0
+    assert torch.equal(res["best_phi"], kw["euler_angles"][idx % 12, 0][:H, :W])
+    assert torch.equal(res["best_defocus"], kw["defocus_values"][idx // 12][:H, :W])
