@@ -56,42 +56,132 @@ __device__ __forceinline__ void store8(uint16_t* dst, const float* v) {
 // one row) each, so the stores are fully coalesced: unit u of a blocked operand
 // with TR-row tiles and KC chunks holds row r, K elements [k0, k0 + 8).
 __device__ __forceinline__ void unit_rk(long long u, int TR, int KC, int& r, int& k0) {
+  // (TR is a power of two, and operands have fewer than 2^32 groups of 64 units)
   const int r8 = (int)(u & 7), kg = (int)((u >> 3) & 7);
-  const long long rest = u >> 6;
-  const int rg = (int)(rest % (TR / 8));
-  const long long tc = rest / (TR / 8);
-  r = (int)(tc / KC) * TR + rg * 8 + r8;
-  k0 = (int)(tc % KC) * kTcKC + kg * 8;
+  const unsigned rest = (unsigned)(u >> 6), rg = rest & (unsigned)(TR / 8 - 1);
+  const unsigned tc = rest >> (31 - __clz(TR / 8)), tile = tc / (unsigned)KC;
+  r = (int)(tile * TR + rg * 8 + r8);
+  k0 = (int)((tc - tile * KC) * kTcKC + kg * 8);
 }
 
-// A of the forward and of the weight gradient: im2col(x) [rows p][k], rows
-// padded to TR, K padded to 64 (zeros).  transpose_k = false: rows are pixels
-// and K runs over ci*9+tap; true: rows are ci*9+tap and K runs over pixels,
-// plus row Cin*9 of ones, whose product with g is the bias gradient.
-__global__ void im2col_kernel(ConvShape c, const bf16t* __restrict__ x, int rows_pad, int k_pad, int TR,
-                              bool transpose_k, uint16_t* __restrict__ out) {
+__device__ __forceinline__ void store8_bits(uint16_t* dst, const uint16_t* v) {
+  uint4 u;
+  uint16_t* h = reinterpret_cast<uint16_t*>(&u);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) h[e] = v[e];
+  *reinterpret_cast<uint4*>(dst) = u;
+}
+
+// What bounds the gathers is integer arithmetic (its pipe runs at half the FP32
+// rate) unless positions are divided out once for many elements and the stride
+// is a template argument; a run-time stride and per-element divisions cost 256
+// samples of the network's step 1,648 us in gcol and 762 us in im2col, units of
+// eight elements with stepped positions 580 and 390, this 193 and 185.
+//
+// A row's 72 consecutive K elements are the 9 taps of 8 channels: one thread
+// takes them (nine 16-byte units), its taps at compile time, its position and
+// the taps that fall inside found once.  A warp has 32 consecutive rows, so its
+// sources are neighbours in the image and its stores whole 128-byte lines.
+// pick(t, offset) gives tap t's offset in a channel plane, or false.
+template <class T, class Pick>
+__device__ __forceinline__ void gather_taps(long long e, int rows_pad, int TR, int k_pad, int channels, int plane_size,
+                                            const T* __restrict__ src, Pick pick, uint16_t* __restrict__ out) {
+  const int KC = k_pad / kTcKC, units = k_pad / 8;
+  const int r = (int)(e % rows_pad), group = (int)(e / rows_pad);
+  int off[9];
+  unsigned in = 0;
+  const size_t first = pick(r, off, in);  // channel 0 of the row's image
+  const T* plane = src + first + (size_t)group * 8 * plane_size;
+  uint16_t v[72];
+#pragma unroll
+  for (int ch = 0; ch < 8; ++ch) {
+    const bool ok = group * 8 + ch < channels;
+#pragma unroll
+    for (int t = 0; t < 9; ++t) {
+      if constexpr (sizeof(T) == 2) {
+        v[ch * 9 + t] = (ok && (in >> t & 1u)) ? (uint16_t)plane[off[t]] : (uint16_t)0;
+      } else {
+        v[ch * 9 + t] = __bfloat16_as_ushort(__float2bfloat16_rn((ok && (in >> t & 1u)) ? plane[off[t]] : 0.f));
+      }
+    }
+    plane += plane_size;
+  }
+  const int tile = r / TR, rl = r - tile * TR;
+#pragma unroll
+  for (int u = 0; u < 9; ++u) {
+    const int ku = group * 9 + u;
+    if (ku < units) {
+      const size_t unit = ((size_t)tile * KC + ku / 8) * (TR * 8) + (rl / 8) * 64 + (ku % 8) * 8 + rl % 8;
+      store8_bits(out + unit * 8, v + u * 8);
+    }
+  }
+}
+__host__ __device__ constexpr int tap_groups(int k_pad) { return (k_pad / 8 + 8) / 9; }
+
+// A of the forward: im2col(x) [rows p][k = ci*9+tap], rows padded to TR, K
+// padded to 64 (zeros).
+template <int S>
+__global__ void __launch_bounds__(256) im2col_kernel(ConvShape c, const uint16_t* __restrict__ x, int rows_pad,
+                                                     int k_pad, int TR, uint16_t* __restrict__ out) {
+  const long long n = (long long)rows_pad * tap_groups(k_pad);
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x)
+    gather_taps(e, rows_pad, TR, k_pad, c.Cin, c.H * c.W, x,
+                [&](int p, int* off, unsigned& in) -> size_t {
+                  if (p >= c.P) return 0;
+                  const unsigned img = (unsigned)p / (unsigned)(c.Ho * c.Wo), pix = p - img * (c.Ho * c.Wo);
+                  const int oy = (int)(pix / (unsigned)c.Wo), ox = (int)pix - oy * c.Wo;
+#pragma unroll
+                  for (int t = 0; t < 9; ++t) {
+                    const int iy = oy * S - 1 + t / 3, ix = ox * S - 1 + t % 3;
+                    off[t] = iy * c.W + ix;
+                    if (iy >= 0 && iy < c.H && ix >= 0 && ix < c.W) in |= 1u << t;
+                  }
+                  return (size_t)img * c.Cin * (c.H * c.W);
+                },
+                out);
+}
+
+// A of the weight gradient: rows k = ci*9+tap, K over output pixels p, plus row
+// Cin*9 of ones, whose product with g is the bias gradient.
+template <int S>
+__global__ void im2col_t_kernel(ConvShape c, const uint16_t* __restrict__ x, int rows_pad, int k_pad, int TR,
+                                uint16_t* __restrict__ out) {
+  constexpr uint16_t kOne = 0x3f80;  // 1 in BF16
   const long long n8 = (long long)rows_pad * (k_pad / 8);
   const int KC = k_pad / kTcKC;
+  const unsigned HoWo = c.Ho * c.Wo;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n8; e += (long long)gridDim.x * blockDim.x) {
-    int r, k0;
-    unit_rk(e, TR, KC, r, k0);
-    float v[8];
+    int k, p0;
+    unit_rk(e, TR, KC, k, p0);
+    uint16_t v[8];
+    const int ci = k / 9, tap = k - (k / 9) * 9;
+    const int dy = tap / 3 - 1, dx = tap % 3 - 1;
+    const unsigned n = (unsigned)p0 / HoWo, pix = (unsigned)p0 - n * HoWo;
+    int oy = (int)(pix / (unsigned)c.Wo), ox = (int)pix - oy * c.Wo;
+    const uint16_t* plane = x + ((size_t)n * c.Cin + ci) * (c.H * c.W);
+    if (c.Wo % 8 == 0 && k < c.K) {  // the eight pixels share an image row
+      const int iy = oy * S + dy, ix = ox * S + dx;
+      const bool row = p0 < c.P && iy >= 0 && iy < c.H;
+      const uint16_t* src = plane + iy * c.W + ix;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = (row && ix + i * S >= 0 && ix + i * S < c.W) ? src[i * S] : (uint16_t)0;
+      store8_bits(out + e * 8, v);
+      continue;
+    }
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const int p = transpose_k ? k0 + i : r;
-      const int k = transpose_k ? r : k0 + i;
-      float val = (transpose_k && k == c.K && p < c.P) ? 1.f : 0.f;  // ones row: sums g into db
-      if (p < c.P && k < c.K) {
-        const int n = p / (c.Ho * c.Wo), pix = p % (c.Ho * c.Wo);
-        const int oy = pix / c.Wo, ox = pix % c.Wo;
-        const int ci = k / 9, tap = k % 9;
-        const int iy = oy * c.s - 1 + tap / 3, ix = ox * c.s - 1 + tap % 3;
-        if (iy >= 0 && iy < c.H && ix >= 0 && ix < c.W)
-          val = __bfloat162float(x[(((size_t)n * c.Cin + ci) * c.H + iy) * c.W + ix]);
+      const int iy = oy * S + dy, ix = ox * S + dx;
+      const bool in = p0 + i < c.P, ok = in && k < c.K && iy >= 0 && iy < c.H && ix >= 0 && ix < c.W;
+      v[i] = ok ? plane[iy * c.W + ix] : (in && k == c.K ? kOne : (uint16_t)0);
+      if (++ox == c.Wo) {
+        ox = 0;
+        if (++oy == c.Ho) {
+          oy = 0;
+          plane += (size_t)c.Cin * (c.H * c.W);
+        }
       }
-      v[i] = val;
     }
-    store8(out + e * 8, v);
+    store8_bits(out + e * 8, v);
   }
 }
 
@@ -133,32 +223,26 @@ __global__ void weights_t_kernel(ConvShape c, const bf16t* __restrict__ w, int r
 
 // A of the input gradient: col(g)[q][co*9 + tap] = g[n][co][oy][ox] for the
 // output pixel whose tap covers input pixel q (zero where none does)
-__global__ void gcol_kernel(ConvShape c, const float* __restrict__ g, int rows_pad, int k_pad,
-                            uint16_t* __restrict__ out) {
-  const long long n8 = (long long)rows_pad * (k_pad / 8);
-  const int KC = k_pad / kTcKC;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n8; e += (long long)gridDim.x * blockDim.x) {
-    int q, k0;
-    unit_rk(e, kTcM, KC, q, k0);
-    float v[8];
+template <int S>
+__global__ void __launch_bounds__(256) gcol_kernel(ConvShape c, const float* __restrict__ g, int rows_pad, int k_pad,
+                                                   uint16_t* __restrict__ out) {
+  const long long n = (long long)rows_pad * tap_groups(k_pad);
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x)
+    gather_taps(e, rows_pad, kTcM, k_pad, c.Cout, c.Ho * c.Wo, g,
+                [&](int q, int* off, unsigned& in) -> size_t {
+                  if (q >= c.Q) return 0;
+                  const unsigned img = (unsigned)q / (unsigned)(c.H * c.W), pix = q - img * (c.H * c.W);
+                  const int iy = (int)(pix / (unsigned)c.W), ix = (int)pix - iy * c.W;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int kt = k0 + i;
-      float val = 0.f;
-      if (q < c.Q && kt < c.Kt) {
-        const int n = q / (c.H * c.W), pix = q % (c.H * c.W);
-        const int iy = pix / c.W, ix = pix % c.W;
-        const int co = kt / 9, tap = kt % 9;
-        const int ty = iy + 1 - tap / 3, tx = ix + 1 - tap % 3;
-        if (ty >= 0 && tx >= 0 && ty % c.s == 0 && tx % c.s == 0) {
-          const int oy = ty / c.s, ox = tx / c.s;
-          if (oy < c.Ho && ox < c.Wo) val = g[(((size_t)n * c.Cout + co) * c.Ho + oy) * c.Wo + ox];
-        }
-      }
-      v[i] = val;
-    }
-    store8(out + e * 8, v);
-  }
+                  for (int t = 0; t < 9; ++t) {
+                    const int ty = iy + 1 - t / 3, tx = ix + 1 - t % 3;
+                    const int oy = ty / S, ox = tx / S;  // used for ty, tx >= 0 only
+                    off[t] = oy * c.Wo + ox;
+                    if (ty >= 0 && tx >= 0 && oy * S == ty && ox * S == tx && oy < c.Ho && ox < c.Wo) in |= 1u << t;
+                  }
+                  return (size_t)img * c.Cout * (c.Ho * c.Wo);
+                },
+                out);
 }
 
 // B of the weight gradient: gT[co][p] = g[n][co][oy][ox]
@@ -166,15 +250,21 @@ __global__ void gT_kernel(ConvShape c, const float* __restrict__ g, int rows_pad
                           uint16_t* __restrict__ out) {
   const long long n8 = (long long)rows_pad * (k_pad / 8);
   const int KC = k_pad / kTcKC;
-  const int HoWo = c.Ho * c.Wo;
+  const unsigned HoWo = c.Ho * c.Wo;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n8; e += (long long)gridDim.x * blockDim.x) {
     int co, p0;
     unit_rk(e, TR, KC, co, p0);
     float v[8];
+    const unsigned n = (unsigned)p0 / HoWo;
+    unsigned pix = (unsigned)p0 - n * HoWo;
+    const float* plane = g + ((size_t)n * c.Cout + co) * HoWo;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const int p = p0 + i;
-      v[i] = (co < c.Cout && p < c.P) ? g[((size_t)(p / HoWo) * c.Cout + co) * HoWo + p % HoWo] : 0.f;
+      v[i] = (co < c.Cout && p0 + i < c.P) ? plane[pix] : 0.f;
+      if (++pix == HoWo) {
+        pix = 0;
+        plane += (size_t)c.Cout * HoWo;
+      }
     }
     store8(out + e * 8, v);
   }
@@ -406,8 +496,8 @@ int lgb_nn_conv3x3_forward(int N, int Cin, int H, int W, int Cout, int stride, i
   uint16_t* bm = reinterpret_cast<uint16_t*>(static_cast<char*>(workspace) + ws.fwd_a);
   const int bn = bn_for(Cout);
   const int kp = round_up(c.K, kTcKC), pp = round_up(c.P, kTcM), cp = round_up(Cout, bn);
-  im2col_kernel<<<grid256((long long)pp * kp / 8), 256, 0, s>>>(c, static_cast<const bf16t*>(x), pp, kp, kTcM, false,
-                                                                 a);
+  (stride == 1 ? im2col_kernel<1> : im2col_kernel<2>)<<<grid256((long long)pp * tap_groups(kp)), 256, 0, s>>>(
+      c, static_cast<const uint16_t*>(x), pp, kp, kTcM, a);
   weights_kernel<<<grid256((long long)cp * kp / 8), 256, 0, s>>>(Cout, c.K, static_cast<const bf16t*>(w), cp, kp, bn,
                                                                  bm);
   if (cudaGetLastError() != cudaSuccess) return LGB_ERR_CUDA;
@@ -434,7 +524,8 @@ int lgb_nn_conv3x3_backward(int N, int Cin, int H, int W, int Cout, int stride, 
     uint16_t* bm = reinterpret_cast<uint16_t*>(base + ws.dx_a);
     const int bn = bn_for(Cin);
     const int kp = round_up(c.Kt, kTcKC), qp = round_up(c.Q, kTcM), cp = round_up(Cin, bn);
-    gcol_kernel<<<grid256((long long)qp * kp / 8), 256, 0, s>>>(c, g, qp, kp, a);
+    (stride == 1 ? gcol_kernel<1> : gcol_kernel<2>)<<<grid256((long long)qp * tap_groups(kp)), 256, 0, s>>>(c, g, qp,
+                                                                                                            kp, a);
     weights_t_kernel<<<grid256((long long)cp * kp / 8), 256, 0, s>>>(c, static_cast<const bf16t*>(w), cp, kp, bn, bm);
     if (cudaGetLastError() != cudaSuccess) return LGB_ERR_CUDA;
     EpiConvDx::Params ep{dx, Cin, H * W, c.Q};
@@ -447,8 +538,8 @@ int lgb_nn_conv3x3_backward(int N, int Cin, int H, int W, int Cout, int stride, 
     uint16_t* bm = reinterpret_cast<uint16_t*>(base + ws.dw_a);
     const int bn = bn_for(Cout);
     const int pk = round_up(c.P, kTcKC), kr = round_up(c.K + 1, kTcM), cp = round_up(Cout, bn);
-    im2col_kernel<<<grid256((long long)kr * pk / 8), 256, 0, s>>>(c, static_cast<const bf16t*>(x), kr, pk, kTcM, true,
-                                                                  a);
+    (stride == 1 ? im2col_t_kernel<1> : im2col_t_kernel<2>)<<<grid256((long long)kr * pk / 8), 256, 0, s>>>(
+        c, static_cast<const uint16_t*>(x), kr, pk, kTcM, a);
     gT_kernel<<<grid256((long long)cp * pk / 8), 256, 0, s>>>(c, g, cp, pk, bn, bm);
     if (cudaGetLastError() != cudaSuccess) return LGB_ERR_CUDA;
     if (cudaMemsetAsync(dw, 0, sizeof(float) * (size_t)Cout * c.K, s) != cudaSuccess) return LGB_ERR_CUDA;

@@ -211,3 +211,61 @@ def test_linear_layer_odd_shapes_match_torch(N, In, Out):
     assert _rel(dx, gq @ w.float()) < 1e-2
     assert _rel(dw, gq.t() @ x.float()) < 1e-2
     assert _rel(db, gq.sum(0)) < 1e-2
+
+
+@pytest.mark.parametrize("N,Cin,H,W,Cout,stride", [(2, 9, 6, 16, 11, 1), (3, 17, 32, 16, 40, 2), (1, 8, 5, 24, 8, 1),
+                                                   (2, 1, 16, 48, 3, 2)])
+def test_conv_gathers_whole_image_rows(N, Cin, H, W, Cout, stride):
+    """The gathers where eight pixels share an image row and channel groups end
+    unevenly, against torch on the same BF16 operands (the tolerance of the odd shapes)."""
+    import ctypes
+
+    from leopard_em_gb300._native import lib
+
+    L = lib()
+    g = torch.Generator().manual_seed(N * 100 + Cin)
+    x = torch.randn(N, Cin, H, W, generator=g).to(torch.bfloat16)
+    w = (0.2 * torch.randn(Cout, Cin, 3, 3, generator=g)).to(torch.bfloat16)
+    Ho, Wo = (H - 1) // stride + 1, (W - 1) // stride + 1
+    gy = torch.randn(N, Cout, Ho, Wo, generator=g)
+    xd, wd, gd = x.to(DEV), w.to(DEV), gy.to(DEV)
+    ws = _layer_ws(L, L.lgb_nn_conv3x3_workspace_size, N, Cin, H, W, Cout, stride)
+    st = torch.zeros(1, dtype=torch.int32, device=DEV)
+    s = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    y = torch.empty(N, Cout, Ho, Wo, dtype=torch.bfloat16, device=DEV)
+    assert L.lgb_nn_conv3x3_forward(N, Cin, H, W, Cout, stride, 0, xd.data_ptr(), wd.data_ptr(), None, y.data_ptr(),
+                                    ws.data_ptr(), ws.numel(), st.data_ptr(), s) == 0
+    dx = torch.empty(N, Cin, H, W, device=DEV)
+    dw = torch.empty(Cout, Cin, 3, 3, device=DEV)
+    db = torch.empty(Cout, device=DEV)
+    assert L.lgb_nn_conv3x3_backward(N, Cin, H, W, Cout, stride, xd.data_ptr(), wd.data_ptr(), gd.data_ptr(),
+                                     dx.data_ptr(), dw.data_ptr(), db.data_ptr(), ws.data_ptr(), ws.numel(),
+                                     st.data_ptr(), s) == 0
+    torch.cuda.synchronize()
+    assert int(st.item()) == 0
+    xr, wr = x.float().requires_grad_(True), w.float().requires_grad_(True)
+    gq = gy.to(torch.bfloat16).float()
+    yr = torch.nn.functional.conv2d(xr, wr, stride=stride, padding=1)
+    yr.backward(gq)
+    assert _rel(y.float(), yr.detach()) < 1e-2
+    assert _rel(dx, xr.grad) < 1e-2
+    assert _rel(dw, wr.grad) < 1e-2
+    assert _rel(db, gq.sum((0, 2, 3))) < 1e-2
+
+
+@pytest.mark.parametrize("n,offset", [(4096, 0), (4097, 0), (4096, 1), (8, 0), (3, 0)])
+def test_relu_backward_bits(n, offset):
+    """Four at a time, scalar tails and unaligned buffers: zero wherever y is not above zero."""
+    import ctypes
+
+    from leopard_em_gb300._native import lib
+
+    y = torch.randn(n + offset).to(torch.bfloat16)
+    y[:3] = torch.tensor([0.0, -0.0, float("nan")]).to(torch.bfloat16)[: len(y[:3])]
+    d = torch.randn(n + offset)
+    yd, dd = y.to(DEV)[offset:], d.to(DEV)[offset:]
+    out = torch.empty(n + offset, device=DEV)[offset:]
+    s = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    assert lib().lgb_nn_relu_backward(n, yd.data_ptr(), dd.data_ptr(), out.data_ptr(), s) == 0
+    ref = torch.where(y[offset:].float() > 0, d[offset:], torch.zeros(n))
+    assert torch.equal(out.cpu(), ref)
