@@ -57,44 +57,50 @@ __global__ void refine_rotations_kernel(const float* __restrict__ euler, const f
 // out[p][cs][df][y][x] = pf[p][y][x] * CTF(p, cs, df; y, x) * exp(-B k^2 / 4)
 // CTF = -sin(chi), chi = -pi lambda k^2 df(theta) + pi/2 Cs lambda^3 k^4 - phase - atan(A / sqrt(1 - A^2)),
 // df(theta) = defocus + astig cos(2 (theta - angle)), Cs = Cs0 / ((px + off)/px)^4.
-// The phase is a polynomial in (kx, ky) evaluated in FP64 without transcendental
-// calls: k^2 cos(2 (theta - a)) = (kx^2 - ky^2) cos 2a + 2 kx ky sin 2a.  It is
-// reduced to [-pi, pi] in FP64 and its sine (and the B envelope) taken in FP32,
-// which keeps the FP64 phase accuracy at a small fraction of the cost of FP64
-// atan2 / cos / sin / exp per filter element.
-__global__ void refine_filters_kernel(const float* __restrict__ pf, const float* __restrict__ du,
-                                      const float* __restrict__ dv, const float* __restrict__ dang,
-                                      const float* __restrict__ dfo, const float* __restrict__ pxo, int P, int C,
-                                      int D, int d, lgb_ctf_params prm, double lambda, float* __restrict__ out) {
-  const int wc = d / 2 + 1;
-  const long long plane = (long long)d * wc;
-  const long long n = (long long)P * C * D * plane;
-  const double pi = 3.14159265358979323846;
-  const double k5 = atan(prm.amplitude_contrast / sqrt(1.0 - prm.amplitude_contrast * prm.amplitude_contrast));
-  const double phase0 = prm.phase_shift_deg * pi / 180.0 + k5;
-  const double lam3 = lambda * lambda * lambda;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-    const int xy = (int)(e % plane);
-    const long long r = e / plane;
-    const int df = (int)(r % D);
-    const int cs = (int)((r / D) % C);
-    const int p = (int)(r / ((long long)D * C));
-    const int y = xy / wc, x = xy % wc;
-    const double ky = (double)(y < (d + 1) / 2 ? y : y - d) / d / prm.pixel_size;
-    const double kx = (double)x / d / prm.pixel_size;
-    const double k2 = kx * kx + ky * ky;
-    float s2a, c2a;  // 2 * angle, in units of pi: angle / 90
-    sincospif(dang[p] / 90.0f, &s2a, &c2a);
-    const double defocus = (double)dfo[df] + 0.5 * ((double)du[p] + (double)dv[p]);
-    const double astig = 0.5 * fabs((double)du[p] - (double)dv[p]);
-    const double dfk2 = defocus * k2 + astig * ((kx * kx - ky * ky) * (double)c2a + 2.0 * kx * ky * (double)s2a);
-    const double rel = ((double)prm.pixel_size + (double)pxo[cs]) / prm.pixel_size;
-    const double csA = prm.spherical_aberration_mm / (rel * rel * rel * rel) * 1e7;
-    const double chi = -pi * lambda * dfk2 + 0.5 * pi * csA * lam3 * k2 * k2 - phase0;
-    const double red = chi - 2.0 * pi * rint(chi / (2.0 * pi));
-    const float ctf = -sinf((float)red);
-    const float env = expf((float)(-prm.b_factor * k2 / 4.0));
-    out[e] = pf[(size_t)p * plane + xy] * (ctf * env);
+// The phase is a polynomial in (kx, ky) without transcendental calls:
+// k^2 cos(2 (theta - a)) = (kx^2 - ky^2) cos 2a + 2 kx ky sin 2a.  It is kept in
+// FP64 turns (chi / 2 pi), reduced to [-1/2, 1/2] by subtracting its nearest
+// integer, and its sine (and the B envelope) taken in FP32.  The FP64 pipe does
+// about one operation per SM per clock, so a thread evaluates the polynomial
+// once for its frequency and takes the defocus offsets in turn, four FP64
+// operations each: 32 particles x 9 defocus x 256 x 129 took 2,912 us with the
+// whole FP64 expression (divisions included) per element, 206 now.
+struct FilterTurns {
+  double inv_size;            // 1 / (d px)
+  double defocus, spherical;  // turns per (Angstrom k^2) and, without Cs, per k^4
+  double phase0;              // constant phase in turns
+};
+
+__global__ void __launch_bounds__(256)
+    refine_filters_kernel(const float* __restrict__ pf, const float* __restrict__ du, const float* __restrict__ dv,
+                          const float* __restrict__ dang, const float* __restrict__ dfo,
+                          const float* __restrict__ pxo, int C, int D, int d, lgb_ctf_params prm, FilterTurns turns,
+                          float* __restrict__ out) {
+  const int wc = d / 2 + 1, plane = d * wc;
+  const int xy = blockIdx.x * blockDim.x + threadIdx.x;
+  if (xy >= plane) return;
+  const int cs = blockIdx.y % C, p = blockIdx.y / C;
+  const int y = xy / wc, x = xy - (xy / wc) * wc;
+  const double ky = (double)(y < (d + 1) / 2 ? y : y - d) * turns.inv_size;
+  const double kx = (double)x * turns.inv_size;
+  const double k2 = kx * kx + ky * ky;
+  float s2a, c2a;  // 2 * angle, in units of pi: angle / 90
+  sincospif(dang[p] / 90.0f, &s2a, &c2a);
+  const double defocus = 0.5 * ((double)du[p] + (double)dv[p]);
+  const double astig = 0.5 * fabs((double)du[p] - (double)dv[p]);
+  const double dfk2 = defocus * k2 + astig * ((kx * kx - ky * ky) * (double)c2a + 2.0 * kx * ky * (double)s2a);
+  const double rel = ((double)prm.pixel_size + (double)pxo[cs]) / prm.pixel_size;
+  const double rel2 = rel * rel;
+  const double spherical = turns.spherical * (prm.spherical_aberration_mm * 1e7 / (rel2 * rel2));
+  const double base = spherical * k2 * k2 - turns.defocus * dfk2 - turns.phase0;
+  const double slope = -turns.defocus * k2;
+  const float weight = -pf[(size_t)p * plane + xy] * expf((float)(-prm.b_factor * k2 / 4.0));
+  float* o = out + (size_t)blockIdx.y * D * plane + xy;
+  constexpr double kRound = 6755399441055744.0;  // 1.5 * 2^52: adding and subtracting rounds to an integer
+  for (int df = 0; df < D; ++df) {
+    const double t = fma(slope, f2d_bits(dfo[df]), base);
+    const double n = __dadd_rn(__dadd_rn(t, kRound), -kRound);
+    o[(size_t)df * plane] = weight * sinpif(2.0f * d2f_bits(t - n));
   }
 }
 
@@ -519,9 +525,21 @@ int lgb_refine_search(const lgb_refine_problem* p, const lgb_ctf_params* ctf, co
 
   repack_stack_kernel<<<grid256((long long)P * H * L.wcp), 256, 0, s>>>(
       static_cast<const float2*>(particle_stack_dft), (long long)P * H, W / 2 + 1, L.wcp, ip);
-  refine_filters_kernel<<<grid256((long long)P * C * D * d * L.wc_t), 256, 0, s>>>(
-      projective_filters, defocus_u, defocus_v, defocus_angle, defocus_offsets, pixel_size_offsets, P, C, D, d, *ctf,
-      electron_wavelength_angstrom(ctf->voltage_kv), filt);
+  const double lambda = electron_wavelength_angstrom(ctf->voltage_kv), amp = ctf->amplitude_contrast;
+  FilterTurns turns;
+  turns.inv_size = 1.0 / (d * ctf->pixel_size);
+  turns.defocus = 0.5 * lambda;
+  turns.spherical = 0.25 * lambda * lambda * lambda;
+  turns.phase0 = ctf->phase_shift_deg / 360.0 + atan(amp / sqrt(1.0 - amp * amp)) / (2.0 * 3.14159265358979323846);
+  // particles x pixel sizes on grid y, in launches of at most 65,535 of them
+  const int per_launch = C <= 65535 ? 65535 / C : 0;
+  if (per_launch < 1) return LGB_ERR_INVALID_ARGUMENT;
+  for (int p0 = 0; p0 < P; p0 += per_launch) {
+    const int np = P - p0 < per_launch ? P - p0 : per_launch;
+    refine_filters_kernel<<<dim3((d * L.wc_t + 255) / 256, np * C), 256, 0, s>>>(
+        projective_filters + (size_t)p0 * d * L.wc_t, defocus_u + p0, defocus_v + p0, defocus_angle + p0,
+        defocus_offsets, pixel_size_offsets, C, D, d, *ctf, turns, filt + (size_t)p0 * C * D * d * L.wc_t);
+  }
   refine_init_kernel<<<(P + 127) / 128, 128, 0, s>>>(P, best_z, best_cc, best_flat, best_offset_begin,
                                                        best_batch_len, key, cc);
   if (cudaGetLastError() != cudaSuccess) return LGB_ERR_CUDA;
