@@ -24,6 +24,7 @@
 #pragma once
 
 #include "fft.cuh"
+#include "reg_dft.cuh"
 
 namespace lgb {
 
@@ -341,39 +342,42 @@ __global__ void __launch_bounds__(ROWS* R1)
 
 // proj_row and the zero-padded row rfft in one kernel, for d = 256 templates
 // and rows of W = 288 (the refinement crops).  Per row y of T[c]: the 256-point
-// c2r as in proj_row_pair_kernel<16, 8> (pixel pairs m = t + 16r in thread t),
-// the row moments, the ifftshift (pair m -> m' = (m + 64) mod 128), then the
-// rfft of the un-normalised row zero padded to W in two register passes
-// (144 = 16 x 9) and the real post-process:
+// c2r through 128 = 16 x 8 complex points, the row moments, the ifftshift (pixel
+// pair m -> m' = (m + 64) mod 128), then the rfft of the un-normalised row zero
+// padded to W through 144 = 16 x 9 points:
 //   A[c][py][k] = sum_{px < d} p[py][px] exp(-2 pi i k px / W),  k <= W/2.
 // The projection never goes to memory.  Its normalisation (p - e) s
 // (utils.py:106-188) is affine, rfft((p - e) s) = s (A - e U) with
 // U[k] = sum_{px < d} exp(-2 pi i k px / W), and is applied by the column pass.
+//
+// What bounds it: the shared-memory data path, which ran at 85 % with 57 % of
+// it bank conflicts when rows were staged, the real transforms' pre- and
+// post-processing read mirrored elements from shared memory, and all roots
+// came from tables.  Now the three transposes are all that crosses it: both
+// mirrored reads are shuffles between the threads t and -t of a row, the first
+// pass reads T directly, the roots of a thread's position stay in registers
+// over the row groups of a CTA and the others are literals.
+// CTAs of 8 rows, six per SM, wait less at the barriers between passes of
+// unequal width than 16-row ones.  9,216 correlograms: 1,959 -> 1,531 us (16 rows
+// 1,662), 288: 76 -> 66.
 template <int ROWS>
-__global__ void __launch_bounds__(ROWS * 16)
-    proj_row_rfft_kernel(const float2* __restrict__ T, double* __restrict__ rowstats, int Wcp,
+__global__ void __launch_bounds__(ROWS * 16, 48 / ROWS)
+    proj_row_rfft_kernel(const float2* __restrict__ T, double* __restrict__ rowstats, int Wcp, int groups,
                          float2* __restrict__ A) {
   constexpr int HT = 256, M = 128, WC = M + 1, NT = 16, S1 = 17;
   constexpr int WH = 144;  // W / 2
   constexpr int C2 = 8;    // c2r: M = 16 x 8
   constexpr int R2 = 9;    // rfft: WH = 16 x 9
-  // Row strides of the shared buffers, chosen for the densely packed first
-  // passes below, where two rows share a half-warp: 152 float2 (xz) and
-  // 153 = R2 * S1 (zb) keep those loads and stores at the fewest bank
-  // conflicts the index maps allow (per-row passes are conflict free at any
-  // stride).
-  constexpr int ZR = 152;
-  static_assert(ZR >= IdxPad16::pad(WH) - 1 && ZR >= WC + 1, "staged row and padded rfft input fit");
-  // xin (the staged row of T, read only by c2r pass 1) and zr (the rfft input,
-  // written from c2r pass 2 on, then Z) share one buffer per row
-  __shared__ float2 xz[ROWS][ZR];
-  __shared__ float2 zb[ROWS][R2 * S1];  // c2r transpose (8 x 17), then rfft transpose (9 x 17)
-  float2(*xin)[ZR] = xz;
-  float2(*zr)[ZR] = xz;
-  __shared__ float2 pre[M];                 // exp(+i pi k / M)
-  __shared__ float2 rootc[15 * (C2 - 1) + 1];  // exp(+2 pi i m / M)
-  __shared__ float2 rootr[15 * (R2 - 1) + 1];  // exp(-2 pi i m / WH)
-  __shared__ float2 post[WH + 1];              // exp(-i pi k / WH)
+  // The two radix-16 passes have fewer DFTs per row (8 and 9) than a row has
+  // threads (16): their (row, DFT) tasks are packed densely onto the CTA's
+  // threads.  Row strides of 8 and 9 (mod 16) float2 keep the packed rows'
+  // accesses conflict free, the others are at any stride.
+  constexpr int SC = C2 * S1, SR = R2 * S1;  // 136 and 153
+  static_assert(SC % 16 == 8 && SR % 16 == 9 && SR >= WH, "conflict-free row strides");
+  __shared__ float2 zb[ROWS * SR];  // c2r transpose (8 x 17 a row), then rfft transpose (9 x 17)
+  __shared__ float2 zr[ROWS * SR];  // rfft input
+  __shared__ float2 pre[M];         // exp(+i pi k / M)
+  __shared__ float2 post[WH + 1];   // exp(-i pi k / WH)
   for (int k = threadIdx.x; k < M; k += blockDim.x) {
     float sn, cs;
     sincospif((float)k / (float)M, &sn, &cs);
@@ -384,116 +388,138 @@ __global__ void __launch_bounds__(ROWS * 16)
     sincospif((float)k / (float)WH, &sn, &cs);
     post[k] = make_float2(cs, -sn);
   }
+  __syncthreads();
   const int c = blockIdx.y;
-  const int g = threadIdx.x / NT, t = threadIdx.x - (threadIdx.x / NT) * NT;
-  const int row0 = blockIdx.x * ROWS;
-  const float2* src = T + ((size_t)c * HT + row0) * WC;
-  for (int e = threadIdx.x; e < ROWS * WC; e += blockDim.x) xin[e / WC][e % WC] = src[e];
-  __syncthreads();
-  // the radix roots are the pre- and post-twiddles at even angles:
-  // exp(+2 pi i m / M) = +-pre[2m mod M], exp(-2 pi i m / WH) = +-post[2m mod WH]
-  // (read from the next pass on, after a barrier)
-  for (int m = threadIdx.x; m < 15 * (C2 - 1) + 1; m += blockDim.x) {
-    const float2 v = pre[(2 * m) & (M - 1)];
-    rootc[m] = 2 * m < M ? v : make_float2(-v.x, -v.y);
-  }
-  for (int m = threadIdx.x; m < 15 * (R2 - 1) + 1; m += blockDim.x) {
-    const float2 v = post[2 * m <= WH ? 2 * m : 2 * m - WH];
-    rootr[m] = 2 * m <= WH ? v : make_float2(-v.x, -v.y);
-  }
-  // The two radix-16 passes have fewer DFTs per row (8 and 9) than a row has
-  // threads (16): their (row, DFT) tasks are packed densely onto the CTA's
-  // threads, so whole warps idle instead of half of every warp's lanes.
-  // ---- c2r pass 1 (radix 16) on the pre-twiddled z[k], k = tt + 8q
-  if (threadIdx.x < ROWS * C2) {
-    const int gg = threadIdx.x / C2, tt = threadIdx.x - (threadIdx.x / C2) * C2;
-    float2 v[16];
+  const int g = threadIdx.x / NT, t = threadIdx.x % NT, lane = threadIdx.x & 31;
+  // roots of this thread's position: exp(+2 pi i r t / M) = +-pre[2 r t mod M] and
+  // exp(-2 pi i r t / WH) = +-post[2 r t mod WH]
+  float2 rootc[C2], rootr[R2];
 #pragma unroll
-    for (int q = 0; q < 16; ++q) {
-      const int k = tt + q * C2;
-      float2 a = xin[gg][k];
-      float2 b = xin[gg][M - k];
-      if (k == 0) { a.y = 0.f; b.y = 0.f; }  // DC and Nyquist: real parts only
-      b.y = -b.y;
-      const float2 xo = cmul(csub(a, b), pre[k]);
-      v[q] = cadd(cadd(a, b), mul_i<1>(xo));
+  for (int r = 1; r < C2; ++r) {
+    const int m = 2 * r * t;
+    const float2 v = pre[m & (M - 1)];
+    rootc[r] = m < M ? v : make_float2(-v.x, -v.y);
+  }
+#pragma unroll
+  for (int r = 1; r < R2; ++r) {
+    const int m = 2 * r * t;
+    const float2 v = post[m <= WH ? m : m - WH];
+    rootr[r] = m <= WH ? v : make_float2(-v.x, -v.y);
+  }
+  const float2 prej = pre[threadIdx.x % C2], postj = post[t];
+#pragma unroll 1
+  for (int grp = 0; grp < groups; ++grp) {
+    const int row0 = (blockIdx.x * groups + grp) * ROWS;
+    // ---- c2r pass 1 (radix 16) over k = tt + 8q
+    if (threadIdx.x < ROWS * C2) {
+      const int gg = threadIdx.x / C2, tt = threadIdx.x % C2;
+      const float2* src = T + ((size_t)c * HT + row0 + gg) * WC;
+      float2 x[16], u[16];
+#pragma unroll
+      for (int q = 0; q < 16; ++q) x[q] = __ldg(src + tt + C2 * q);
+      const float2 nyquist = tt == 0 ? __ldg(src + M) : make_float2(0.f, 0.f);
+      const int mirror = (lane & ~(C2 - 1)) | ((C2 - tt) & (C2 - 1));  // M - k = (8 - tt) + 8 (15 - q)
+      static_for<16>([&](auto q_) {
+        constexpr int q = decltype(q_)::value;
+        float2 a = x[q], b;
+        b.x = __shfl_sync(0xffffffffu, x[15 - q].x, mirror);
+        b.y = __shfl_sync(0xffffffffu, x[15 - q].y, mirror);
+        const float2 own = q ? x[(16 - q) % 16] : nyquist;
+        if (tt == 0) b = own;
+        if (q == 0 && tt == 0) a.y = b.y = 0.f;  // DC and Nyquist: real parts only
+        b.y = -b.y;
+        const float2 xo = mul_root<q, 32, +1>(cmul(csub(a, b), prej));
+        u[q] = cadd(cadd(a, b), mul_i<1>(xo));
+      });
+      Dft<16, +1>::run(u);
+#pragma unroll
+      for (int q = 0; q < 16; ++q) zb[gg * SC + tt * S1 + q] = u[q];
     }
-    Dft<16, +1>::run(v);
+    __syncthreads();
+    // ---- c2r pass 2 (radix 8): pixel pairs m = t + 16r, moments, shifted rfft input
+    {
+      const int y = row0 + g;
+      const int py = (y + HT - HT / 2) % HT;
+      float2 w[C2];
 #pragma unroll
-    for (int q = 0; q < 16; ++q) zb[gg][tt * S1 + q] = v[q];
-  }
-  __syncthreads();
-  // ---- c2r pass 2 (radix 8): pixel pairs m = t + 16r, moments, shifted rfft input
-  const int y = row0 + g;
-  const int py = (y + HT - HT / 2) % HT;
-  {
-    float2 w[C2];
+      for (int r = 0; r < C2; ++r) {
+        w[r] = zb[g * SC + r * S1 + t];
+        if (r) w[r] = cmul(w[r], rootc[r]);
+      }
+      Dft<C2, +1>::run(w);
+      const float scale = 1.0f / ((float)HT * (float)HT);
+      const bool edge_row = (py == 0) || (py == HT - 1);
+      float s1 = 0.f, s2 = 0.f, se = 0.f;
 #pragma unroll
-    for (int r = 0; r < C2; ++r) w[r] = cmul(zb[g][r * S1 + t], rootc[r * t]);
-    Dft<C2, +1>::run(w);
-    const float scale = 1.0f / ((float)HT * (float)HT);
-    const bool edge_row = (py == 0) || (py == HT - 1);
-    float s1 = 0.f, s2 = 0.f, se = 0.f;
+      for (int r = 0; r < C2; ++r) {
+        const int m = t + r * 16;
+        const float a = w[r].x * scale, b = w[r].y * scale;
+        const int mp = (m + M / 2) & (M - 1);  // ifftshift: px = 2 mp, 2 mp + 1
+        zr[g * SR + mp] = make_float2(a, b);
+        s1 += a + b;
+        s2 = fmaf(a, a, fmaf(b, b, s2));
+        if (edge_row) {
+          se += a + b;
+        } else {
+          if (mp == 0) se += a;
+          if (mp == M - 1) se += b;
+        }
+      }
 #pragma unroll
-    for (int r = 0; r < C2; ++r) {
-      const int m = t + r * 16;
-      const float a = w[r].x * scale, b = w[r].y * scale;
-      const int mp = (m + M / 2) & (M - 1);  // ifftshift: px = 2 mp, 2 mp + 1
-      zr[g][IdxPad16::f(mp)] = make_float2(a, b);
-      s1 += a + b;
-      s2 = fmaf(a, a, fmaf(b, b, s2));
-      if (edge_row) {
-        se += a + b;
-      } else {
-        if (mp == 0) se += a;
-        if (mp == M - 1) se += b;
+      for (int o = 8; o > 0; o >>= 1) {
+        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+        s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+        se += __shfl_xor_sync(0xffffffffu, se, o);
+      }
+      if (t == 0) {
+        double* rs = rowstats + ((size_t)c * HT + py) * 3;
+        rs[0] = (double)s1;
+        rs[1] = (double)s2;
+        rs[2] = (double)se;
       }
     }
-    zr[g][IdxPad16::f(M + t)] = make_float2(0.f, 0.f);  // zero padding m' = 128..143
+    __syncthreads();
+    // ---- rfft pass 1 (radix 16) over m' = tt + 9q; m' >= 128 is the zero padding
+    if (threadIdx.x < ROWS * R2) {
+      const int gg = threadIdx.x / R2, tt = threadIdx.x - (threadIdx.x / R2) * R2;
+      float2 v[16];
 #pragma unroll
-    for (int o = 8; o > 0; o >>= 1) {
-      s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-      s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-      se += __shfl_xor_sync(0xffffffffu, se, o);
+      for (int q = 0; q < 16; ++q)
+        v[q] = R2 * q + R2 - 1 < M || tt + R2 * q < M ? zr[gg * SR + tt + R2 * q] : make_float2(0.f, 0.f);
+      Dft<16, -1>::run(v);
+#pragma unroll
+      for (int q = 0; q < 16; ++q) zb[gg * SR + tt * S1 + q] = v[q];
     }
-    if (t == 0) {
-      double* rs = rowstats + ((size_t)c * HT + py) * 3;
-      rs[0] = (double)s1;
-      rs[1] = (double)s2;
-      rs[2] = (double)se;
+    __syncthreads();
+    // ---- rfft pass 2 (radix 9): Z[t + 16r], then the real post-process with
+    // Z[WH - k] = Z[(16 - t) + 16 (8 - r)]
+    {
+      const int py = (row0 + g + HT - HT / 2) % HT;
+      float2 u[R2];
+#pragma unroll
+      for (int r = 0; r < R2; ++r) {
+        u[r] = zb[g * SR + r * S1 + t];
+        if (r) u[r] = cmul(u[r], rootr[r]);
+      }
+      Dft<R2, -1>::run(u);
+      float2* out = A + ((size_t)c * HT + py) * Wcp;
+      const int mirror = (lane & 16) | ((16 - t) & 15);
+      static_for<R2>([&](auto r_) {
+        constexpr int r = decltype(r_)::value;
+        float2 zm;
+        zm.x = __shfl_sync(0xffffffffu, u[8 - r].x, mirror);
+        zm.y = __shfl_sync(0xffffffffu, u[8 - r].y, mirror);
+        if (t == 0) zm = u[(9 - r) % 9];
+        zm.y = -zm.y;
+        const float2 xe = cscale(cadd(u[r], zm), 0.5f);
+        const float2 xo = mul_i<-1>(cscale(csub(u[r], zm), 0.5f));
+        out[t + 16 * r] = cadd(xe, mul_root<r, 18, -1>(cmul(xo, postj)));
+      });
+      if (t == 0) out[WH] = make_float2(u[0].x - u[0].y, 0.f);
+      for (int k = WH + 1 + t; k < Wcp; k += NT) out[k] = make_float2(0.f, 0.f);
     }
+    __syncthreads();  // zb is read
   }
-  __syncthreads();
-  // ---- rfft pass 1 (radix 16) over m' = tt + 9q, tasks packed as above
-  if (threadIdx.x < ROWS * R2) {
-    const int gg = threadIdx.x / R2, tt = threadIdx.x - (threadIdx.x / R2) * R2;
-    float2 v[16];
-#pragma unroll
-    for (int q = 0; q < 16; ++q) v[q] = zr[gg][IdxPad16::f(tt + q * R2)];
-    Dft<16, -1>::run(v);
-#pragma unroll
-    for (int q = 0; q < 16; ++q) zb[gg][tt * S1 + q] = v[q];
-  }
-  __syncthreads();
-  // ---- rfft pass 2 (radix 9): Z[t + 16r]
-  {
-    float2 u[R2];
-#pragma unroll
-    for (int r = 0; r < R2; ++r) u[r] = cmul(zb[g][r * S1 + t], rootr[r * t]);
-    Dft<R2, -1>::run(u);
-#pragma unroll
-    for (int r = 0; r < R2; ++r) zr[g][IdxPad16::f(t + 16 * r)] = u[r];
-  }
-  __syncthreads();
-  float2* out = A + ((size_t)c * HT + py) * Wcp;
-  for (int k = t; k <= WH; k += NT) {
-    const float2 Zk = zr[g][IdxPad16::f(k == WH ? 0 : k)];
-    const float2 Zm = cconj(zr[g][IdxPad16::f(k == 0 ? 0 : WH - k)]);
-    const float2 xe = cscale(cadd(Zk, Zm), 0.5f);
-    const float2 xo = mul_i<-1>(cscale(csub(Zk, Zm), 0.5f));
-    out[k] = cadd(xe, cmul(post[k], xo));
-  }
-  for (int k = WH + 1 + t; k < Wcp; k += NT) out[k] = make_float2(0.f, 0.f);
 }
 
 // Normalisation constants of utils.py:106-188 from the per-row moments:
