@@ -13,7 +13,6 @@ bool supported_col(int H) {
     case 64:
     case 256:
     case 288:
-    case 512:
 #define X(n) case n:
     LGB_COL_TAB_SIZES(X)
     LGB_COL_REG_SIZES(X)
@@ -93,8 +92,6 @@ int launch_colpass(int H, const void* A, const void* Ip, int h, int Wcp, int n_c
   if (cpi < 1 || y_rows < 1 || y_rows > H || Wcp % kColGroup) return LGB_ERR_INVALID_ARGUMENT;
   if (norm && (H != 288 || norm_w < 2 || norm_w / 2 + 1 > Wcp || norm_stride < 1)) return LGB_ERR_UNSUPPORTED_SIZE;
   switch (H) {
-    case 512:
-      return colpass_fused_t<8, 3>(A, Ip, h, Wcp, n_c, cpi, y_rows, waves, Y, s);
     case 256:
       return colpass_fused_t<16, 2>(A, Ip, h, Wcp, n_c, cpi, y_rows, waves, Y, s);
     case 64:

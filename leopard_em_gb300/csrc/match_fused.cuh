@@ -1,6 +1,6 @@
 // Register-fused column passes of the plain FP32 search.
 //
-// colpass_fused_kernel<R, P>  (H = R^P = 64, 256, 512, one butterfly per thread per pass)
+// colpass_fused_kernel<R, P>  (H = R^P = 64, 256, one butterfly per thread per pass)
 //   The forward FFT's last Stockham pass leaves element j + q*H/R of the
 //   column in thread j, and the inverse FFT's first pass consumes exactly those
 //   elements in the same thread: forward-last -> cross power -> inverse-first
@@ -60,12 +60,6 @@ struct UniformPlan<R, 2> {
   using type = Radices<R, R>;
   static constexpr int N = R * R;
 };
-template <int R>
-struct UniformPlan<R, 3> {
-  using type = Radices<R, R, R>;
-  static constexpr int N = R * R * R;
-};
-
 template <int R, int P>
 struct ColFused {
   using RL = typename UniformPlan<R, P>::type;

@@ -47,7 +47,7 @@ int launch_colpass(int H, const void* A, const void* Ip, int h, int Wcp, int n_c
                    int norm_w = 0);
 // Its lengths in two register passes (match_cols_reg.cuh), one translation unit
 // each so that they compile in parallel.
-#define LGB_COL_REG_SIZES(X) X(576) X(1024) X(2048) X(2880) X(3072) X(3840) X(4096) X(5760)
+#define LGB_COL_REG_SIZES(X) X(512) X(576) X(1024) X(2048) X(2880) X(3072) X(3840) X(4096) X(5760)
 #define X(n)                                                                                                  \
   int launch_colpass_##n(const void* A, const void* Ip, int h, int Wcp, int n_c, int c_per_image, int y_rows, \
                          int waves, void* Y, cudaStream_t s);

@@ -7,8 +7,8 @@
 //   slice / proj_col / proj_row / pad_rfft / colpass                (shared with the search;
 //                            288^2 crops with d = 256: proj_row + pad_rfft fused, the
 //                            normalisation applied by the column pass)
-//   refine_rowpass_kernel    rows y < crop_h only: c2r, valid crop, z = (cc - mean)/std,
-//   (_pair for W = 288)      packed (z, pixel-major flat index) arg-max and max cc per particle
+//   refine_rowpass_pair_kernel  rows y < crop_h only: c2r, valid crop, z = (cc - mean)/std,
+//                            packed (z, pixel-major flat index) arg-max and max cc per particle
 //   refine_commit_kernel     strict '>' against the particle's best so far
 // The filters (per-particle projective filter x CTF stack with B envelope) are
 // built once per call by refine_filters_kernel.
@@ -117,87 +117,14 @@ __device__ __forceinline__ float unord_f(unsigned u) {
 // largest key is the largest z and, among equal z, the first pixel in
 // row-major order and then the first correlogram: the order in which the
 // reference's torch.max over correlograms and then over pixels resolves ties.
-template <int WH, int NT>
-__global__ void __launch_bounds__(NT)
-    refine_rowpass_kernel(const float2* __restrict__ Y, int y_rows, int Wcp, int n_cpp, int c_per_block,
-                          int crop_w, float scale, const float* __restrict__ corr_mean,
-                          const float* __restrict__ corr_std, int crop_h, unsigned long long* __restrict__ slot_key,
-                          unsigned* __restrict__ slot_cc) {
-  constexpr int ZS = IdxPad16::pad(WH) + 2;
-  __shared__ float2 xr[WH + 4];
-  __shared__ float2 z[ZS];
-  // c2r pre-twiddles and FFT twiddles, filled once and reused by every correlogram
-  __shared__ float2 pre[WH];
-  __shared__ float2 tab[FftTable<WH>::SIZE + 1];
-  __shared__ unsigned long long red_key[1];
-  __shared__ unsigned red_cc[1];
-  const int y = blockIdx.x, p = blockIdx.y, t = threadIdx.x;
-  fill_fft_table<WH>(tab, t, NT);
-  for (int k = t; k < WH; k += NT) {
-    float sn, cs;
-    sincospif((float)k / (float)WH, &sn, &cs);
-    pre[k] = make_float2(cs, sn);
-  }
-  unsigned long long best_key = 0ull;
-  unsigned best_cc = 0u;
-  const float* mrow = corr_mean + ((size_t)p * crop_h + y) * crop_w;
-  const float* srow = corr_std + ((size_t)p * crop_h + y) * crop_w;
-  // this CTA's share of the particle's correlograms (blockIdx.z); the slots
-  // combine the shares with atomicMax
-  const int c_begin = blockIdx.z * c_per_block;
-  const int c_end = min(n_cpp, c_begin + c_per_block);
-  for (int c = c_begin; c < c_end; ++c) {
-    const float2* row = Y + (((size_t)p * n_cpp + c) * y_rows + y) * Wcp;
-    for (int k = t; k <= WH; k += NT) xr[k] = row[k];
-    __syncthreads();
-    for (int k = t; k < WH; k += NT) {
-      float2 A = xr[k];
-      float2 B = xr[WH - k];
-      if (k == 0) { A.y = 0.f; B.y = 0.f; }
-      B.y = -B.y;
-      const float2 xo = cmul(csub(A, B), pre[k]);
-      z[IdxPad16::f(k)] = cadd(cadd(A, B), mul_i<1>(xo));
-    }
-    __syncthreads();
-    block_fft_tab<WH, NT, +1, IdxPad16>(z, tab, t);
-    for (int m = t; 2 * m < crop_w; m += NT) {
-      const float2 v = z[IdxPad16::f(m)];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int x = 2 * m + h;
-        if (x >= crop_w) break;
-        const float cc = (h ? v.y : v.x) * scale;
-        const float zz = (cc - mrow[x]) / srow[x];
-        const unsigned flat = (unsigned)((y * crop_w + x) * n_cpp + c);
-        const unsigned long long key = ((unsigned long long)ord_f(zz) << 32) | (unsigned long long)(~flat);
-        best_key = key > best_key ? key : best_key;
-        const unsigned oc = ord_f(cc);
-        best_cc = oc > best_cc ? oc : best_cc;
-      }
-    }
-    __syncthreads();
-  }
-  // block reduction through shared atomics (NT need not be a multiple of 32)
-  if (t == 0) {
-    red_key[0] = 0ull;
-    red_cc[0] = 0u;
-  }
-  __syncthreads();
-  atomicMax(&red_key[0], best_key);
-  atomicMax(&red_cc[0], best_cc);
-  __syncthreads();
-  if (t == 0) {
-    atomicMax(slot_key + p, red_key[0]);
-    atomicMax(slot_cc + p, red_cc[0]);
-  }
-}
-
-// The same row pass for WH = R1*R2 (144 = 16*9) in two register passes, ROWS
-// correlograms of one crop row per CTA (R1 threads each): the c2r
-// pre-twiddle is applied while loading the radix-R1 inputs k = t + R2*q from
-// the staged row; shared transpose M1[t][q]; radix R2 with twiddles w^(r*t)
-// leaves pixel pairs m = t + R1*r in thread t.  Same keys and reduction as
-// refine_rowpass_kernel.
+//
+// c2r of WH = R1*R2 points in two register passes, ROWS correlograms of one
+// crop row per CTA (R1 threads each): the c2r pre-twiddle is applied while
+// loading the radix-R1 inputs k = t + R2*q from the staged row; shared transpose
+// M1[t][q]; radix R2 with twiddles w^(r*t) leaves pixel pairs m = t + R1*r in
+// thread t.  One row per CTA through the generic block transform (16 of 256
+// threads busy) was bound by its barriers: 4 particles of 512 crops, 175
+// correlograms each, 529 -> 203 us.
 template <int R1, int R2, int ROWS>
 __global__ void __launch_bounds__(ROWS* R1, 3)
     refine_rowpass_pair_kernel(const float2* __restrict__ Y, int y_rows, int Wcp, int n_cpp, int c_per_block,
@@ -206,10 +133,10 @@ __global__ void __launch_bounds__(ROWS* R1, 3)
                                unsigned long long* __restrict__ slot_key, unsigned* __restrict__ slot_cc) {
   constexpr int WH = R1 * R2, NT = R1, S1 = R1 + 1, NROOT = (R1 - 1) * (R2 - 1) + 1;
   static_assert(R1 >= R2, "second pass uses every thread of the row");
-  // row strides 9 (mod 16) float2: the first pass packs rows two to a
-  // half-warp, and this stride keeps their loads and stores conflict free
-  constexpr int XS = WH + 1 + ((9 - (WH + 1) % 16) + 16) % 16;
-  constexpr int ZS = R2 * S1 + ((9 - (R2 * S1) % 16) + 16) % 16;
+  // row strides R2 (mod 16) float2: the first pass packs R2 tasks a row densely
+  // onto the lanes, and this stride keeps their loads and stores conflict free
+  constexpr int XS = WH + 1 + ((R2 - (WH + 1) % 16) + 16) % 16;
+  constexpr int ZS = R2 * S1 + ((R2 - (R2 * S1) % 16) + 16) % 16;
   __shared__ float2 xr[ROWS][XS];
   __shared__ float2 zb[ROWS][ZS];
   __shared__ float2 pre[WH];      // exp(+i pi k / WH)
@@ -247,7 +174,7 @@ __global__ void __launch_bounds__(ROWS* R1, 3)
       for (int k = t; k <= WH; k += NT) xr[g][k] = row[k];
     }
     __syncthreads();
-    // first pass: R2 (< R1) DFTs per row, the (row, DFT) tasks packed densely
+    // first pass: R2 (<= R1) DFTs per row, the (row, DFT) tasks packed densely
     // onto the CTA's threads so that whole warps idle instead of lanes
     if (threadIdx.x < ROWS * R2 && cb + (int)threadIdx.x / R2 < c_end) {
       const int gg = threadIdx.x / R2, tt = threadIdx.x - (threadIdx.x / R2) * R2;
@@ -335,12 +262,14 @@ __global__ void refine_init_kernel(int P, float* best_z, float* best_cc, int* be
   slot_cc[p] = 0u;
 }
 
-#define LGB_REFINE_ROW_SIZES(X) X(24) X(32) X(64) X(128) X(144) X(256)
+// W/2 = R1 R2 and the rows per CTA (256 threads; 128 for the longest, whose rows fill shared memory)
+#define LGB_REFINE_ROW_SIZES(X) \
+  X(24, 8, 3, 32) X(32, 8, 4, 32) X(64, 8, 8, 32) X(128, 16, 8, 16) X(144, 16, 9, 16) X(256, 16, 16, 8)
 
 bool supported_refine_row(int W) {
   if (W % 2) return false;
   switch (W / 2) {
-#define X(n) case n:
+#define X(n, r1, r2, rows) case n:
     LGB_REFINE_ROW_SIZES(X)
 #undef X
     return true;
@@ -349,32 +278,14 @@ bool supported_refine_row(int W) {
   }
 }
 
-template <int WH>
+template <int R1, int R2, int ROWS>
 static int refine_rowpass_t(const void* Y, int y_rows, int Wcp, int n_cpp, int P, int crop_h, int crop_w,
                             float scale, const float* mean, const float* std_, unsigned long long* key, unsigned* cc,
                             cudaStream_t s) {
-  if constexpr (WH == 144) {
-    // two register passes (16 x 9), 16 correlograms per step, two steps per CTA
-    constexpr int ROWS = 16;
-    const int per = 2 * ROWS;
-    dim3 grid(crop_h, P, (n_cpp + per - 1) / per);
-    refine_rowpass_pair_kernel<16, 9, ROWS><<<grid, ROWS * 16, 0, s>>>(
-        static_cast<const float2*>(Y), y_rows, Wcp, n_cpp, per, crop_w, scale, mean, std_, crop_h, key, cc);
-    return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
-  }
-  constexpr int NT = row_threads(WH);
-  // split each particle's correlograms until the grid covers ~4 waves of the SMs
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  int split = 1;
-  while (split < n_cpp && crop_h * P * split < 4 * sms) split *= 2;
-  if (split > n_cpp) split = n_cpp;
-  const int per = (n_cpp + split - 1) / split;
-  split = (n_cpp + per - 1) / per;
-  dim3 grid(crop_h, P, split);
-  refine_rowpass_kernel<WH, NT><<<grid, NT, 0, s>>>(static_cast<const float2*>(Y), y_rows, Wcp, n_cpp, per, crop_w,
-                                                    scale, mean, std_, crop_h, key, cc);
+  const int per = 2 * ROWS;  // two steps per CTA
+  dim3 grid(crop_h, P, (n_cpp + per - 1) / per);
+  refine_rowpass_pair_kernel<R1, R2, ROWS><<<grid, ROWS * R1, 0, s>>>(
+      static_cast<const float2*>(Y), y_rows, Wcp, n_cpp, per, crop_w, scale, mean, std_, crop_h, key, cc);
   return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
 }
 
@@ -383,9 +294,9 @@ int launch_refine_rowpass(int W, const void* Y, int y_rows, int Wcp, int n_cpp, 
                           cudaStream_t s) {
   if (W % 2) return LGB_ERR_UNSUPPORTED_SIZE;
   switch (W / 2) {
-#define X(n) \
-  case n:    \
-    return refine_rowpass_t<n>(Y, y_rows, Wcp, n_cpp, P, crop_h, crop_w, scale, mean, std_, key, cc, s);
+#define X(n, r1, r2, rows) \
+  case n:                  \
+    return refine_rowpass_t<r1, r2, rows>(Y, y_rows, Wcp, n_cpp, P, crop_h, crop_w, scale, mean, std_, key, cc, s);
     LGB_REFINE_ROW_SIZES(X)
 #undef X
     default:

@@ -230,7 +230,8 @@ def test_production_configuration_against_oracle():
     [
         # the register column passes: every length, with few and many non-zero rows (the dense
         # first pass where the template reaches it), and a cut micrograph on the padded grid
-        (576, 80, 48, 1), (576, 256, 256, 1), (1024, 64, 32, 1), (1024, 288, 288, 1), (2048, 64, 48, 2),
+        (512, 80, 48, 1), (512, 96, 96, 1), (512, 288, 288, 1), (576, 80, 48, 1), (576, 256, 256, 1),
+        (1024, 64, 32, 1), (1024, 288, 288, 1), (2048, 64, 48, 2),
         (2880, 48, 32, 1), (3072, 64, 64, 1), (3072, 512, 512, 1), (3840, 48, 48, 1), (3840, 512, 512, 1),
         (4096, 64, 64, 3), (4090, 64, 32, 1), (5760, 48, 48, 1), (5701, 64, 64, 1),
     ],

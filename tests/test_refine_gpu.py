@@ -145,3 +145,17 @@ def test_learned_proposals_match_plain_grid_snr_with_fewer_correlations():
     assert zl >= zp
     assert info["correlations_per_particle"] < info["full_grid_correlations"] / 5
     assert info["fallback"] <= info_gn["fallback"]
+
+@pytest.mark.parametrize("n_p,H,d,n_off,D,C,batch", [(2, 48, 32, 37, 1, 1, 40), (1, 64, 48, 9, 4, 1, 7),
+                                                     (2, 128, 96, 7, 3, 1, 5), (1, 256, 128, 5, 2, 2, 3),
+                                                     (1, 512, 192, 4, 2, 1, 3), (1, 288, 256, 35, 1, 1, 32)])
+def test_refine_crop_lengths_against_oracle(n_p, H, d, n_off, D, C, batch):
+    """Every crop row length: uneven correlogram groups, one and several offset
+    batches, one and several row groups per block (the tolerances above)."""
+    kw = _synthetic_refine(n_p, H, d, n_off, D, C, seed=H + n_off)
+    gpu = core_refine_template(**kw, device=torch.device("cuda:0"), batch_size=batch)
+    ref = orr.core_refine_template_cpu(**kw, batch_size=batch)
+    for k in ("angle_idx", "refined_pos_y", "refined_pos_x", "refined_defocus_offset", "refined_pixel_size_offset"):
+        assert torch.equal(gpu[k].to(torch.float64), ref[k].to(torch.float64)), k
+    assert _close(gpu["refined_z_score"].numpy(), ref["refined_z_score"].numpy())
+    assert _close(gpu["refined_cross_correlation"].numpy(), ref["refined_cross_correlation"].numpy())
