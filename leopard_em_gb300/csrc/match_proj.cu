@@ -8,10 +8,17 @@ namespace lgb {
 // Fourier-slice extraction with trilinear interpolation.
 // Output slices[b][r][kx], r in fft order (the reference's ifftshift of the
 // fftshifted slice), DC set to 0, multiplied by -1.
+//
+// What bounds it: the sectors that a warp's gathers touch.  A warp samples a
+// patch of 8 columns x 4 rows: whatever the orientation, its points share
+// volume rows, where 32 columns of one row, as before, lie in up to 32 of them.
+// 300 slices of 256: 128 -> 118 us; 24 slices of 64 a batch: 10.3 -> 6.6.  Loading
+// the 16 B that hold both x neighbours where they are aligned: 130.
 // ---------------------------------------------------------------------------
-__global__ void slice_kernel(const float2* __restrict__ vol, int d, const float* __restrict__ euler, int o0,
-                             const int* __restrict__ o0_dev, const float* __restrict__ rotations,
-                             float2* __restrict__ slices) {
+__global__ void __launch_bounds__(256)
+    slice_kernel(const float2* __restrict__ vol, int d, const float* __restrict__ euler, int o0,
+                 const int* __restrict__ o0_dev, const float* __restrict__ rotations, int tiles,
+                 float2* __restrict__ slices) {
   const int b = blockIdx.y;
   __shared__ float R[9];
   if (threadIdx.x == 0) {
@@ -23,44 +30,44 @@ __global__ void slice_kernel(const float2* __restrict__ vol, int d, const float*
     }
   }
   __syncthreads();
-  const int wc = d / 2 + 1;
-  const int n_el = d * wc;
+  const int wc = d / 2 + 1, half = d / 2;
   const float fd = (float)d;
-  const int half = d / 2;
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n_el; e += gridDim.x * blockDim.x) {
-    const int r = e / wc, kx = e - (e / wc) * wc;
-    const float fy = (float)(r < (d + 1) / 2 ? r : r - d) / fd;
-    const float fx = (float)kx / fd;
-    float X = R[0] * fx + R[1] * fy;
-    float Y = R[3] * fx + R[4] * fy;
-    float Z = R[6] * fx + R[7] * fy;
-    const bool cj = X < 0.f;
-    if (cj) { X = -X; Y = -Y; Z = -Z; }
-    const float cz = Z * fd + (float)half, cy = Y * fd + (float)half, cx = X * fd;
-    float2 val = make_float2(0.f, 0.f);
-    if (cz >= 0.f && cz <= (float)(d - 1) && cy >= 0.f && cy <= (float)(d - 1) && cx >= 0.f &&
-        cx <= (float)(wc - 1)) {
-      const int z0 = (int)floorf(cz), y0 = (int)floorf(cy), x0 = (int)floorf(cx);
-      const float tz = cz - (float)z0, ty = cy - (float)y0, tx = cx - (float)x0;
-      const int z1 = min(z0 + 1, d - 1), y1 = min(y0 + 1, d - 1), x1 = min(x0 + 1, wc - 1);
-      const int zz[2] = {z0, z1}, yy[2] = {y0, y1}, xx[2] = {x0, x1};
-      const float wz[2] = {1.f - tz, tz}, wy[2] = {1.f - ty, ty}, wx[2] = {1.f - tx, tx};
+  // warp -> patch: `tiles` patches cover a strip of four rows
+  const int w = blockIdx.x * 8 + threadIdx.x / 32, lane = threadIdx.x & 31;
+  const int strip = w / tiles;
+  const int r = strip * 4 + lane / 8, kx = (w - strip * tiles) * 8 + lane % 8;
+  if (r >= d || kx >= wc) return;
+  const float fy = (float)(r < (d + 1) / 2 ? r : r - d) / fd;
+  const float fx = (float)kx / fd;
+  float X = R[0] * fx + R[1] * fy;
+  float Y = R[3] * fx + R[4] * fy;
+  float Z = R[6] * fx + R[7] * fy;
+  const bool cj = X < 0.f;
+  if (cj) { X = -X; Y = -Y; Z = -Z; }
+  const float cz = Z * fd + (float)half, cy = Y * fd + (float)half, cx = X * fd;
+  float2 val = make_float2(0.f, 0.f);
+  if (cz >= 0.f && cz <= (float)(d - 1) && cy >= 0.f && cy <= (float)(d - 1) && cx >= 0.f && cx <= (float)(wc - 1)) {
+    const int z0 = (int)floorf(cz), y0 = (int)floorf(cy), x0 = (int)floorf(cx);
+    const float tz = cz - (float)z0, ty = cy - (float)y0, tx = cx - (float)x0;
+    const int z1 = min(z0 + 1, d - 1), y1 = min(y0 + 1, d - 1), x1 = min(x0 + 1, wc - 1);
+    const int zz[2] = {z0, z1}, yy[2] = {y0, y1}, xx[2] = {x0, x1};
+    const float wz[2] = {1.f - tz, tz}, wy[2] = {1.f - ty, ty}, wx[2] = {1.f - tx, tx};
 #pragma unroll
-      for (int a = 0; a < 2; ++a)
+    for (int a = 0; a < 2; ++a)
 #pragma unroll
-        for (int bb = 0; bb < 2; ++bb)
+      for (int bb = 0; bb < 2; ++bb)
 #pragma unroll
-          for (int cc = 0; cc < 2; ++cc) {
-            const float w = wz[a] * wy[bb] * wx[cc];
-            const float2 s = __ldg(vol + ((size_t)zz[a] * d + yy[bb]) * wc + xx[cc]);
-            val.x = fmaf(s.x, w, val.x);
-            val.y = fmaf(s.y, w, val.y);
-          }
-    }
-    if (cj) val.y = -val.y;
-    if (e == 0) val = make_float2(0.f, 0.f);
-    slices[(size_t)b * n_el + e] = make_float2(-val.x, -val.y);
+        for (int cc = 0; cc < 2; ++cc) {
+          const float wt = wz[a] * wy[bb] * wx[cc];
+          // d <= 512: the volume's elements count in 32 bits
+          const float2 s = __ldg(vol + ((unsigned)(zz[a] * d + yy[bb]) * (unsigned)wc + (unsigned)xx[cc]));
+          val.x = fmaf(s.x, wt, val.x);
+          val.y = fmaf(s.y, wt, val.y);
+        }
   }
+  if (cj) val.y = -val.y;
+  if (r == 0 && kx == 0) val = make_float2(0.f, 0.f);
+  slices[((size_t)b * d + r) * wc + kx] = make_float2(-val.x, -val.y);
 }
 
 
@@ -79,9 +86,9 @@ bool supported_template(int h) {
 
 int launch_slice(const void* vol, int d, const float* euler, int o0, const int* o0_dev, int nb,
                  const float* rotations, void* slices, cudaStream_t s) {
-  const int n_el = d * (d / 2 + 1);
-  dim3 grid((n_el + 255) / 256, nb);
-  slice_kernel<<<grid, 256, 0, s>>>(static_cast<const float2*>(vol), d, euler, o0, o0_dev, rotations,
+  const int tiles = (d / 2 + 1 + 7) / 8, patches = tiles * ((d + 3) / 4);
+  dim3 grid((patches + 7) / 8, nb);
+  slice_kernel<<<grid, 256, 0, s>>>(static_cast<const float2*>(vol), d, euler, o0, o0_dev, rotations, tiles,
                                     static_cast<float2*>(slices));
   return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
 }
