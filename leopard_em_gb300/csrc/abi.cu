@@ -20,14 +20,6 @@ __global__ void init_stats_kernel(long long n, float* mip, int* best, double* s1
   }
 }
 
-__global__ void repack_image_kernel(const float2* __restrict__ src, int H, int wc, int wcp, float2* __restrict__ dst) {
-  const long long n = (long long)H * wcp;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const int y = (int)(i / wcp), k = (int)(i % wcp);
-    dst[i] = k < wc ? src[(size_t)y * wc + k] : make_float2(0.f, 0.f);
-  }
-}
-
 __global__ void filters_kernel(const float* __restrict__ ctf, const float* __restrict__ wf, long long n_filters,
                                int plane, float* __restrict__ out) {
   const long long n = n_filters * plane;
@@ -210,7 +202,7 @@ static int run_batch(const SearchArgs& a, int o0, const int* o0_dev, int nb, boo
   }
   {
     StageScope sc(LGB_STAGE_COLPASS, s, prof);
-    if ((st = launch_colpass(H, A, ip, h, L.wcp, n_c, n_c, y_rows, p->col_waves, Y, s))) return st;
+    if ((st = launch_colpass(H, A, ip, L.wcp, h, L.wcp, n_c, n_c, y_rows, p->col_waves, Y, s))) return st;
   }
   {
     StageScope sc(LGB_STAGE_ROWPASS, s, prof);
@@ -315,7 +307,7 @@ int lgb_match_prepare_image(const lgb_match_problem* p, const void* image_dft, v
   const MatchLayout L = layout_of(p);
   if (workspace_bytes < L.total) return LGB_ERR_WORKSPACE_TOO_SMALL;
   float2* ip = reinterpret_cast<float2*>(static_cast<char*>(workspace) + L.ip);
-  repack_image_kernel<<<grid_for((long long)p->image_h * L.wcp), 256, 0, (cudaStream_t)stream>>>(
+  repack_rows_kernel<<<(p->image_h + 7) / 8, 256, 0, (cudaStream_t)stream>>>(
       static_cast<const float2*>(image_dft), p->image_h, L.wc_img, L.wcp, ip);
   return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
 }

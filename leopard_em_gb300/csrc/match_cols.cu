@@ -39,7 +39,7 @@ static int colpass_split(int groups, int n_c, int waves, int* per) {
 }
 
 template <int HN>
-static int colpass_tab_t(const void* A, const void* Ip, int h, int Wcp, int n_c, int cpi, int y_rows, int waves,
+static int colpass_tab_t(const void* A, const void* Ip, int ips, int h, int Wcp, int n_c, int cpi, int y_rows, int waves,
                          void* Y, cudaStream_t s) {
   using CT = ColTab<HN>;
   if (cudaFuncSetAttribute(colpass_tab_kernel<HN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CT::SMEM) !=
@@ -49,13 +49,13 @@ static int colpass_tab_t(const void* A, const void* Ip, int h, int Wcp, int n_c,
   const int groups = (Wcp + CT::G - 1) / CT::G;
   const int split = colpass_split(groups, n_c, waves, &per);
   colpass_tab_kernel<HN><<<dim3(groups, split), CT::G * CT::NT, CT::SMEM, s>>>(
-      static_cast<const float2*>(A), static_cast<const float2*>(Ip), h, Wcp, n_c, per, cpi, y_rows,
+      static_cast<const float2*>(A), static_cast<const float2*>(Ip), ips, h, Wcp, n_c, per, cpi, y_rows,
       static_cast<float2*>(Y));
   return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
 }
 
 template <int R, int P>
-static int colpass_fused_t(const void* A, const void* Ip, int h, int Wcp, int n_c, int cpi, int y_rows, int waves,
+static int colpass_fused_t(const void* A, const void* Ip, int ips, int h, int Wcp, int n_c, int cpi, int y_rows, int waves,
                            void* Y, cudaStream_t s) {
   using CF = ColFused<R, P>;
   if (cudaFuncSetAttribute(colpass_fused_kernel<R, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CF::SMEM) !=
@@ -66,46 +66,47 @@ static int colpass_fused_t(const void* A, const void* Ip, int h, int Wcp, int n_
   const int split = colpass_split(groups, n_c, waves, &per);
   dim3 grid(groups, split);
   colpass_fused_kernel<R, P><<<grid, CF::THREADS, CF::SMEM, s>>>(
-      static_cast<const float2*>(A), static_cast<const float2*>(Ip), h, Wcp, n_c, per, cpi, y_rows,
+      static_cast<const float2*>(A), static_cast<const float2*>(Ip), ips, h, Wcp, n_c, per, cpi, y_rows,
       static_cast<float2*>(Y));
   return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
 }
 
 template <int R1, int R2>
-static int colpass_pair_t(const void* A, const void* Ip, int h, int Wcp, int n_c, int cpi, int y_rows, int waves,
+static int colpass_pair_t(const void* A, const void* Ip, int ips, int h, int Wcp, int n_c, int cpi, int y_rows, int waves,
                           void* Y, cudaStream_t s, const float2* norm, int norm_stride, int norm_w) {
   using CP = ColPair<R1, R2>;
-  if (cudaFuncSetAttribute(colpass_pair_kernel<R1, R2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CP::SMEM) !=
-      cudaSuccess)
+  // valid crops of refinement templates need a few rows only
+  auto* kernel = y_rows <= 2 * R2 ? colpass_pair_kernel<R1, R2, 2> : colpass_pair_kernel<R1, R2, R1>;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CP::SMEM) != cudaSuccess)
     return LGB_ERR_CUDA;
   int per = 1;
   const int groups = (Wcp + CP::G - 1) / CP::G;
   const int split = colpass_split(groups, n_c, waves, &per);
-  colpass_pair_kernel<R1, R2><<<dim3(groups, split), CP::THREADS, CP::SMEM, s>>>(
-      static_cast<const float2*>(A), static_cast<const float2*>(Ip), h, Wcp, n_c, per, cpi, y_rows,
+  kernel<<<dim3(groups, split), CP::THREADS, CP::SMEM, s>>>(
+      static_cast<const float2*>(A), static_cast<const float2*>(Ip), ips, h, Wcp, n_c, per, cpi, y_rows,
       static_cast<float2*>(Y), norm, norm_stride, norm_w);
   return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
 }
 
-int launch_colpass(int H, const void* A, const void* Ip, int h, int Wcp, int n_c, int cpi, int y_rows, int waves,
+int launch_colpass(int H, const void* A, const void* Ip, int ips, int h, int Wcp, int n_c, int cpi, int y_rows, int waves,
                    void* Y, cudaStream_t s, const float2* norm, int norm_stride, int norm_w) {
-  if (cpi < 1 || y_rows < 1 || y_rows > H || Wcp % kColGroup) return LGB_ERR_INVALID_ARGUMENT;
+  if (cpi < 1 || ips < Wcp - 3 || y_rows < 1 || y_rows > H || Wcp % kColGroup) return LGB_ERR_INVALID_ARGUMENT;
   if (norm && (H != 288 || norm_w < 2 || norm_w / 2 + 1 > Wcp || norm_stride < 1)) return LGB_ERR_UNSUPPORTED_SIZE;
   switch (H) {
     case 256:
-      return colpass_fused_t<16, 2>(A, Ip, h, Wcp, n_c, cpi, y_rows, waves, Y, s);
+      return colpass_fused_t<16, 2>(A, Ip, ips, h, Wcp, n_c, cpi, y_rows, waves, Y, s);
     case 64:
-      return colpass_fused_t<8, 2>(A, Ip, h, Wcp, n_c, cpi, y_rows, waves, Y, s);
+      return colpass_fused_t<8, 2>(A, Ip, ips, h, Wcp, n_c, cpi, y_rows, waves, Y, s);
     case 288:
-      return colpass_pair_t<16, 18>(A, Ip, h, Wcp, n_c, cpi, y_rows, waves, Y, s, norm, norm_stride, norm_w);
+      return colpass_pair_t<16, 18>(A, Ip, ips, h, Wcp, n_c, cpi, y_rows, waves, Y, s, norm, norm_stride, norm_w);
 #define X(n) \
   case n:    \
-    return launch_colpass_##n(A, Ip, h, Wcp, n_c, cpi, y_rows, waves, Y, s);
+    return launch_colpass_##n(A, Ip, ips, h, Wcp, n_c, cpi, y_rows, waves, Y, s);
     LGB_COL_REG_SIZES(X)
 #undef X
 #define X(n) \
   case n:    \
-    return colpass_tab_t<n>(A, Ip, h, Wcp, n_c, cpi, y_rows, waves, Y, s);
+    return colpass_tab_t<n>(A, Ip, ips, h, Wcp, n_c, cpi, y_rows, waves, Y, s);
     LGB_COL_TAB_SIZES(X)
 #undef X
     default:

@@ -100,7 +100,7 @@ __device__ __forceinline__ void apply_roots(float2* v, const float2* tab, int st
 
 template <class C, bool SPARSE>
 __global__ void __launch_bounds__(C::THREADS, C::MINB)
-    colpass_reg_kernel(const float2* __restrict__ A, const float2* __restrict__ Ip, int h, int Wcp, int n_c,
+    colpass_reg_kernel(const float2* __restrict__ A, const float2* __restrict__ Ip, int ips, int h, int Wcp, int n_c,
                        int c_per_block, int c_per_image, int y_rows, float2* __restrict__ Y) {
   constexpr int R1 = C::R1, R2 = C::R2, N = C::N, G = C::G, NT = C::NT, D1 = C::D1, S1 = C::S1, S2 = C::S2;
   constexpr int CH = C::CH;
@@ -138,11 +138,11 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
   int image = c_begin / c_per_image;
   float2 first[R2];
   {
-    const float2* ip = Ip + (size_t)image * N * Wcp + kx;
+    const float2* ip = Ip + (size_t)image * N * ips + kx;
 #pragma unroll
     for (int s = 0; s < R2; ++s) {
       const int row = t + R1 * DftNT<C::R2A, C::R2B, -1>::out(s);
-      first[s] = (col_ok && act2 && c_begin < c_end) ? __ldg(ip + (size_t)row * Wcp) : make_float2(0.f, 0.f);
+      first[s] = (kx < ips && act2 && c_begin < c_end) ? __ldg(ip + (size_t)row * ips) : make_float2(0.f, 0.f);
     }
   }
   if constexpr (C::TWO) {
@@ -178,14 +178,14 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
     // ---- this image's columns -> tensor memory, in the slot order of P
     if (c / c_per_image != image) {
       image = c / c_per_image;
-      const float2* ip = Ip + (size_t)image * N * Wcp + kx;
+      const float2* ip = Ip + (size_t)image * N * ips + kx;
 #pragma unroll
       for (int s0 = 0; s0 < R2; s0 += CH) {
         float2 w[CH];
 #pragma unroll
         for (int i = 0; i < CH; ++i) {
           const int row = t + R1 * DftNT<C::R2A, C::R2B, -1>::out(s0 + i);
-          w[i] = (col_ok && act2) ? __ldg(ip + (size_t)row * Wcp) : make_float2(0.f, 0.f);
+          w[i] = (kx < ips && act2) ? __ldg(ip + (size_t)row * ips) : make_float2(0.f, 0.f);
         }
         tmem_put<CH>(tm + 2 * s0, w);
       }
@@ -302,7 +302,7 @@ inline int colpass_per_block(int groups, int n_c, int slots, int waves) {
 }
 
 template <class C, bool SPARSE>
-int colpass_reg_launch(const void* A, const void* Ip, int h, int Wcp, int n_c, int cpi, int y_rows, int waves, void* Y,
+int colpass_reg_launch(const void* A, const void* Ip, int ips, int h, int Wcp, int n_c, int cpi, int y_rows, int waves, void* Y,
                        cudaStream_t s) {
   if (cudaFuncSetAttribute(colpass_reg_kernel<C, SPARSE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)C::SMEM) != cudaSuccess)
@@ -313,7 +313,7 @@ int colpass_reg_launch(const void* A, const void* Ip, int h, int Wcp, int n_c, i
   const int groups = (Wcp + C::G - 1) / C::G;
   const int per = colpass_per_block(groups, n_c, sms * C::MINB, waves);
   colpass_reg_kernel<C, SPARSE><<<dim3(groups, (n_c + per - 1) / per), C::THREADS, C::SMEM, s>>>(
-      static_cast<const float2*>(A), static_cast<const float2*>(Ip), h, Wcp, n_c, per, cpi, y_rows,
+      static_cast<const float2*>(A), static_cast<const float2*>(Ip), ips, h, Wcp, n_c, per, cpi, y_rows,
       static_cast<float2*>(Y));
   return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
 }
@@ -322,13 +322,13 @@ int colpass_reg_launch(const void* A, const void* Ip, int h, int Wcp, int n_c, i
 // at most kMaxTemplate rows, so the long columns need no other.
 constexpr int kMaxTemplate = 512;
 template <class C>
-int colpass_reg_t(const void* A, const void* Ip, int h, int Wcp, int n_c, int cpi, int y_rows, int waves, void* Y,
+int colpass_reg_t(const void* A, const void* Ip, int ips, int h, int Wcp, int n_c, int cpi, int y_rows, int waves, void* Y,
                   cudaStream_t s) {
   if (h > kMaxTemplate) return LGB_ERR_UNSUPPORTED_SIZE;
   if constexpr (C::R1B * C::R2 < kMaxTemplate) {
-    if (h > C::R1B * C::R2) return colpass_reg_launch<C, false>(A, Ip, h, Wcp, n_c, cpi, y_rows, waves, Y, s);
+    if (h > C::R1B * C::R2) return colpass_reg_launch<C, false>(A, Ip, ips, h, Wcp, n_c, cpi, y_rows, waves, Y, s);
   }
-  return colpass_reg_launch<C, true>(A, Ip, h, Wcp, n_c, cpi, y_rows, waves, Y, s);
+  return colpass_reg_launch<C, true>(A, Ip, ips, h, Wcp, n_c, cpi, y_rows, waves, Y, s);
 }
 
 }  // namespace lgb

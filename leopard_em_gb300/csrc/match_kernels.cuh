@@ -32,6 +32,24 @@ constexpr int kColGroup = 4;  // columns per colpass CTA: 4 x 8 B = one 32 B sec
 
 __host__ __device__ inline int pad4(int n) { return (n + 3) & ~3; }
 
+// Spectrum rows of wc columns -> rows of wcp, zero filled: one warp per row (64-bit
+// divisions per element held the flat form to 3.0 TB/s; this 7.4, partly L2, at 86k rows of 145).
+static __global__ void __launch_bounds__(256)
+    repack_rows_kernel(const float2* __restrict__ src, long long rows, int wc, int wcp, float2* __restrict__ dst) {
+  const long long row = blockIdx.x * 8LL + threadIdx.x / 32;
+  if (row >= rows) return;
+  const float2* s = src + row * wc;
+  float2* d = dst + row * wcp;
+  for (int k = threadIdx.x & 31; k < wcp; k += 256) {  // eight loads in flight
+    float2 v[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = k + 32 * q < wc ? __ldg(s + k + 32 * q) : make_float2(0.f, 0.f);
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (k + 32 * q < wcp) d[k + 32 * q] = v[q];
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Euler (ZYZ, degrees) -> R = Rz(phi) Ry(theta) Rz(psi), in FP64.
 // ---------------------------------------------------------------------------
@@ -524,8 +542,9 @@ __global__ void __launch_bounds__(ROWS * 16, 48 / ROWS)
 
 // Normalisation constants of utils.py:106-188 from the per-row moments:
 // returns edge mean e and scale s such that normalised = (p - e) * s.
-// Called by all 32 lanes of warp 0 (the launcher guarantees a full warp).
-__device__ inline void projection_norm_constants(const double* rs, int h, int H, int W, float* e_out,
+// Called by all 32 lanes of warp 0 (the launcher guarantees a full warp);
+// lane 0 gets the constants and, returned, the projection's sum.
+__device__ inline double projection_norm_constants(const double* rs, int h, int H, int W, float* e_out,
                                                  float* s_out) {
   // warp 0 reduces h rows
   double s1 = 0, s2 = 0, se = 0;
@@ -554,6 +573,7 @@ __device__ inline void projection_norm_constants(const double* rs, int h, int H,
     *e_out = (float)e;
     *s_out = (float)(sqrt((double)H * (double)W) / sqrt(var));
   }
+  return s1;
 }
 
 // ---------------------------------------------------------------------------

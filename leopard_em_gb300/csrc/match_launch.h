@@ -30,27 +30,33 @@ bool supported_proj_row_rfft(int h, int W);
 int launch_proj_row_rfft(int h, int W, const void* T, int n_c, double* rowstats, int Wcp, void* A, cudaStream_t s);
 // Per-correlogram normalisation constants (e, s) from the row moments, stored
 // as a float2 over rowstats[c][0][0].
-int launch_norm_constants(double* rowstats, int n_c, int h, int norm_h, int norm_w, cudaStream_t s);
+// offset (or null): image c's DC bin (dc[c * dc_stride]) times the normalised
+// projection's, times scale.
+int launch_norm_constants(double* rowstats, int n_c, int h, int norm_h, int norm_w, cudaStream_t s,
+                          const float2* dc = nullptr, size_t dc_stride = 0, float scale = 0.f,
+                          float* offset = nullptr);
 // Projections normalised for a norm_h x norm_w micrograph (utils.py:106-188),
 // rfft'd at length W (W >= norm_w: zero padding beyond the micrograph).
+// norm_ready: rowstats already holds the constants of launch_norm_constants.
 int launch_pad_rfft(int W, const float* proj, const double* rowstats, int h, int norm_h, int norm_w, int Wcp,
-                    int n_c, void* A, cudaStream_t s);
-// Ip holds one padded spectrum per image; correlogram c uses image c / c_per_image.
+                    int n_c, void* A, cudaStream_t s, bool norm_ready = false);
+// Ip holds one spectrum per image, H rows of ips columns (W/2 + 1 <= ips <= Wcp,
+// Wcp = W/2 + 1 rounded up to 4); correlogram c uses image c / c_per_image.
 // Only rows y < y_rows of each inverse column transform are stored (Y is [n_c][y_rows][Wcp]).
 // waves: the correlogram range is split until the grid covers about waves x
 // the SM count (0 = 4).
 // norm (H = 288 only; null otherwise): A holds un-normalised row spectra of
 // length norm_w rows and correlogram c is normalised on load as
 // s (A - e U[kx]), (e, s) = norm[c * norm_stride], U[k] = sum_{x < h} exp(-2 pi i k x / norm_w).
-int launch_colpass(int H, const void* A, const void* Ip, int h, int Wcp, int n_c, int c_per_image, int y_rows,
+int launch_colpass(int H, const void* A, const void* Ip, int ips, int h, int Wcp, int n_c, int c_per_image, int y_rows,
                    int waves, void* Y, cudaStream_t s, const float2* norm = nullptr, int norm_stride = 0,
                    int norm_w = 0);
 // Its lengths in two register passes (match_cols_reg.cuh), one translation unit
 // each so that they compile in parallel.
 #define LGB_COL_REG_SIZES(X) X(512) X(576) X(1024) X(2048) X(2880) X(3072) X(3840) X(4096) X(5760)
 #define X(n)                                                                                                  \
-  int launch_colpass_##n(const void* A, const void* Ip, int h, int Wcp, int n_c, int c_per_image, int y_rows, \
-                         int waves, void* Y, cudaStream_t s);
+  int launch_colpass_##n(const void* A, const void* Ip, int ips, int h, int Wcp, int n_c, int c_per_image,    \
+                         int y_rows, int waves, void* Y, cudaStream_t s);
 LGB_COL_REG_SIZES(X)
 #undef X
 // Rows y < y_rows of the H x W correlograms (Y is [n_c][y_rows][Wcp]); global

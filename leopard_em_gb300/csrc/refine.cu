@@ -359,25 +359,9 @@ static RefineLayout refine_layout(const lgb_refine_problem* p) {
   return L;
 }
 
-__global__ void repack_stack_kernel(const float2* __restrict__ src, long long rows, int wc, int wcp,
-                                    float2* __restrict__ dst) {
-  const long long n = rows * wcp;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const long long y = i / wcp;
-    const int k = (int)(i % wcp);
-    dst[i] = k < wc ? src[y * wc + k] : make_float2(0.f, 0.f);
-  }
-}
-
 static double electron_wavelength_angstrom(double kv) {
   const double v = kv * 1e3, h = 6.62607015e-34, m0 = 9.1093837015e-31, e = 1.602176634e-19, c = 299792458.0;
   return h / sqrt(2 * m0 * e * v * (1 + e * v / (2 * m0 * c * c))) * 1e10;
-}
-
-static int grid256(long long n) {
-  long long g = (n + 255) / 256;
-  if (g > 65535LL * 16) g = 65535LL * 16;
-  return (int)(g < 1 ? 1 : g);
 }
 
 }  // namespace lgb
@@ -434,7 +418,7 @@ int lgb_refine_search(const lgb_refine_problem* p, const lgb_ctf_params* ctf, co
   const int P = p->n_particles, H = p->image_h, W = p->image_w, d = p->template_size;
   const int C = p->n_pixel_sizes, D = p->n_defocus;
 
-  repack_stack_kernel<<<grid256((long long)P * H * L.wcp), 256, 0, s>>>(
+  repack_rows_kernel<<<(unsigned)(((long long)P * H + 7) / 8), 256, 0, s>>>(
       static_cast<const float2*>(particle_stack_dft), (long long)P * H, W / 2 + 1, L.wcp, ip);
   const double lambda = electron_wavelength_angstrom(ctf->voltage_kv), amp = ctf->amplitude_contrast;
   FilterTurns turns;
@@ -486,7 +470,7 @@ int lgb_refine_search(const lgb_refine_problem* p, const lgb_ctf_params* ctf, co
       {
         StageScope sc(LGB_STAGE_COLPASS, s, prof);
         // (e, s) of correlogram c: float2 at rowstats[c][0][0], d * 3 doubles apart
-        if ((st = launch_colpass(H, A, ip, d, L.wcp, n_c, n_cpp, L.crop_h, 0, Y, s,
+        if ((st = launch_colpass(H, A, ip, L.wcp, d, L.wcp, n_c, n_cpp, L.crop_h, 0, Y, s,
                                  reinterpret_cast<const float2*>(rowstats), d * 3, W)))
           return st;
       }
@@ -501,7 +485,7 @@ int lgb_refine_search(const lgb_refine_problem* p, const lgb_ctf_params* ctf, co
       }
       {
         StageScope sc(LGB_STAGE_COLPASS, s, prof);
-        if ((st = launch_colpass(H, A, ip, d, L.wcp, n_c, n_cpp, L.crop_h, 0, Y, s))) return st;
+        if ((st = launch_colpass(H, A, ip, L.wcp, d, L.wcp, n_c, n_cpp, L.crop_h, 0, Y, s))) return st;
       }
     }
     {

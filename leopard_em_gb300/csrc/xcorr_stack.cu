@@ -14,38 +14,6 @@
 
 namespace lgb {
 
-__global__ void repack_stack_kernel(const float2* __restrict__ src, long long n_particles, int H, int wc, int wcp,
-                                    float2* __restrict__ dst) {
-  const long long n = n_particles * H * wcp;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const long long row = i / wcp;
-    const int k = (int)(i - row * wcp);
-    dst[i] = k < wc ? src[row * wc + k] : make_float2(0.f, 0.f);
-  }
-}
-
-// one warp per particle: offset[p] = Re(I00 * conj(P00)) * scale
-__global__ void dc_offset_kernel(int n_particles, int H, int d, int wcp, const float2* __restrict__ Ip,
-                                 const float2* __restrict__ A, float scale, float* __restrict__ offset) {
-  const int p = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-  const int lane = threadIdx.x & 31;
-  if (p >= n_particles) return;
-  double pr = 0.0, pi = 0.0;
-  for (int y = lane; y < d; y += 32) {
-    const float2 a = A[((size_t)p * d + y) * wcp];
-    pr += a.x;
-    pi += a.y;
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    pr += __shfl_down_sync(0xffffffffu, pr, o);
-    pi += __shfl_down_sync(0xffffffffu, pi, o);
-  }
-  if (lane == 0) {
-    const float2 I = Ip[(size_t)p * H * wcp];
-    offset[p] = (float)(((double)I.x * pr + (double)I.y * pi) * (double)scale);
-  }
-}
-
 // row y of particle p: c2r of length W = 2*WH, scale, DC term, crop
 template <int WH, int NT>
 __global__ void __launch_bounds__(NT) rowstore_kernel(const float2* __restrict__ Y, int y_rows, int Wcp, float scale,
@@ -120,7 +88,7 @@ static int launch_rowstore(int W, const void* Y, int y_rows, int Wcp, int P, flo
 }
 
 struct XcorrLayout {
-  size_t ip, slices, t, proj, rowstats, a, y, off, total;
+  size_t slices, t, proj, rowstats, a, y, off, total;
   int wc, wcp, wc_t, out_h, out_w;
 };
 
@@ -134,7 +102,6 @@ static XcorrLayout xcorr_layout(int G, int H, int W, int d, int mode) {
   L.out_h = mode == 0 ? H - d + 1 : H;
   L.out_w = mode == 0 ? W - d + 1 : W;
   size_t off = 0;
-  L.ip = off; off += al256((size_t)G * H * L.wcp * sizeof(float2));
   L.slices = off; off += al256((size_t)G * d * L.wc_t * sizeof(float2));
   L.t = off; off += al256((size_t)G * d * L.wc_t * sizeof(float2));
   L.proj = off; off += al256((size_t)G * d * d * sizeof(float));
@@ -177,7 +144,6 @@ int lgb_xcorr_stack(int n_particles, int group, int H, int W, int d, int mode, c
   if (workspace_bytes < L.total) return LGB_ERR_WORKSPACE_TOO_SMALL;
   cudaStream_t s = (cudaStream_t)stream;
   char* ws = static_cast<char*>(workspace);
-  float2* ip = reinterpret_cast<float2*>(ws + L.ip);
   void* A = ws + L.a;
   void* Y = ws + L.y;
   float* off = reinterpret_cast<float*>(ws + L.off);
@@ -186,26 +152,32 @@ int lgb_xcorr_stack(int n_particles, int group, int H, int W, int d, int mode, c
   for (int p0 = 0; p0 < n_particles; p0 += group) {
     const int G = n_particles - p0 < group ? n_particles - p0 : group;
     const float2* src = static_cast<const float2*>(particle_dft) + (size_t)p0 * H * L.wc;
-    const long long n = (long long)G * H * L.wcp;
-    long long blocks = (n + 255) / 256;
-    if (blocks > 65535LL * 8) blocks = 65535LL * 8;
-    repack_stack_kernel<<<(int)blocks, 256, 0, s>>>(src, G, H, L.wc, L.wcp, ip);
-    if (cudaGetLastError() != cudaSuccess) return LGB_ERR_CUDA;
     if ((st = launch_slice(template_dft, d, nullptr, 0, nullptr, G, rotations + (size_t)p0 * 9, ws + L.slices, s)))
       return st;
     // per particle one slice (nb = 1) and one filter (n_cd = 1): c = p
     if ((st = launch_proj_col(d, ws + L.slices, projective_filters + (size_t)p0 * d * L.wc_t, 1, 1, G, ws + L.t, s)))
       return st;
-    if ((st = launch_proj_row(d, ws + L.t, G, reinterpret_cast<float*>(ws + L.proj),
-                              reinterpret_cast<double*>(ws + L.rowstats), s)))
+    double* rowstats = reinterpret_cast<double*>(ws + L.rowstats);
+    float* proj = reinterpret_cast<float*>(ws + L.proj);
+    // 288 crops of a 256 template: the projection rows and their padded rfft in
+    // one kernel, the normalisation applied by the column pass (as in the refinement)
+    const bool fused = supported_proj_row_rfft(d, W) && H == 288;
+    if (fused)
+      st = launch_proj_row_rfft(d, W, ws + L.t, G, rowstats, L.wcp, A, s);
+    else
+      st = launch_proj_row(d, ws + L.t, G, proj, rowstats, s);
+    if (st) return st;
+    if ((st = launch_norm_constants(rowstats, G, d, H, W, s, src, (size_t)H * L.wc, scale, off))) return st;
+    const float2* norm = nullptr;
+    if (fused)
+      norm = reinterpret_cast<const float2*>(rowstats);  // (e, s) of particle p, d * 3 doubles apart
+    else if ((st = launch_pad_rfft(W, proj, rowstats, d, H, W, L.wcp, G, A, s, true)))
       return st;
-    if ((st = launch_pad_rfft(W, reinterpret_cast<float*>(ws + L.proj), reinterpret_cast<double*>(ws + L.rowstats), d,
-                              H, W, L.wcp, G, A, s)))
+    // correlogram p against particle image p (one image per correlogram, read
+    // once: straight from the caller's rows, whose misaligned sectors cost less
+    // than the 27 us of a padded copy at 300 crops of 288^2)
+    if ((st = launch_colpass(H, A, src, L.wc, d, L.wcp, G, 1, L.out_h, 0, Y, s, norm, norm ? d * 3 : 0, norm ? W : 0)))
       return st;
-    // correlogram p against particle image p (one image per correlogram)
-    if ((st = launch_colpass(H, A, ip, d, L.wcp, G, 1, L.out_h, 0, Y, s))) return st;
-    dc_offset_kernel<<<(G + 7) / 8, 256, 0, s>>>(G, H, d, L.wcp, ip, static_cast<const float2*>(A), scale, off);
-    if (cudaGetLastError() != cudaSuccess) return LGB_ERR_CUDA;
     if ((st = launch_rowstore(W, Y, L.out_h, L.wcp, G, scale, off, L.out_w,
                               out + (size_t)p0 * L.out_h * L.out_w, s)))
       return st;

@@ -76,6 +76,14 @@ def test_device_argument_errors():
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("H,W,d,mode", [(64, 64, 48, "valid"), (128, 128, 96, "same"), (256, 256, 192, "valid"),
+                                        (288, 288, 256, "same"), (288, 288, 64, "same")])
+def test_device_reads_the_particles_own_rows(H, W, d, mode):
+    """Images of W/2 + 1 columns read in place by the short column passes; projections normalised there or before."""
+    test_device_matches_oracle_register_column_lengths(H, W, d, mode)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("H,W,d,mode", [(576, 80, 48, "same"), (1024, 64, 32, "valid"), (2048, 48, 48, "same")])
 def test_device_matches_oracle_register_column_lengths(H, W, d, mode):
     """The register column passes with another image for each correlogram."""
