@@ -268,6 +268,23 @@ int lgb_refine_search(const lgb_refine_problem* problem, const lgb_ctf_params* c
                       int* best_flat, int* best_offset_begin, int* best_batch_len, void* workspace,
                       size_t workspace_bytes, void* stream);
 
+/* What the host needs of lgb_refine_search's results, in one buffer (replaces
+ * core_refine_template.py:503-551 up to the Euler angles).  raw (device): best_z,
+ * best_cc, best_flat, best_offset_begin, best_batch_len, N words each.  packed
+ * (device) gets 13 words a particle: z, cc, y, x, angle index, defocus offset,
+ * pixel-size offset, the offset's and the particle's three angles. */
+int lgb_refine_collect(int n_particles, int crop_w, int n_pixel_sizes, int n_defocus, const void* raw,
+                       const float* euler_angles, const float* euler_offsets, const float* defocus_offsets,
+                       const float* pixel_size_offsets, void* packed, void* stream);
+
+/* Host side: packed -> result arrays (all host).  Angles of R(offset) @
+ * R(particle) in FP64, wrapped as core_refine_template.py:180-191; positions relative to
+ * the crop's middle.  euler_angles: the particles' angles in FP64, or null to
+ * take the packed ones. */
+int lgb_refine_decode(int n_particles, int crop_h, int crop_w, const void* packed, const double* euler_angles,
+                      float* cc, float* z, float* angles, float* defocus_offset, float* pixel_size_offset,
+                      long long* pos_y, long long* pos_x, long long* angle_idx);
+
 /* Precision form of lgb_match_search (mode 1: BF16 hi + lo, mode 2: FP16 hi +
  * lo operands): the inverse column DFT of the cross power and the row c2r
  * DFT run as split-precision DFT-GEMMs on the tcgen05 tensor cores with FP32

@@ -100,6 +100,8 @@ _SIGNATURES = {
     "lgb_refine_supported": ([ctypes.POINTER(RefineProblem)], _I),
     "lgb_refine_workspace_size": ([ctypes.POINTER(RefineProblem), ctypes.POINTER(_SZ)], _I),
     "lgb_refine_search": ([ctypes.POINTER(RefineProblem), ctypes.POINTER(CtfParams)] + [_P] * 18 + [_SZ, _P], _I),
+    "lgb_refine_collect": ([_I] * 4 + [_P] * 7, _I),
+    "lgb_refine_decode": ([_I] * 3 + [_P] * 10, _I),
     "lgb_match_precision_supported": ([_PROB, _I], _I),
     "lgb_match_precision_workspace_size": ([_PROB, ctypes.POINTER(_SZ)], _I),
     "lgb_match_search_precision": ([_PROB, _I, _P, _P, _P, _I, _I, _P, _P, _P, _P, _P, _SZ, _P, _P], _I),

@@ -5,8 +5,9 @@ Same arguments and returned keys as Leopard-EM's
 (backend/core_refine_template.py:33-202).  The per-particle Python loop with
 per-batch host synchronisation (:447-473, :678-751) becomes one C-ABI call per
 group of particles: every particle's CTF stack, offset batches, correlograms,
-z-scores and strict '>' best-so-far updates stay on the device; the host only
-decodes the winning flat index and composes the Euler angles (:503-551).
+z-scores, strict '>' best-so-far updates and the winners' indices and offsets
+stay on the device; one copy brings them back and the host only composes the
+Euler angles (:503-551).
 """
 
 from __future__ import annotations
@@ -16,7 +17,6 @@ import warnings
 
 import torch
 
-from .. import rotations as rot
 from .._native import check, lib
 from .._native import RefineProblem, CtfParams
 
@@ -41,11 +41,11 @@ def _ctf_params(ctf_kwargs: dict) -> CtfParams:
     )
 
 
-def refine_particles_device(particle_stack_dft, template_dft, euler_angles, euler_angle_offsets, defocus_offsets,
-                            defocus_u, defocus_v, defocus_angle, pixel_size_offsets, corr_mean, corr_std, ctf_kwargs,
-                            projective_filters, device, batch_size=32, max_correlograms_per_call=16384):
-    """Run the local grid for every particle; returns raw per-particle device
-    results (best z, its batch's max cc, flat index, batch start, batch length)."""
+def _search(particle_stack_dft, template_dft, euler_angles, euler_angle_offsets, defocus_offsets, defocus_u, defocus_v,
+            defocus_angle, pixel_size_offsets, corr_mean, corr_std, ctf_kwargs, projective_filters, device, batch_size,
+            max_correlograms_per_call=16384):
+    """Enqueue the local grid of every particle; returns the device results (int32 [5, N]: the words of best z,
+    its batch's max cc, flat index, batch start, batch length) and the device copies of the angles and offsets."""
     dev = _device(device)
     N, H, wc_img = particle_stack_dft.shape
     W = 2 * (wc_img - 1)
@@ -67,9 +67,7 @@ def refine_particles_device(particle_stack_dft, template_dft, euler_angles, eule
     prm = _ctf_params(ctf_kwargs)
     per_call = max(1, min(N, max_correlograms_per_call // max(1, C * D * B)))
     L = lib()
-    out = {k: torch.empty(N, dtype=dt, device=dev) for k, dt in
-           [("z", torch.float32), ("cc", torch.float32), ("flat", torch.int32), ("o0", torch.int32),
-            ("nb", torch.int32)]}
+    raw = torch.empty((5, N), dtype=torch.int32, device=dev)
     with torch.cuda.device(dev):
         s = ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
         f32 = dict(device=dev, dtype=torch.float32)
@@ -77,6 +75,7 @@ def refine_particles_device(particle_stack_dft, template_dft, euler_angles, eule
         offs = euler_angle_offsets.to(**f32).contiguous()
         dfo = defocus_offsets.to(**f32).contiguous()
         pxo = pixel_size_offsets.to(**f32).contiguous()
+        eul = euler_angles.to(**f32).contiguous()
         ws = None
         for a in range(0, N, per_call):
             b = min(N, a + per_call)
@@ -87,27 +86,34 @@ def refine_particles_device(particle_stack_dft, template_dft, euler_angles, eule
             check(L.lgb_refine_workspace_size(ctypes.byref(prob), ctypes.byref(need)), "refine workspace")
             if ws is None or ws.numel() < need.value:
                 ws = torch.empty(int(need.value), dtype=torch.uint8, device=dev)
-            args = [
-                particle_stack_dft[a:b].to(dev, torch.complex64).contiguous(),
-                euler_angles[a:b].to(**f32).contiguous(),
-                defocus_u[a:b].to(**f32).contiguous(),
-                defocus_v[a:b].to(**f32).contiguous(),
-                defocus_angle[a:b].to(**f32).contiguous(),
-                corr_mean[a:b].to(**f32).contiguous(),
-                corr_std[a:b].to(**f32).contiguous(),
-                projective_filters[a:b].to(**f32).contiguous(),
-            ]
-            ps, eul, du, dv, dang, cm, cs_, pf = args
+            part = [defocus_u, defocus_v, defocus_angle, corr_mean, corr_std, projective_filters]
+            ps = particle_stack_dft
+            if b - a < N:
+                part = [t[a:b] for t in part]
+                ps = ps[a:b]
+            ps = ps.to(dev, torch.complex64).contiguous()
+            du, dv, dang, cm, cs_, pf = [t.to(**f32).contiguous() for t in part]
+            out = [raw.data_ptr() + 4 * (k * N + a) for k in range(5)]
             check(
                 L.lgb_refine_search(
-                    ctypes.byref(prob), ctypes.byref(prm), ps.data_ptr(), tdft.data_ptr(), eul.data_ptr(),
+                    ctypes.byref(prob), ctypes.byref(prm), ps.data_ptr(), tdft.data_ptr(), eul.data_ptr() + 12 * a,
                     offs.data_ptr(), du.data_ptr(), dv.data_ptr(), dang.data_ptr(), dfo.data_ptr(), pxo.data_ptr(),
-                    cm.data_ptr(), cs_.data_ptr(), pf.data_ptr(), out["z"][a:b].data_ptr(),
-                    out["cc"][a:b].data_ptr(), out["flat"][a:b].data_ptr(), out["o0"][a:b].data_ptr(),
-                    out["nb"][a:b].data_ptr(), ws.data_ptr(), ws.numel(), s),
+                    cm.data_ptr(), cs_.data_ptr(), pf.data_ptr(), *out, ws.data_ptr(), ws.numel(), s),
                 "lgb_refine_search",
             )
-    return out
+    return raw, eul, offs, dfo, pxo
+
+
+def refine_particles_device(particle_stack_dft, template_dft, euler_angles, euler_angle_offsets, defocus_offsets,
+                            defocus_u, defocus_v, defocus_angle, pixel_size_offsets, corr_mean, corr_std, ctf_kwargs,
+                            projective_filters, device, batch_size=32, max_correlograms_per_call=16384):
+    """Run the local grid for every particle; returns raw per-particle device
+    results (best z, its batch's max cc, flat index, batch start, batch length)."""
+    raw = _search(particle_stack_dft, template_dft, euler_angles, euler_angle_offsets, defocus_offsets, defocus_u,
+                  defocus_v, defocus_angle, pixel_size_offsets, corr_mean, corr_std, ctf_kwargs, projective_filters,
+                  device, batch_size, max_correlograms_per_call)[0]
+    z, cc, flat, o0, nb = raw.unbind()
+    return {"z": z.view(torch.float32), "cc": cc.view(torch.float32), "flat": flat, "o0": o0, "nb": nb}
 
 
 def core_refine_template(
@@ -138,55 +144,46 @@ def core_refine_template(
         raise ValueError("anisotropic magnification (mag_matrix) is not supported by leopard_em_gb300")
     if num_cuda_streams > 1:
         warnings.warn("num_cuda_streams is ignored: one fused kernel sequence per particle group", stacklevel=2)
-    raw = refine_particles_device(particle_stack_dft, template_dft, euler_angles, euler_angle_offsets,
-                                  defocus_offsets, defocus_u, defocus_v, defocus_angle, pixel_size_offsets, corr_mean,
-                                  corr_std, ctf_kwargs, projective_filters, device, batch_size)
-    raw = {k: v.cpu() for k, v in raw.items()}
-    return decode_refine_results(raw, particle_stack_dft.shape, template_dft.shape[0], euler_angles,
-                                 euler_angle_offsets, defocus_offsets, pixel_size_offsets)
-
-
-def decode_refine_results(raw, stack_shape, d, euler_angles, euler_angle_offsets, defocus_offsets,
-                          pixel_size_offsets):
-    """Flat index -> (offsets, position, angle index); Euler composition and
-    wrapping as core_refine_template.py:503-551 and :180-191."""
-    N, H, wc_img = stack_shape
-    W = 2 * (wc_img - 1)
-    crop_w = W - d + 1
+    raw, eul, offs, dfo, pxo = _search(particle_stack_dft, template_dft, euler_angles, euler_angle_offsets,
+                                       defocus_offsets, defocus_u, defocus_v, defocus_angle, pixel_size_offsets,
+                                       corr_mean, corr_std, ctf_kwargs, projective_filters, device, batch_size)
+    N, H, wc_img = particle_stack_dft.shape
+    d = template_dft.shape[0]
+    crop_h, crop_w = H - d + 1, 2 * (wc_img - 1) - d + 1
     D, C = int(defocus_offsets.shape[0]), int(pixel_size_offsets.shape[0])
-    offs = euler_angle_offsets.cpu().to(torch.float32)
-    dfo = defocus_offsets.cpu().to(torch.float32)
-    pxo = pixel_size_offsets.cpu().to(torch.float32)
-    flat = raw["flat"].long()
-    nb = raw["nb"].long().clamp_min(1)
-    ok = flat >= 0
-    f = flat.clamp_min(0)
-    n_cpp = C * D * nb
-    c = f % n_cpp
-    pix = f // n_cpp
-    y = torch.where(ok, pix // crop_w, torch.zeros_like(pix))
-    x = torch.where(ok, pix % crop_w, torch.zeros_like(pix))
-    cs_idx = c // (D * nb)
-    df_idx = (c // nb) % D
-    a_idx = c % nb
-    angle_idx = torch.where(ok, raw["o0"].long() + a_idx, torch.zeros_like(a_idx))
-    off_angles = torch.where(ok[:, None], offs[angle_idx], torch.zeros(N, 3))
-    df_off = torch.where(ok, dfo[df_idx], torch.zeros(N))
-    px_off = torch.where(ok, pxo[cs_idx], torch.zeros(N))
-    eul = rot.combine_euler_angles(off_angles.double(), euler_angles.cpu().double()).to(torch.float32)
-    eul[:, 0] = torch.where(eul[:, 0] < 0, eul[:, 0] + 360, eul[:, 0])
-    eul[:, 1] = torch.where(eul[:, 1] < 0, eul[:, 1] + 180, eul[:, 1])
-    eul[:, 2] = torch.where(eul[:, 2] < 0, eul[:, 2] + 360, eul[:, 2])
-    return {
-        "refined_cross_correlation": raw["cc"].to(torch.float32),
-        "refined_z_score": raw["z"].to(torch.float32),
-        "refined_euler_angles": eul,
-        "refined_defocus_offset": df_off,
-        "refined_pixel_size_offset": px_off,
-        "refined_pos_y": y - (H - d + 1) // 2,
-        "refined_pos_x": x - (W - d + 1) // 2,
-        "angle_idx": angle_idx,
+    # the poses as given, in FP64; FP32 poses that are on the device come back with the results
+    pose64 = None
+    if euler_angles.dtype != torch.float32 or not euler_angles.is_cuda:
+        pose64 = euler_angles.cpu().to(torch.float64).contiguous()
+    L = lib()
+    packed = torch.empty((N, REFINE_WORDS), dtype=torch.int32, device=raw.device)
+    with torch.cuda.device(raw.device):
+        s = ctypes.c_void_p(torch.cuda.current_stream(raw.device).cuda_stream)
+        check(L.lgb_refine_collect(N, crop_w, C, D, raw.data_ptr(), eul.data_ptr(), offs.data_ptr(), dfo.data_ptr(),
+                                   pxo.data_ptr(), packed.data_ptr(), s), "lgb_refine_collect")
+    return decode_refine_results(packed.cpu(), pose64, crop_h, crop_w)
+
+
+REFINE_WORDS = 13  # 32-bit words a particle in lgb_refine_collect's output
+
+
+def decode_refine_results(packed, pose64, crop_h, crop_w):
+    """Result dictionary from lgb_refine_collect's words (CPU): Euler composition and
+    wrapping as core_refine_template.py:503-551 and :180-191."""
+    N = packed.shape[0]
+    out = {
+        "refined_cross_correlation": torch.empty(N, dtype=torch.float32),
+        "refined_z_score": torch.empty(N, dtype=torch.float32),
+        "refined_euler_angles": torch.empty((N, 3), dtype=torch.float32),
+        "refined_defocus_offset": torch.empty(N, dtype=torch.float32),
+        "refined_pixel_size_offset": torch.empty(N, dtype=torch.float32),
+        "refined_pos_y": torch.empty(N, dtype=torch.int64),
+        "refined_pos_x": torch.empty(N, dtype=torch.int64),
+        "angle_idx": torch.empty(N, dtype=torch.int64),
     }
+    check(lib().lgb_refine_decode(N, crop_h, crop_w, packed.data_ptr(), None if pose64 is None else pose64.data_ptr(),
+                                  *[t.data_ptr() for t in out.values()]), "lgb_refine_decode")
+    return out
 
 
 def cross_correlate_particle_stack(

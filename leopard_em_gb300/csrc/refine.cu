@@ -14,6 +14,7 @@
 // built once per call by refine_filters_kernel.
 // Reference: backend/core_refine_template.py:555-767, utils/ctf_utils.py:19-116.
 #include <math.h>
+#include <string.h>
 
 #include "profiler.h"
 #include "match_kernels.cuh"
@@ -247,6 +248,56 @@ __global__ void refine_commit_kernel(int P, unsigned long long* slot_key, unsign
   }
   slot_key[p] = 0ull;
   slot_cc[p] = 0u;
+}
+
+// Result words a particle of lgb_refine_collect.
+enum { RW_Z, RW_CC, RW_Y, RW_X, RW_ANGLE, RW_DEFOCUS, RW_PIXEL, RW_OFFSET, RW_POSE = RW_OFFSET + 3, RW_WORDS = RW_POSE + 3 };
+
+// Winning flat index -> position, angle index and offsets, one thread a
+// particle.  It is here for the copies that it saves: eight results and offset
+// tables came back one by one, and torch decoded them in some seventy host
+// calls (one particle: 988 -> 386 us a call).
+__global__ void refine_collect_kernel(int P, int crop_w, int n_cd, int D, const unsigned* __restrict__ raw,
+                                      const float* __restrict__ euler, const float* __restrict__ offsets,
+                                      const float* __restrict__ defocus, const float* __restrict__ pixel,
+                                      unsigned* __restrict__ packed) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= P) return;
+  const int flat = (int)raw[2 * (size_t)P + p], o0 = (int)raw[3 * (size_t)P + p];
+  const int nb = max((int)raw[4 * (size_t)P + p], 1);
+  unsigned* out = packed + (size_t)p * RW_WORDS;
+  out[RW_Z] = raw[p];
+  out[RW_CC] = raw[(size_t)P + p];
+  int y = 0, x = 0, angle = 0;
+  float df = 0.f, px = 0.f, off[3] = {0.f, 0.f, 0.f};
+  if (flat >= 0) {  // else no batch beat the initial value
+    const int n_cpp = n_cd * nb, c = flat % n_cpp, pix = flat / n_cpp;
+    y = pix / crop_w;
+    x = pix % crop_w;
+    px = pixel[c / (D * nb)];
+    df = defocus[(c / nb) % D];
+    angle = o0 + c % nb;
+    for (int i = 0; i < 3; ++i) off[i] = offsets[3 * (size_t)angle + i];
+  }
+  out[RW_Y] = y;
+  out[RW_X] = x;
+  out[RW_ANGLE] = angle;
+  out[RW_DEFOCUS] = __float_as_uint(df);
+  out[RW_PIXEL] = __float_as_uint(px);
+  for (int i = 0; i < 3; ++i) {
+    out[RW_OFFSET + i] = __float_as_uint(off[i]);
+    out[RW_POSE + i] = __float_as_uint(euler[3 * (size_t)p + i]);
+  }
+}
+
+// ZYZ angles (degrees) -> R = Rz(phi) Ry(theta) Rz(psi), host
+static void host_rotation(const double* e, double* R) {
+  const double k = 3.14159265358979323846 / 180.0;
+  const double cp = cos(e[0] * k), sp = sin(e[0] * k), ct = cos(e[1] * k), st = sin(e[1] * k), cs = cos(e[2] * k),
+               ss = sin(e[2] * k);
+  const double r[9] = {cp * ct * cs - sp * ss, -cp * ct * ss - sp * cs, cp * st,  sp * ct * cs + cp * ss,
+                       -sp * ct * ss + cp * cs, sp * st, -st * cs, st * ss, ct};
+  memcpy(R, r, sizeof r);
 }
 
 __global__ void refine_init_kernel(int P, float* best_z, float* best_cc, int* best_flat, int* best_o0, int* best_nb,
@@ -497,6 +548,64 @@ int lgb_refine_search(const lgb_refine_problem* p, const lgb_ctf_params* ctf, co
     refine_commit_kernel<<<(P + 127) / 128, 128, 0, s>>>(P, key, cc, o0, nb, best_z, best_cc, best_flat,
                                                            best_offset_begin, best_batch_len);
     if (cudaGetLastError() != cudaSuccess) return LGB_ERR_CUDA;
+  }
+  return LGB_OK;
+}
+
+int lgb_refine_collect(int n_particles, int crop_w, int n_pixel_sizes, int n_defocus, const void* raw,
+                       const float* euler_angles, const float* euler_offsets, const float* defocus_offsets,
+                       const float* pixel_size_offsets, void* packed, void* stream) {
+  if (n_particles == 0) return LGB_OK;
+  if (n_particles < 0 || crop_w < 1 || n_pixel_sizes < 1 || n_defocus < 1 || !raw || !euler_angles || !euler_offsets ||
+      !defocus_offsets || !pixel_size_offsets || !packed)
+    return LGB_ERR_INVALID_ARGUMENT;
+  refine_collect_kernel<<<(n_particles + 63) / 64, 64, 0, (cudaStream_t)stream>>>(
+      n_particles, crop_w, n_pixel_sizes * n_defocus, n_defocus, static_cast<const unsigned*>(raw), euler_angles,
+      euler_offsets, defocus_offsets, pixel_size_offsets, static_cast<unsigned*>(packed));
+  return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
+}
+
+int lgb_refine_decode(int n_particles, int crop_h, int crop_w, const void* packed, const double* euler_angles,
+                      float* cc, float* z, float* angles, float* defocus_offset, float* pixel_size_offset,
+                      long long* pos_y, long long* pos_x, long long* angle_idx) {
+  if (n_particles == 0) return LGB_OK;
+  if (n_particles < 0 || !packed || !cc || !z || !angles || !defocus_offset || !pixel_size_offset || !pos_y || !pos_x ||
+      !angle_idx)
+    return LGB_ERR_INVALID_ARGUMENT;
+  for (int p = 0; p < n_particles; ++p) {
+    int w[RW_WORDS];
+    float f[RW_WORDS];
+    memcpy(w, static_cast<const char*>(packed) + (size_t)p * sizeof w, sizeof w);
+    memcpy(f, w, sizeof f);
+    z[p] = f[RW_Z];
+    cc[p] = f[RW_CC];
+    pos_y[p] = (long long)w[RW_Y] - crop_h / 2;
+    pos_x[p] = (long long)w[RW_X] - crop_w / 2;
+    angle_idx[p] = w[RW_ANGLE];
+    defocus_offset[p] = f[RW_DEFOCUS];
+    pixel_size_offset[p] = f[RW_PIXEL];
+    double a[3], b[3], A[9], B[9], R[9];
+    for (int i = 0; i < 3; ++i) {
+      a[i] = f[RW_OFFSET + i];
+      b[i] = euler_angles ? euler_angles[3 * (size_t)p + i] : f[RW_POSE + i];
+    }
+    host_rotation(a, A);
+    host_rotation(b, B);
+    for (int i = 0; i < 9; ++i) {
+      R[i] = 0.0;  // (0 + -0 = 0: an angle of a zero row is atan2(0, .))
+      for (int k = 0; k < 3; ++k) R[i] += A[3 * (i / 3) + k] * B[3 * k + i % 3];
+    }
+    const double deg = 180.0 / 3.14159265358979323846;
+    const double c = R[8] < -1.0 ? -1.0 : (R[8] > 1.0 ? 1.0 : R[8]);
+    float* e = angles + 3 * (size_t)p;
+    e[0] = (float)(atan2(R[5], R[2]) * deg);
+    e[1] = (float)(acos(c) * deg);
+    // (volatile: folded into a multiply-add, the negation would give a zero the other sign)
+    volatile double r20 = R[6];
+    e[2] = (float)(atan2(R[7], -r20) * deg);
+    if (e[0] < 0.f) e[0] += 360.f;
+    if (e[1] < 0.f) e[1] += 180.f;
+    if (e[2] < 0.f) e[2] += 360.f;
   }
   return LGB_OK;
 }
