@@ -307,9 +307,7 @@ int lgb_match_prepare_image(const lgb_match_problem* p, const void* image_dft, v
   const MatchLayout L = layout_of(p);
   if (workspace_bytes < L.total) return LGB_ERR_WORKSPACE_TOO_SMALL;
   float2* ip = reinterpret_cast<float2*>(static_cast<char*>(workspace) + L.ip);
-  repack_rows_kernel<<<(p->image_h + 7) / 8, 256, 0, (cudaStream_t)stream>>>(
-      static_cast<const float2*>(image_dft), p->image_h, L.wc_img, L.wcp, ip);
-  return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
+  return launch_repack_rows(image_dft, p->image_h, L.wc_img, L.wcp, ip, (cudaStream_t)stream);
 }
 
 int lgb_match_filters(const lgb_match_problem* p, const float* ctf_filters, const float* whitening,

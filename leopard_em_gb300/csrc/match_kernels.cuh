@@ -32,24 +32,6 @@ constexpr int kColGroup = 4;  // columns per colpass CTA: 4 x 8 B = one 32 B sec
 
 __host__ __device__ inline int pad4(int n) { return (n + 3) & ~3; }
 
-// Spectrum rows of wc columns -> rows of wcp, zero filled: one warp per row (64-bit
-// divisions per element held the flat form to 3.0 TB/s; this 7.4, partly L2, at 86k rows of 145).
-static __global__ void __launch_bounds__(256)
-    repack_rows_kernel(const float2* __restrict__ src, long long rows, int wc, int wcp, float2* __restrict__ dst) {
-  const long long row = blockIdx.x * 8LL + threadIdx.x / 32;
-  if (row >= rows) return;
-  const float2* s = src + row * wc;
-  float2* d = dst + row * wcp;
-  for (int k = threadIdx.x & 31; k < wcp; k += 256) {  // eight loads in flight
-    float2 v[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) v[q] = k + 32 * q < wc ? __ldg(s + k + 32 * q) : make_float2(0.f, 0.f);
-#pragma unroll
-    for (int q = 0; q < 8; ++q)
-      if (k + 32 * q < wcp) d[k + 32 * q] = v[q];
-  }
-}
-
 // ---------------------------------------------------------------------------
 // Euler (ZYZ, degrees) -> R = Rz(phi) Ry(theta) Rz(psi), in FP64.
 // ---------------------------------------------------------------------------

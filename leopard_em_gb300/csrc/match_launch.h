@@ -28,6 +28,8 @@ int launch_proj_row(int h, const void* T, int n_c, float* proj, double* rowstats
 // in rowstats.  The column pass then applies the normalisation (norm below).
 bool supported_proj_row_rfft(int h, int W);
 int launch_proj_row_rfft(int h, int W, const void* T, int n_c, double* rowstats, int Wcp, void* A, cudaStream_t s);
+// Rows of wc complex elements -> rows of wcp, zero filled.
+int launch_repack_rows(const void* src, long long rows, int wc, int wcp, void* dst, cudaStream_t s);
 // Per-correlogram normalisation constants (e, s) from the row moments, stored
 // as a float2 over rowstats[c][0][0].
 // offset (or null): image c's DC bin (dc[c * dc_stride]) times the normalised

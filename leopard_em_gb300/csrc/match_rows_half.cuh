@@ -27,11 +27,14 @@
 
 namespace lgb {
 
-template <int WH_, int NT_, int ROWS_, class RL_, int MINB_>
+// SPLIT > 1: a CTA has one row and shares its correlograms out to SPLIT groups
+// of NT threads, whose statistics meet in shared memory.
+template <int WH_, int NT_, int ROWS_, class RL_, int MINB_, int SPLIT_ = 1>
 struct RowHalf {
   using RL = RL_;
-  static constexpr int WH = WH_, NT = NT_, ROWS = ROWS_, MINB = MINB_;
-  static constexpr int THREADS = NT * ROWS;
+  static constexpr int WH = WH_, NT = NT_, ROWS = ROWS_, MINB = MINB_, SPLIT = SPLIT_;
+  static_assert(SPLIT == 1 || ROWS == 1, "one row per CTA where it is split");
+  static constexpr int THREADS = NT * ROWS * SPLIT;
   static constexpr int R1 = Head<RL>::value, RLAST = Last<RL>::value;
   static constexpr int NB1 = WH / R1, PER1 = (NB1 + NT - 1) / NT;
   static constexpr int NBL = WH / RLAST, PERL = (NBL + NT - 1) / NT;
@@ -39,7 +42,9 @@ struct RowHalf {
   static constexpr int WCP = (WH + 1 + 3) / 4 * 4;          // row stride of Y
   static constexpr int ZS = (IdxPad16::pad(WH) + 2) / 2 * 2;
   static constexpr int TAB = TableSize<1, RL>::value;
-  static constexpr size_t SMEM = sizeof(float2) * ((size_t)ROWS * (WCP + ZS) + TAB);
+  static constexpr size_t SMEM = sizeof(float2) * ((size_t)ROWS * SPLIT * (WCP + ZS) + TAB);
+  // a group's statistics pass through its own rows, sums after maxima
+  static_assert(SPLIT == 1 || 2 * (WCP + ZS) >= 4 * PX * NT, "room for the statistics");
 };
 
 template <class C>
@@ -51,19 +56,23 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
   constexpr int WH = C::WH, NT = C::NT, ROWS = C::ROWS, R1 = C::R1, RLAST = C::RLAST, NB1 = C::NB1, NBL = C::NBL,
                 PERL = C::PERL, PER1 = C::PER1, PX = C::PX;
   extern __shared__ float2 rhsm[];
-  const int g = ROWS == 1 ? 0 : threadIdx.x / NT, t = ROWS == 1 ? threadIdx.x : threadIdx.x - g * NT;
-  float2* xs = rhsm + g * C::WCP;
-  float2* z = rhsm + ROWS * C::WCP + g * C::ZS;
-  float2* tab = rhsm + ROWS * (C::WCP + C::ZS);
+  constexpr int SPLIT = C::SPLIT, SLOTS = ROWS * SPLIT;
+  const int slot = SLOTS == 1 ? 0 : threadIdx.x / NT, t = SLOTS == 1 ? threadIdx.x : threadIdx.x - slot * NT;
+  const int g = SPLIT == 1 ? slot : 0, part = SPLIT == 1 ? 0 : slot;
+  float2* xs = rhsm + slot * (C::WCP + C::ZS);
+  float2* z = xs + C::WCP;
+  float2* tab = rhsm + SLOTS * (C::WCP + C::ZS);
+  // this group's correlograms
+  const int per = SPLIT == 1 ? n_c : (n_c + SPLIT - 1) / SPLIT, c0 = SPLIT == 1 ? 0 : part * per;
   // row y of correlogram c -> xs, 16 bytes a copy
   auto stage = [&](int y, int c) {
-    if (y < y_rows) {
+    if (y < y_rows && (SPLIT == 1 || c < n_c)) {
       const float2* src = Y + ((size_t)c * y_rows + y) * C::WCP;
       for (int i = t; i < C::WCP / 2; i += NT) cp_async16(xs + 2 * i, src + 2 * i);
     }
     cp_async_commit();
   };
-  stage(blockIdx.x * ROWS + g, 0);
+  stage(blockIdx.x * ROWS + g, c0);
   FillTables<WH, 1, RL>::run(tab, threadIdx.x, C::THREADS);
   // c2r pre-twiddle exp(+i pi k / WH) at k = j + q NB1: exp(i pi j / WH), kept
   // in registers, times the constant exp(i pi q / R1)
@@ -90,7 +99,7 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
 #pragma unroll
     for (int i = 0; i < PX; ++i) arg[i] = 0u;
 #pragma unroll 1
-    for (int c = 0; c < n_c; ++c) {
+    for (int c = c0; c < c0 + per; ++c) {
       cp_async_wait<0>();
       __syncthreads();
 #pragma unroll
@@ -114,15 +123,15 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
       }
       __syncthreads();
       // the staged row is read: the next one comes in during the other passes
-      if (c + 1 < n_c)
+      if (c + 1 < c0 + per)
         stage(y, c + 1);
-      else if (y0 + gridDim.x * ROWS < y_rows)
-        stage(y + gridDim.x * ROWS, 0);
+      else if (SPLIT == 1 && y0 + gridDim.x * ROWS < y_rows)
+        stage(y + gridDim.x * ROWS, c0);
       TablePasses<WH, NT, +1, IdxPad16, R1, typename Middle<RL>::type>::run(z, tab, t);
 #pragma unroll
       for (int p = 0; p < PERL; ++p) {
         const int j = t + p * NT;
-        if (NBL == PERL * NT || j < NBL) {
+        if ((NBL == PERL * NT || j < NBL) && (SPLIT == 1 || c < n_c)) {
           float2 v[RLAST];
           const int fj = IdxPad16::f(j);
 #pragma unroll
@@ -149,8 +158,63 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
         }
       }
     }
+    // ---- the groups' statistics, in the order of their correlograms (a tie goes to the first)
+    if constexpr (SPLIT > 1) {
+      float* mine = reinterpret_cast<float*>(xs);
+      __syncthreads();
+      if (part) {
+#pragma unroll
+        for (int i = 0; i < 2 * PX; ++i) mine[i * NT + t] = top[i];
+#pragma unroll
+        for (int i = 0; i < PX; ++i) mine[(2 * PX + i) * NT + t] = __uint_as_float(arg[i]);
+      }
+      __syncthreads();
+      if (!part) {
+#pragma unroll 1
+        for (int o = 1; o < SPLIT; ++o) {
+          const float* other = mine + o * 2 * (C::WCP + C::ZS);
+#pragma unroll
+          for (int i = 0; i < PX; ++i) {
+            const float a = other[2 * i * NT + t], b = other[(2 * i + 1) * NT + t];
+            const unsigned at = __float_as_uint(other[(2 * PX + i) * NT + t]);
+            if (a > top[2 * i]) {
+              top[2 * i] = a;
+              arg[i] = (arg[i] & 0xffff0000u) | (at & 0xffffu);
+            }
+            if (b > top[2 * i + 1]) {
+              top[2 * i + 1] = b;
+              arg[i] = (arg[i] & 0xffffu) | (at & 0xffff0000u);
+            }
+          }
+        }
+      }
+      __syncthreads();
+      if (part) {
+#pragma unroll
+        for (int i = 0; i < 2 * PX; ++i) {
+          mine[i * NT + t] = sm[i];
+          mine[(2 * PX + i) * NT + t] = sq[i];
+        }
+      }
+      __syncthreads();
+      if (!part) {
+#pragma unroll 1
+        for (int o = 1; o < SPLIT; ++o) {
+          const float* other = mine + o * 2 * (C::WCP + C::ZS);
+#pragma unroll
+          for (int i = 0; i < 2 * PX; ++i) {
+            sm[i] += other[i * NT + t];
+            sq[i] += other[(2 * PX + i) * NT + t];
+          }
+        }
+      }
+      if (y0 + gridDim.x < y_rows) {  // the next row's first data
+        __syncthreads();
+        stage(y + gridDim.x, c0);
+      }
+    }
     // ---- one read-modify-write of the maps
-    if (y < y_rows) {
+    if (y < y_rows && !part) {
 #pragma unroll
       for (int p = 0; p < PERL; ++p) {
         const int j = t + p * NT;
@@ -201,23 +265,38 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
 }
 
 template <class C>
-int rowpass_half_t(const void* Y, int H, int y_rows, int Wcp, int n_c, int nb, int n_orient, int o0,
-                   const int* o0_dev, float* mip, int* best, double* s1, double* s2, cudaStream_t s) {
-  if (Wcp != C::WCP) return LGB_ERR_INVALID_ARGUMENT;
-  if (n_c > 0xffff) return LGB_ERR_INVALID_ARGUMENT;  // batch indices are kept in 16 bits
+int rowpass_half_launch(const void* Y, int H, int y_rows, int n_c, int nb, int n_orient, int o0, const int* o0_dev,
+                        float* mip, int* best, double* s1, double* s2, int sms, cudaStream_t s) {
   if (cudaFuncSetAttribute(rowpass_half_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM) !=
           cudaSuccess ||
       cudaFuncSetAttribute(rowpass_half_kernel<C>, cudaFuncAttributePreferredSharedMemoryCarveout,
                            cudaSharedmemCarveoutMaxShared) != cudaSuccess)
     return LGB_ERR_CUDA;
   const float scale = 1.0f / ((float)H * (float)(2 * C::WH));
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int groups = (y_rows + C::ROWS - 1) / C::ROWS, ctas = sms * C::MINB;
   rowpass_half_kernel<C><<<groups < ctas ? groups : ctas, C::THREADS, C::SMEM, s>>>(
       static_cast<const float2*>(Y), y_rows, n_c, nb, n_orient, o0, o0_dev, scale, mip, best, s1, s2);
   return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
+}
+
+// C, or the first of the SPLIT forms in Cs (most groups first) whose rows are
+// all resident at once and whose groups have two correlograms or more (one each
+// measured no better).
+template <class C, class... Cs>
+int rowpass_half_t(const void* Y, int H, int y_rows, int Wcp, int n_c, int nb, int n_orient, int o0,
+                   const int* o0_dev, float* mip, int* best, double* s1, double* s2, cudaStream_t s) {
+  if (Wcp != C::WCP) return LGB_ERR_INVALID_ARGUMENT;
+  if (n_c > 0xffff) return LGB_ERR_INVALID_ARGUMENT;  // batch indices are kept in 16 bits
+  int dev = 0, sms = 0, st = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const bool done = ((y_rows <= sms * Cs::MINB && n_c >= 2 * Cs::SPLIT &&
+                      (st = rowpass_half_launch<Cs>(Y, H, y_rows, n_c, nb, n_orient, o0, o0_dev, mip, best, s1, s2, sms,
+                                                    s),
+                       true)) ||
+                     ...);
+  if (done) return st;
+  return rowpass_half_launch<C>(Y, H, y_rows, n_c, nb, n_orient, o0, o0_dev, mip, best, s1, s2, sms, s);
 }
 
 }  // namespace lgb

@@ -469,8 +469,8 @@ int lgb_refine_search(const lgb_refine_problem* p, const lgb_ctf_params* ctf, co
   const int P = p->n_particles, H = p->image_h, W = p->image_w, d = p->template_size;
   const int C = p->n_pixel_sizes, D = p->n_defocus;
 
-  repack_rows_kernel<<<(unsigned)(((long long)P * H + 7) / 8), 256, 0, s>>>(
-      static_cast<const float2*>(particle_stack_dft), (long long)P * H, W / 2 + 1, L.wcp, ip);
+  int st;
+  if ((st = launch_repack_rows(particle_stack_dft, (long long)P * H, W / 2 + 1, L.wcp, ip, s))) return st;
   const double lambda = electron_wavelength_angstrom(ctf->voltage_kv), amp = ctf->amplitude_contrast;
   FilterTurns turns;
   turns.inv_size = 1.0 / (d * ctf->pixel_size);
@@ -492,7 +492,6 @@ int lgb_refine_search(const lgb_refine_problem* p, const lgb_ctf_params* ctf, co
   const float scale = 1.0f / ((float)H * (float)W);
   const bool prof = profiling_on();
   const bool fused_rfft = refine_fused_rfft(d, W, H);
-  int st;
   for (int o0 = 0; o0 < p->n_offsets; o0 += p->offset_batch) {
     const int nb = (p->n_offsets - o0) < p->offset_batch ? (p->n_offsets - o0) : p->offset_batch;
     const int n_cpp = L.n_cd * nb;

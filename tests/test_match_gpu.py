@@ -272,6 +272,13 @@ def test_long_row_pass_against_oracle(W, H, n_o, batch, n_df):
     _assert_parity(gpu, ref, second=ref["second_best"])
 
 
+@pytest.mark.parametrize("W,batch", [(512, 17), (512, 9), (1024, 13), (1024, 7), (2048, 7)])
+@pytest.mark.parametrize("H", [48, 64])
+def test_split_row_pass_against_oracle(W, batch, H):
+    """Rows whose correlograms are shared out to 8 / 4, 6 / 3 and 3 groups: unequal shares, groups without any."""
+    test_long_row_pass_against_oracle(W, H, 2 * batch + 3, batch, 1)
+
+
 @pytest.mark.parametrize("W", [512, 4096])
 def test_not_finite_correlograms_stay_apart(W):
     """A filter plane of NaN spoils its own correlograms only: they never win,
