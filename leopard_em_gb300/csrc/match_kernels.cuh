@@ -33,23 +33,29 @@ constexpr int kColGroup = 4;  // columns per colpass CTA: 4 x 8 B = one 32 B sec
 __host__ __device__ inline int pad4(int n) { return (n + 3) & ~3; }
 
 // ---------------------------------------------------------------------------
-// Euler (ZYZ, degrees) -> R = Rz(phi) Ry(theta) Rz(psi), in FP64.
+// Sines and cosines of ZYZ Euler angles, FP64 -> R = Rz(phi) Ry(theta) Rz(psi).
+// (FP64 sincos is a chain of a microsecond: callers give each angle a thread.)
 // ---------------------------------------------------------------------------
-__device__ inline void euler_zyz_to_rotmat(const float* e, float* R) {
-  const double k = 3.14159265358979323846 / 180.0;
-  double sp, cp, st, ct, ss, cs;
-  sincos((double)e[0] * k, &sp, &cp);
-  sincos((double)e[1] * k, &st, &ct);
-  sincos((double)e[2] * k, &ss, &cs);
-  R[0] = (float)(cp * ct * cs - sp * ss);
-  R[1] = (float)(-cp * ct * ss - sp * cs);
-  R[2] = (float)(cp * st);
-  R[3] = (float)(sp * ct * cs + cp * ss);
-  R[4] = (float)(-sp * ct * ss + cp * cs);
-  R[5] = (float)(sp * st);
-  R[6] = (float)(-st * cs);
-  R[7] = (float)(st * ss);
-  R[8] = (float)ct;
+struct SinCos {
+  double s, c;
+};
+__device__ inline SinCos sincos_degrees(float a) {
+  SinCos v;
+  sincos((double)a * (3.14159265358979323846 / 180.0), &v.s, &v.c);
+  return v;
+}
+template <class T>
+__device__ inline void rotmat_zyz(const SinCos* e, T* R) {
+  const double sp = e[0].s, cp = e[0].c, st = e[1].s, ct = e[1].c, ss = e[2].s, cs = e[2].c;
+  R[0] = (T)(cp * ct * cs - sp * ss);
+  R[1] = (T)(-cp * ct * ss - sp * cs);
+  R[2] = (T)(cp * st);
+  R[3] = (T)(sp * ct * cs + cp * ss);
+  R[4] = (T)(-sp * ct * ss + cp * cs);
+  R[5] = (T)(sp * st);
+  R[6] = (T)(-st * cs);
+  R[7] = (T)(st * ss);
+  R[8] = (T)ct;
 }
 
 // ---------------------------------------------------------------------------
@@ -522,16 +528,31 @@ __global__ void __launch_bounds__(ROWS * 16, 48 / ROWS)
   }
 }
 
+// Factors of the normalisation that depend on sizes alone: the FP64 divisions
+// and the square root of them were half of norm_constants_kernel's time.
+struct NormSizes {
+  int h;
+  double inv_edge;   // 1 / (4 h - 4)
+  double n;          // h^2
+  double mean;       // rel^2 / n, rel = n / (H W)
+  double border;     // (H - h) (W - h)
+  double root;       // sqrt(H W)
+  NormSizes() = default;
+  NormSizes(int h_, int H, int W)
+      : h(h_), inv_edge(1.0 / (4.0 * h_ - 4.0)), n((double)h_ * h_), mean(n / ((double)H * W) / ((double)H * W)),
+        border((double)(H - h_) * (double)(W - h_)), root(sqrt((double)H * (double)W)) {}
+};
+
 // Normalisation constants of utils.py:106-188 from the per-row moments:
 // returns edge mean e and scale s such that normalised = (p - e) * s.
 // Called by all 32 lanes of warp 0 (the launcher guarantees a full warp);
 // lane 0 gets the constants and, returned, the projection's sum.
-__device__ inline double projection_norm_constants(const double* rs, int h, int H, int W, float* e_out,
-                                                 float* s_out) {
+__device__ inline double projection_norm_constants(const double* rs, const NormSizes& ns, float* e_out, float* s_out) {
   // warp 0 reduces h rows
   double s1 = 0, s2 = 0, se = 0;
   const int lane = threadIdx.x & 31;
-  for (int r = lane; r < h; r += 32) {
+#pragma unroll 4
+  for (int r = lane; r < ns.h; r += 32) {
     s1 += rs[3 * r];
     s2 += rs[3 * r + 1];
     se += rs[3 * r + 2];
@@ -543,17 +564,15 @@ __device__ inline double projection_norm_constants(const double* rs, int h, int 
     se += __shfl_down_sync(0xffffffffu, se, o);
   }
   if (lane == 0) {
-    const double n = (double)h * (double)h;
-    const double e = se / (double)(4 * h - 4);
-    const double S1 = s1 - n * e;                  // sum of (p - e)
-    const double S2 = s2 - 2.0 * e * s1 + n * e * e;  // sum of (p - e)^2
-    const double rel = n / ((double)H * (double)W);
-    const double mean = (S1 / n) * rel * rel;
-    double var = S2 - 2.0 * mean * S1 + n * mean * mean;
-    var += (double)(H - h) * (double)(W - h) * mean * mean;
+    const double e = se * ns.inv_edge;
+    const double S1 = s1 - ns.n * e;                     // sum of (p - e)
+    const double S2 = s2 - 2.0 * e * s1 + ns.n * e * e;  // sum of (p - e)^2
+    const double mean = S1 * ns.mean;
+    double var = S2 - 2.0 * mean * S1 + ns.n * mean * mean;
+    var += ns.border * mean * mean;
     if (var < 1e-8) var = 1e-8;
     *e_out = (float)e;
-    *s_out = (float)(sqrt((double)H * (double)W) / sqrt(var));
+    *s_out = (float)(ns.root * rsqrt(var));
   }
   return s1;
 }
@@ -569,8 +588,8 @@ __device__ inline double projection_norm_constants(const double* rs, int h, int 
 // small transforms, where a CTA holds many rows to amortise the fill).
 template <int WH, int ROWS, bool TAB>
 __global__ void __launch_bounds__(ROWS* FftThreads<WH>::value)
-    pad_rfft_kernel(const float* __restrict__ proj, const double* __restrict__ rowstats, int h, int norm_h,
-                    int norm_w, int Wcp, int norm_ready, float2* __restrict__ A) {
+    pad_rfft_kernel(const float* __restrict__ proj, const double* __restrict__ rowstats, int h, NormSizes sizes,
+                    int Wcp, int norm_ready, float2* __restrict__ A) {
   constexpr int NT = FftThreads<WH>::value;
   constexpr int ZS = IdxPad16::pad(WH) + 2;
   __shared__ float2 z[ROWS][ZS];
@@ -595,7 +614,7 @@ __global__ void __launch_bounds__(ROWS* FftThreads<WH>::value)
       norm[1] = es.y;
     }
   } else if (threadIdx.x < 32) {
-    projection_norm_constants(rowstats + (size_t)c * h * 3, h, norm_h, norm_w, &norm[0], &norm[1]);
+    projection_norm_constants(rowstats + (size_t)c * h * 3, sizes, &norm[0], &norm[1]);
   }
   __syncthreads();
   const float e = norm[0], s = norm[1];

@@ -12,7 +12,8 @@ namespace lgb {
 // What bounds it: the sectors that a warp's gathers touch.  A warp samples a
 // patch of 8 columns x 4 rows: whatever the orientation, its points share
 // volume rows, where 32 columns of one row, as before, lie in up to 32 of them.
-// 300 slices of 256: 128 -> 118 us; 24 slices of 64 a batch: 10.3 -> 6.6.  Loading
+// 300 slices of 256: 128 -> 118 us; 32 slices of 64 a batch: 7.0 -> 6.7,
+// 5.0 with a thread for each FP64 sincos.  Loading
 // the 16 B that hold both x neighbours where they are aligned: 130.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
@@ -21,13 +22,16 @@ __global__ void __launch_bounds__(256)
                  float2* __restrict__ slices) {
   const int b = blockIdx.y;
   __shared__ float R[9];
-  if (threadIdx.x == 0) {
-    if (rotations) {
-      for (int i = 0; i < 9; ++i) R[i] = rotations[9 * (size_t)b + i];
-    } else {
+  __shared__ SinCos angle[3];
+  if (rotations) {
+    if (threadIdx.x < 9) R[threadIdx.x] = rotations[9 * (size_t)b + threadIdx.x];
+  } else {
+    if (threadIdx.x < 3) {
       const int o = o0 + (o0_dev ? *o0_dev : 0) + b;
-      euler_zyz_to_rotmat(euler + 3 * (size_t)o, R);
+      angle[threadIdx.x] = sincos_degrees(euler[3 * (size_t)o + threadIdx.x]);
     }
+    __syncwarp();
+    if (threadIdx.x == 0) rotmat_zyz(angle, R);
   }
   __syncthreads();
   const int wc = d / 2 + 1, half = d / 2;

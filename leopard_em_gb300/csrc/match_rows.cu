@@ -36,14 +36,14 @@ int launch_repack_rows(const void* src, long long rows, int wc, int wcp, void* d
 // takes Re(I00 conj(P00)) scale, P00 = s (sum of the projection - e h^2).
 // The FP64 pipe bounds it (a warp-wide add holds it for 32 cycles), so the
 // warps are CTAs of their own, spread over the SMs: 300 correlograms
-// 10.4 us in CTAs of eight warps, 7.3 now.
+// 10.4 us in CTAs of eight warps, 7.3 in one each, 5.0 without the divisions.
 __global__ void __launch_bounds__(32)
-    norm_constants_kernel(double* __restrict__ rowstats, int h, int norm_h, int norm_w, const float2* __restrict__ dc,
-                          size_t dc_stride, float scale, float* __restrict__ offset) {
-  const int c = blockIdx.x;
+    norm_constants_kernel(double* __restrict__ rowstats, NormSizes sizes, const float2* __restrict__ dc, size_t dc_stride,
+                          float scale, float* __restrict__ offset) {
+  const int c = blockIdx.x, h = sizes.h;
   double* rs = rowstats + (size_t)c * h * 3;
   float e = 0.f, s = 0.f;
-  const double sum = projection_norm_constants(rs, h, norm_h, norm_w, &e, &s);
+  const double sum = projection_norm_constants(rs, sizes, &e, &s);
   __syncwarp();
   if (threadIdx.x == 0) {
     *reinterpret_cast<float2*>(rs) = make_float2(e, s);
@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(32)
 
 int launch_norm_constants(double* rowstats, int n_c, int h, int norm_h, int norm_w, cudaStream_t s, const float2* dc,
                           size_t dc_stride, float scale, float* offset) {
-  norm_constants_kernel<<<n_c, 32, 0, s>>>(rowstats, h, norm_h, norm_w, dc, dc_stride, scale, offset);
+  norm_constants_kernel<<<n_c, 32, 0, s>>>(rowstats, NormSizes(h, norm_h, norm_w), dc, dc_stride, scale, offset);
   return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
 }
 
@@ -115,7 +115,7 @@ static int pad_rfft_t(const float* proj, const double* rowstats, int h, int norm
     }
     dim3 grid(ctas, n_c);
     // shared twiddle tables where a CTA transforms >= 4 rows
-    pad_rfft_kernel<WH, ROWS, (ROWS >= 4)><<<grid, ROWS * NT, 0, s>>>(proj, rowstats, h, norm_h, norm_w, Wcp,
+    pad_rfft_kernel<WH, ROWS, (ROWS >= 4)><<<grid, ROWS * NT, 0, s>>>(proj, rowstats, h, NormSizes(h, norm_h, norm_w), Wcp,
                                                                       ready, static_cast<float2*>(A));
     return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
   }

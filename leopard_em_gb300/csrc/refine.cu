@@ -22,32 +22,28 @@
 
 namespace lgb {
 
-__device__ inline void euler_zyz_d(const float* e, double* R) {
-  const double k = 3.14159265358979323846 / 180.0;
-  double sp, cp, st, ct, ss, cs;
-  sincos((double)e[0] * k, &sp, &cp);
-  sincos((double)e[1] * k, &st, &ct);
-  sincos((double)e[2] * k, &ss, &cs);
-  R[0] = cp * ct * cs - sp * ss;
-  R[1] = -cp * ct * ss - sp * cs;
-  R[2] = cp * st;
-  R[3] = sp * ct * cs + cp * ss;
-  R[4] = -sp * ct * ss + cp * cs;
-  R[5] = sp * st;
-  R[6] = -st * cs;
-  R[7] = st * ss;
-  R[8] = ct;
-}
-
-// rot[(p*nb + b)*9] = R(offsets[o0 + b]) @ R(euler[p])
-__global__ void refine_rotations_kernel(const float* __restrict__ euler, const float* __restrict__ offsets, int o0,
-                                        int nb, int n_particles, float* __restrict__ rot) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n_particles * nb) return;
-  const int p = i / nb, b = i % nb;
+// rot[(p*nb + b)*9] = R(offsets[o0 + b]) @ R(euler[p]): 32 rotations a CTA, a
+// thread an angle, then a thread a rotation (all six FP64 sincos in one thread:
+// 9.6 us for 32 rotations, 5.6 now).
+constexpr int kRotations = 32;
+__global__ void __launch_bounds__(6 * kRotations)
+    refine_rotations_kernel(const float* __restrict__ euler, const float* __restrict__ offsets, int o0, int nb,
+                            int n_particles, float* __restrict__ rot) {
+  __shared__ SinCos angle[kRotations][6];
+  const int n = n_particles * nb, first = blockIdx.x * kRotations;
+  {
+    const int item = threadIdx.x / 6, k = threadIdx.x % 6, i = first + item;
+    if (i < n) {
+      const int p = i / nb, b = i % nb;
+      angle[item][k] = sincos_degrees(k < 3 ? offsets[3 * (size_t)(o0 + b) + k] : euler[3 * (size_t)p + k - 3]);
+    }
+  }
+  __syncthreads();
+  const int i = first + threadIdx.x;
+  if (threadIdx.x >= kRotations || i >= n) return;
   double A[9], B[9];
-  euler_zyz_d(offsets + 3 * (size_t)(o0 + b), A);
-  euler_zyz_d(euler + 3 * (size_t)p, B);
+  rotmat_zyz(angle[threadIdx.x], A);
+  rotmat_zyz(angle[threadIdx.x] + 3, B);
 #pragma unroll
   for (int r = 0; r < 3; ++r)
 #pragma unroll
@@ -496,7 +492,8 @@ int lgb_refine_search(const lgb_refine_problem* p, const lgb_ctf_params* ctf, co
     const int nb = (p->n_offsets - o0) < p->offset_batch ? (p->n_offsets - o0) : p->offset_batch;
     const int n_cpp = L.n_cd * nb;
     const int n_c = P * n_cpp;
-    refine_rotations_kernel<<<(P * nb + 127) / 128, 128, 0, s>>>(euler_angles, euler_offsets, o0, nb, P, rot);
+    refine_rotations_kernel<<<(P * nb + kRotations - 1) / kRotations, 6 * kRotations, 0, s>>>(
+        euler_angles, euler_offsets, o0, nb, P, rot);
     if (cudaGetLastError() != cudaSuccess) return LGB_ERR_CUDA;
     {
       StageScope sc(LGB_STAGE_SLICE, s, prof);
