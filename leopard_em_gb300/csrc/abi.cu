@@ -116,7 +116,10 @@ static int grid_for(long long n) {
 }
 
 __global__ void set_cursor_kernel(int* cursor, int value) { *cursor = value; }
-__global__ void advance_cursor_kernel(int* cursor, int step) { *cursor += step; }
+__global__ void advance_cursor_kernel(int* cursor, int step) {
+  chain_wait();
+  *cursor += step;
+}
 
 // Validated pointers and layout of one search call.
 struct SearchArgs {
@@ -364,8 +367,7 @@ int lgb_match_search_graph(const lgb_match_problem* p, const void* template_dft,
       for (int m = 0; m < batches_per_graph && st == LGB_OK; ++m)
         st = run_batch(a, m * p->orientation_batch, cursor, p->orientation_batch, false, cs);
       if (st == LGB_OK) {
-        advance_cursor_kernel<<<1, 1, 0, cs>>>(cursor, (int)chunk);
-        if (cudaGetLastError() != cudaSuccess) st = LGB_ERR_CUDA;
+        st = launch_chained(advance_cursor_kernel, dim3(1), dim3(1), 0, cs, cursor, (int)chunk);
       }
       if (cudaStreamEndCapture(cs, &graph) != cudaSuccess && st == LGB_OK) st = LGB_ERR_CUDA;
     }

@@ -48,10 +48,9 @@ static int colpass_tab_t(const void* A, const void* Ip, int ips, int h, int Wcp,
   int per = 1;
   const int groups = (Wcp + CT::G - 1) / CT::G;
   const int split = colpass_split(groups, n_c, waves, &per);
-  colpass_tab_kernel<HN><<<dim3(groups, split), CT::G * CT::NT, CT::SMEM, s>>>(
-      static_cast<const float2*>(A), static_cast<const float2*>(Ip), ips, h, Wcp, n_c, per, cpi, y_rows,
-      static_cast<float2*>(Y));
-  return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
+  return launch_chained(colpass_tab_kernel<HN>, dim3(groups, split), dim3(CT::G * CT::NT), CT::SMEM, s,
+                        static_cast<const float2*>(A), static_cast<const float2*>(Ip), ips, h, Wcp, n_c, per, cpi,
+                        y_rows, static_cast<float2*>(Y));
 }
 
 template <int R, int P>
@@ -65,10 +64,9 @@ static int colpass_fused_t(const void* A, const void* Ip, int ips, int h, int Wc
   const int groups = Wcp / kColGroup;
   const int split = colpass_split(groups, n_c, waves, &per);
   dim3 grid(groups, split);
-  colpass_fused_kernel<R, P><<<grid, CF::THREADS, CF::SMEM, s>>>(
-      static_cast<const float2*>(A), static_cast<const float2*>(Ip), ips, h, Wcp, n_c, per, cpi, y_rows,
-      static_cast<float2*>(Y));
-  return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
+  return launch_chained(colpass_fused_kernel<R, P>, grid, dim3(CF::THREADS), CF::SMEM, s,
+                        static_cast<const float2*>(A), static_cast<const float2*>(Ip), ips, h, Wcp, n_c, per, cpi,
+                        y_rows, static_cast<float2*>(Y));
 }
 
 template <int R1, int R2>
@@ -82,10 +80,9 @@ static int colpass_pair_t(const void* A, const void* Ip, int ips, int h, int Wcp
   int per = 1;
   const int groups = (Wcp + CP::G - 1) / CP::G;
   const int split = colpass_split(groups, n_c, waves, &per);
-  kernel<<<dim3(groups, split), CP::THREADS, CP::SMEM, s>>>(
-      static_cast<const float2*>(A), static_cast<const float2*>(Ip), ips, h, Wcp, n_c, per, cpi, y_rows,
-      static_cast<float2*>(Y), norm, norm_stride, norm_w);
-  return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
+  return launch_chained(kernel, dim3(groups, split), dim3(CP::THREADS), CP::SMEM, s, static_cast<const float2*>(A),
+                        static_cast<const float2*>(Ip), ips, h, Wcp, n_c, per, cpi, y_rows, static_cast<float2*>(Y), norm,
+                        norm_stride, norm_w);
 }
 
 int launch_colpass(int H, const void* A, const void* Ip, int ips, int h, int Wcp, int n_c, int cpi, int y_rows, int waves,

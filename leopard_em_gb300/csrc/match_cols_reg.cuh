@@ -133,18 +133,6 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
                        : make_float2(0.f, 0.f);
     }
   };
-  if (SPARSE && c_begin < c_end) fetch(c_begin);
-  // the first image's columns come in while the roots are computed
-  int image = c_begin / c_per_image;
-  float2 first[R2];
-  {
-    const float2* ip = Ip + (size_t)image * N * ips + kx;
-#pragma unroll
-    for (int s = 0; s < R2; ++s) {
-      const int row = t + R1 * DftNT<C::R2A, C::R2B, -1>::out(s);
-      first[s] = (kx < ips && act2 && c_begin < c_end) ? __ldg(ip + (size_t)row * ips) : make_float2(0.f, 0.f);
-    }
-  }
   if constexpr (C::TWO) {
     auto fill = [&](float2* dst, int r_hi, int nb) {  // rows 0..7: r, rows 8..: 8 (row - 8)
       for (int e = threadIdx.x; e < (8 + r_hi) * nb; e += C::THREADS) {
@@ -162,6 +150,20 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
       float sn, cs;
       sincospif(2.0f * (float)(r * b) / (float)N, &sn, &cs);
       tab[r * C::TS + b] = make_float2(cs, -sn);
+    }
+  }
+  chain_wait();
+  LGB_CHAIN_INPUT(A);
+  LGB_CHAIN_INPUT(Ip);
+  if (SPARSE && c_begin < c_end) fetch(c_begin);
+  int image = c_begin / c_per_image;
+  float2 first[R2];
+  {
+    const float2* ip = Ip + (size_t)image * N * ips + kx;
+#pragma unroll
+    for (int s = 0; s < R2; ++s) {
+      const int row = t + R1 * DftNT<C::R2A, C::R2B, -1>::out(s);
+      first[s] = (kx < ips && act2 && c_begin < c_end) ? __ldg(ip + (size_t)row * ips) : make_float2(0.f, 0.f);
     }
   }
   tmem_barrier();
@@ -312,10 +314,9 @@ int colpass_reg_launch(const void* A, const void* Ip, int ips, int h, int Wcp, i
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int groups = (Wcp + C::G - 1) / C::G;
   const int per = colpass_per_block(groups, n_c, sms * C::MINB, waves);
-  colpass_reg_kernel<C, SPARSE><<<dim3(groups, (n_c + per - 1) / per), C::THREADS, C::SMEM, s>>>(
-      static_cast<const float2*>(A), static_cast<const float2*>(Ip), ips, h, Wcp, n_c, per, cpi, y_rows,
-      static_cast<float2*>(Y));
-  return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
+  return launch_chained(colpass_reg_kernel<C, SPARSE>, dim3(groups, (n_c + per - 1) / per), dim3(C::THREADS), C::SMEM, s,
+                        static_cast<const float2*>(A), static_cast<const float2*>(Ip), ips, h, Wcp, n_c, per, cpi,
+                        y_rows, static_cast<float2*>(Y));
 }
 
 // The sparse form reads inputs q < R1B only: rows h <= R1B R2.  Templates have

@@ -95,6 +95,9 @@ __global__ void __launch_bounds__(ColFused<R, P>::THREADS, 1)
   const int c_end = min(n_c, c_begin + c_per_block);
   // first-pass sparse form: at most two non-zero inputs per butterfly when h <= 2*NB
   const bool sparse = h <= 2 * NB;
+  chain_wait();
+  LGB_CHAIN_INPUT(A);
+  LGB_CHAIN_INPUT(Ip);
   __syncthreads();
 
   const int fj = IdxPad16::f(j);
@@ -208,6 +211,9 @@ __global__ void __launch_bounds__(ColTab<HN>::G* ColTab<HN>::NT)
   const int c_end = min(n_c, c_begin + c_per_block);
   const int g = threadIdx.x / NT, t = threadIdx.x - (threadIdx.x / NT) * NT;
   float2* x = ctsm + g * STRIDE;
+  chain_wait();
+  LGB_CHAIN_INPUT(A);
+  LGB_CHAIN_INPUT(Ip);
   __syncthreads();
 #pragma unroll 1
   for (int c = c_begin; c < c_end; ++c) {
@@ -306,6 +312,10 @@ __global__ void __launch_bounds__(ColPair<R1, R2>::THREADS, 4)
       U = make_float2(ca * mag, -sa * mag);
     }
   }
+  chain_wait();
+  LGB_CHAIN_INPUT(A);
+  LGB_CHAIN_INPUT(Ip);
+  LGB_CHAIN_INPUT(norm);
   __syncthreads();
 #pragma unroll 1
   for (int c = c_begin; c < c_end; ++c) {

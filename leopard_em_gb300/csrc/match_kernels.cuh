@@ -23,6 +23,7 @@
 // the column pass, colpass_pair_kernel in match_fused.cuh).
 #pragma once
 
+#include "chain.cuh"
 #include "fft.cuh"
 #include "reg_dft.cuh"
 
@@ -69,6 +70,9 @@ __global__ void __launch_bounds__(COLS* FftThreads<HT>::value)
   constexpr int WC = HT / 2 + 1;
   constexpr int STRIDE = IdxPad16::pad(HT) + 2;
   __shared__ float2 buf[COLS * STRIDE];
+  chain_wait();
+  LGB_CHAIN_INPUT(slices);
+  LGB_CHAIN_INPUT(pf);
   // c = (p*n_cd + cd)*nb + b: slices are per (p, b), filters per (p, cd)
   const int c = blockIdx.y;
   const int pc = c / nb, b = c - (c / nb) * nb;
@@ -126,6 +130,9 @@ __global__ void __launch_bounds__(ProjColPair<R1, R2>::G* ProjColPair<R1, R2>::N
     sincospif(2.0f * (float)m / (float)HT, &sn, &cs);
     root[m] = make_float2(cs, sn);
   }
+  chain_wait();
+  LGB_CHAIN_INPUT(slices);
+  LGB_CHAIN_INPUT(pf);
   // c = (p*n_cd + cd)*nb + b: slices are per (p, b), filters per (p, cd)
   const int c = blockIdx.y;
   const int pc = c / nb, b = c - (c / nb) * nb;
@@ -182,6 +189,8 @@ __global__ void __launch_bounds__(ROWS* FftThreads<HT / 2>::value)
   __shared__ float2 xin[ROWS][WC];
   __shared__ float2 z[ROWS][ZS];
   __shared__ float part[ROWS * NT][3];
+  chain_wait();
+  LGB_CHAIN_INPUT(T);
   const int c = blockIdx.y;
   const int g = threadIdx.x / NT, t = threadIdx.x - (threadIdx.x / NT) * NT;
   const int row0 = blockIdx.x * ROWS;
@@ -279,6 +288,8 @@ __global__ void __launch_bounds__(ROWS* R1)
     sincospif(2.0f * (float)m / (float)M, &sn, &cs);
     root[m] = make_float2(cs, sn);
   }
+  chain_wait();
+  LGB_CHAIN_INPUT(T);
   const int c = blockIdx.y;
   const int g = threadIdx.x / NT, t = threadIdx.x - (threadIdx.x / NT) * NT;
   const int row0 = blockIdx.x * ROWS;
@@ -413,6 +424,8 @@ __global__ void __launch_bounds__(ROWS * 16, 48 / ROWS)
     rootr[r] = m <= WH ? v : make_float2(-v.x, -v.y);
   }
   const float2 prej = pre[threadIdx.x % C2], postj = post[t];
+  chain_wait();
+  LGB_CHAIN_INPUT(T);
 #pragma unroll 1
   for (int grp = 0; grp < groups; ++grp) {
     const int row0 = (blockIdx.x * groups + grp) * ROWS;
@@ -604,6 +617,9 @@ __global__ void __launch_bounds__(ROWS* FftThreads<WH>::value)
     }
   }
   const int c = blockIdx.y;
+  chain_wait();
+  LGB_CHAIN_INPUT(proj);
+  LGB_CHAIN_INPUT(rowstats);
   // norm_ready: constants (e, s) precomputed by norm_constants_kernel as a
   // float2 over rowstats[c][0][0]; otherwise warp 0 reduces the row moments here
   __shared__ float norm[2];
@@ -683,6 +699,9 @@ __global__ void __launch_bounds__(ROWS* FftThreads<WH>::value, (PadRows<WH, ROWS
     sincospif((float)k / (float)WH, &sn, &cs);
     post[k] = make_float2(cs, -sn);
   }
+  chain_wait();
+  LGB_CHAIN_INPUT(proj);
+  LGB_CHAIN_INPUT(rowstats);
   const int c = blockIdx.y;
   const float2 es = *reinterpret_cast<const float2*>(rowstats + (size_t)c * h * 3);
   const float e = es.x, s = es.y;
@@ -762,6 +781,8 @@ __global__ void __launch_bounds__(NT, 2)
     sincospif((float)k / (float)WH, &sn, &cs);
     pre[k] = make_float2(cs, sn);
   }
+  chain_wait();
+  LGB_CHAIN_INPUT(Y);
   float bmax[2 * PIX], bs[2 * PIX], bss[2 * PIX];
   int barg[2 * PIX];
 #pragma unroll

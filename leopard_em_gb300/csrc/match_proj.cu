@@ -20,6 +20,10 @@ __global__ void __launch_bounds__(256)
     slice_kernel(const float2* __restrict__ vol, int d, const float* __restrict__ euler, int o0,
                  const int* __restrict__ o0_dev, const float* __restrict__ rotations, int tiles,
                  float2* __restrict__ slices) {
+  chain_wait();
+  LGB_CHAIN_INPUT(vol);
+  LGB_CHAIN_INPUT(euler);
+  LGB_CHAIN_INPUT(rotations);
   const int b = blockIdx.y;
   __shared__ float R[9];
   __shared__ SinCos angle[3];
@@ -92,9 +96,8 @@ int launch_slice(const void* vol, int d, const float* euler, int o0, const int* 
                  const float* rotations, void* slices, cudaStream_t s) {
   const int tiles = (d / 2 + 1 + 7) / 8, patches = tiles * ((d + 3) / 4);
   dim3 grid((patches + 7) / 8, nb);
-  slice_kernel<<<grid, 256, 0, s>>>(static_cast<const float2*>(vol), d, euler, o0, o0_dev, rotations, tiles,
-                                    static_cast<float2*>(slices));
-  return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
+  return launch_chained(slice_kernel, grid, dim3(256), 0, s, static_cast<const float2*>(vol), d, euler, o0, o0_dev,
+                        rotations, tiles, static_cast<float2*>(slices));
 }
 
 constexpr int kProjCols = 8;
@@ -107,14 +110,12 @@ static int proj_col_t(const void* slices, const float* pf, int nb, int n_cd, int
     // two register passes (16 x 16), 8 columns per CTA
     using PC = ProjColPair<16, 16>;
     dim3 pgrid((WC + PC::G - 1) / PC::G, n_c);
-    proj_col_pair_kernel<16, 16><<<pgrid, PC::G * PC::NT, 0, s>>>(static_cast<const float2*>(slices), pf, nb, n_cd,
-                                                                  static_cast<float2*>(T));
-    return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
+    return launch_chained(proj_col_pair_kernel<16, 16>, pgrid, dim3(PC::G * PC::NT), 0, s,
+                          static_cast<const float2*>(slices), pf, nb, n_cd, static_cast<float2*>(T));
   }
   dim3 grid((WC + kProjCols - 1) / kProjCols, n_c);
-  proj_col_kernel<HT, kProjCols><<<grid, kProjCols * FftThreads<HT>::value, 0, s>>>(
-      static_cast<const float2*>(slices), pf, nb, n_cd, static_cast<float2*>(T));
-  return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
+  return launch_chained(proj_col_kernel<HT, kProjCols>, grid, dim3(kProjCols * FftThreads<HT>::value), 0, s,
+                        static_cast<const float2*>(slices), pf, nb, n_cd, static_cast<float2*>(T));
 }
 
 template <int HT>
@@ -123,13 +124,11 @@ static int proj_row_t(const void* T, int n_c, float* proj, double* rowstats, cud
   dim3 grid(HT / kProjRows, n_c);
   if constexpr (HT == 256) {
     // two register passes (16 x 8) of the 128-point c2r, 16 threads per row
-    proj_row_pair_kernel<16, 8, kProjRows><<<grid, kProjRows * 16, 0, s>>>(static_cast<const float2*>(T), proj,
-                                                                           rowstats);
-    return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
+    return launch_chained(proj_row_pair_kernel<16, 8, kProjRows>, grid, dim3(kProjRows * 16), 0, s,
+                          static_cast<const float2*>(T), proj, rowstats);
   }
-  proj_row_kernel<HT, kProjRows><<<grid, kProjRows * FftThreads<HT / 2>::value, 0, s>>>(
-      static_cast<const float2*>(T), proj, rowstats);
-  return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
+  return launch_chained(proj_row_kernel<HT, kProjRows>, grid, dim3(kProjRows * FftThreads<HT / 2>::value), 0, s,
+                        static_cast<const float2*>(T), proj, rowstats);
 }
 
 bool supported_proj_row_rfft(int h, int W) { return h == 256 && W == 288; }
@@ -145,9 +144,8 @@ int launch_proj_row_rfft(int h, int W, const void* T, int n_c, double* rowstats,
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   int groups = 8;
   while (groups > 1 && (long long)n_c * (256 / (ROWS * groups)) < 12LL * sms) groups /= 2;
-  proj_row_rfft_kernel<ROWS><<<dim3(256 / (ROWS * groups), n_c), ROWS * 16, 0, s>>>(
-      static_cast<const float2*>(T), rowstats, Wcp, groups, static_cast<float2*>(A));
-  return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
+  return launch_chained(proj_row_rfft_kernel<ROWS>, dim3(256 / (ROWS * groups), n_c), dim3(ROWS * 16), 0, s,
+                        static_cast<const float2*>(T), rowstats, Wcp, groups, static_cast<float2*>(A));
 }
 
 int launch_proj_col(int h, const void* slices, const float* pf, int nb, int n_cd, int n_c, void* T, cudaStream_t s) {

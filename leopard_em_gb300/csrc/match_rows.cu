@@ -40,6 +40,8 @@ int launch_repack_rows(const void* src, long long rows, int wc, int wcp, void* d
 __global__ void __launch_bounds__(32)
     norm_constants_kernel(double* __restrict__ rowstats, NormSizes sizes, const float2* __restrict__ dc, size_t dc_stride,
                           float scale, float* __restrict__ offset) {
+  chain_wait();
+  LGB_CHAIN_INPUT(dc);
   const int c = blockIdx.x, h = sizes.h;
   double* rs = rowstats + (size_t)c * h * 3;
   float e = 0.f, s = 0.f;
@@ -56,8 +58,8 @@ __global__ void __launch_bounds__(32)
 
 int launch_norm_constants(double* rowstats, int n_c, int h, int norm_h, int norm_w, cudaStream_t s, const float2* dc,
                           size_t dc_stride, float scale, float* offset) {
-  norm_constants_kernel<<<n_c, 32, 0, s>>>(rowstats, NormSizes(h, norm_h, norm_w), dc, dc_stride, scale, offset);
-  return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
+  return launch_chained(norm_constants_kernel, dim3(n_c), dim3(32), 0, s, rowstats, NormSizes(h, norm_h, norm_w), dc,
+                        dc_stride, scale, offset);
 }
 
 
@@ -95,9 +97,8 @@ static int pad_rfft_t(const float* proj, const double* rowstats, int h, int norm
     if (cudaFuncSetAttribute(pad_rfft_rows_kernel<WH, ROWS, RPC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)PR::SMEM) != cudaSuccess)
       return LGB_ERR_CUDA;
-    pad_rfft_rows_kernel<WH, ROWS, RPC><<<dim3((h + RPC - 1) / RPC, n_c), ROWS * NT, PR::SMEM, s>>>(
-        proj, rowstats, h, Wcp, static_cast<float2*>(A));
-    return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
+    return launch_chained(pad_rfft_rows_kernel<WH, ROWS, RPC>, dim3((h + RPC - 1) / RPC, n_c), dim3(ROWS * NT), PR::SMEM,
+                          s, proj, rowstats, h, Wcp, static_cast<float2*>(A));
   } else {
     // at least one full warp: the normalisation reduction shuffles across warp 0
     constexpr int ROWS0 = NT >= 128 ? 2 : (NT >= 32 ? 4 : (NT >= 16 ? 8 : 16));
@@ -115,9 +116,8 @@ static int pad_rfft_t(const float* proj, const double* rowstats, int h, int norm
     }
     dim3 grid(ctas, n_c);
     // shared twiddle tables where a CTA transforms >= 4 rows
-    pad_rfft_kernel<WH, ROWS, (ROWS >= 4)><<<grid, ROWS * NT, 0, s>>>(proj, rowstats, h, NormSizes(h, norm_h, norm_w), Wcp,
-                                                                      ready, static_cast<float2*>(A));
-    return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
+    return launch_chained(pad_rfft_kernel<WH, ROWS, (ROWS >= 4)>, grid, dim3(ROWS * NT), 0, s, proj, rowstats, h,
+                          NormSizes(h, norm_h, norm_w), Wcp, ready, static_cast<float2*>(A));
   }
 }
 
@@ -130,9 +130,8 @@ static int rowpass_t(const void* Y, int H, int y_rows, int Wcp, int n_c, int nb,
       cudaSuccess)
     return LGB_ERR_CUDA;
   const float scale = 1.0f / ((float)H * (float)(2 * WH));
-  rowpass_kernel<WH, NT><<<y_rows, NT, SMEM, s>>>(static_cast<const float2*>(Y), y_rows, Wcp, n_c, nb, n_orient,
-                                                  o0, o0_dev, scale, mip, best, s1, s2);
-  return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
+  return launch_chained(rowpass_kernel<WH, NT>, dim3(y_rows), dim3(NT), SMEM, s, static_cast<const float2*>(Y), y_rows,
+                        Wcp, n_c, nb, n_orient, o0, o0_dev, scale, mip, best, s1, s2);
 }
 
 int launch_pad_rfft(int W, const float* proj, const double* rowstats, int h, int norm_h, int norm_w, int Wcp,

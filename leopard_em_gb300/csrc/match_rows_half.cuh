@@ -72,7 +72,6 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
     }
     cp_async_commit();
   };
-  stage(blockIdx.x * ROWS + g, c0);
   FillTables<WH, 1, RL>::run(tab, threadIdx.x, C::THREADS);
   // c2r pre-twiddle exp(+i pi k / WH) at k = j + q NB1: exp(i pi j / WH), kept
   // in registers, times the constant exp(i pi q / R1)
@@ -84,6 +83,9 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
     prej[p] = make_float2(cs, sn);
   }
   const float2* tab_last = tab + TableSize<1, typename DropLast<RL>::type>::value;
+  chain_wait();
+  LGB_CHAIN_INPUT(Y);
+  stage(blockIdx.x * ROWS + g, c0);
   if (o0_dev) o0 += *o0_dev;
   const float scale2 = scale * scale;
 #pragma unroll 1
@@ -274,9 +276,8 @@ int rowpass_half_launch(const void* Y, int H, int y_rows, int n_c, int nb, int n
     return LGB_ERR_CUDA;
   const float scale = 1.0f / ((float)H * (float)(2 * C::WH));
   const int groups = (y_rows + C::ROWS - 1) / C::ROWS, ctas = sms * C::MINB;
-  rowpass_half_kernel<C><<<groups < ctas ? groups : ctas, C::THREADS, C::SMEM, s>>>(
-      static_cast<const float2*>(Y), y_rows, n_c, nb, n_orient, o0, o0_dev, scale, mip, best, s1, s2);
-  return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
+  return launch_chained(rowpass_half_kernel<C>, dim3(groups < ctas ? groups : ctas), dim3(C::THREADS), C::SMEM, s,
+                        static_cast<const float2*>(Y), y_rows, n_c, nb, n_orient, o0, o0_dev, scale, mip, best, s1, s2);
 }
 
 // C, or the first of the SPLIT forms in Cs (most groups first) whose rows are

@@ -30,6 +30,9 @@ __global__ void __launch_bounds__(6 * kRotations)
     refine_rotations_kernel(const float* __restrict__ euler, const float* __restrict__ offsets, int o0, int nb,
                             int n_particles, float* __restrict__ rot) {
   __shared__ SinCos angle[kRotations][6];
+  chain_wait();
+  LGB_CHAIN_INPUT(euler);
+  LGB_CHAIN_INPUT(offsets);
   const int n = n_particles * nb, first = blockIdx.x * kRotations;
   {
     const int item = threadIdx.x / 6, k = threadIdx.x % 6, i = first + item;
@@ -154,6 +157,10 @@ __global__ void __launch_bounds__(ROWS* R1, 3)
     red_key[0] = 0ull;
     red_cc[0] = 0u;
   }
+  chain_wait();
+  LGB_CHAIN_INPUT(Y);
+  LGB_CHAIN_INPUT(corr_mean);
+  LGB_CHAIN_INPUT(corr_std);
   const int y = blockIdx.x, p = blockIdx.y;
   const int g = threadIdx.x / NT, t = threadIdx.x - (threadIdx.x / NT) * NT;
   unsigned long long best_key = 0ull;
@@ -229,6 +236,7 @@ __global__ void __launch_bounds__(ROWS* R1, 3)
 // then reset of the batch slots.
 __global__ void refine_commit_kernel(int P, unsigned long long* slot_key, unsigned* slot_cc, int o0, int nb,
                                      float* best_z, float* best_cc, int* best_flat, int* best_o0, int* best_nb) {
+  chain_wait();
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= P) return;
   const unsigned long long key = slot_key[p];
@@ -257,6 +265,12 @@ __global__ void refine_collect_kernel(int P, int crop_w, int n_cd, int D, const 
                                       const float* __restrict__ euler, const float* __restrict__ offsets,
                                       const float* __restrict__ defocus, const float* __restrict__ pixel,
                                       unsigned* __restrict__ packed) {
+  chain_wait();
+  LGB_CHAIN_INPUT(raw);
+  LGB_CHAIN_INPUT(euler);
+  LGB_CHAIN_INPUT(offsets);
+  LGB_CHAIN_INPUT(defocus);
+  LGB_CHAIN_INPUT(pixel);
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= P) return;
   const int flat = (int)raw[2 * (size_t)P + p], o0 = (int)raw[3 * (size_t)P + p];
@@ -331,9 +345,9 @@ static int refine_rowpass_t(const void* Y, int y_rows, int Wcp, int n_cpp, int P
                             cudaStream_t s) {
   const int per = 2 * ROWS;  // two steps per CTA
   dim3 grid(crop_h, P, (n_cpp + per - 1) / per);
-  refine_rowpass_pair_kernel<R1, R2, ROWS><<<grid, ROWS * R1, 0, s>>>(
-      static_cast<const float2*>(Y), y_rows, Wcp, n_cpp, per, crop_w, scale, mean, std_, crop_h, key, cc);
-  return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
+  return launch_chained(refine_rowpass_pair_kernel<R1, R2, ROWS>, grid, dim3(ROWS * R1), 0, s,
+                        static_cast<const float2*>(Y), y_rows, Wcp, n_cpp, per, crop_w, scale, mean, std_, crop_h, key,
+                        cc);
 }
 
 int launch_refine_rowpass(int W, const void* Y, int y_rows, int Wcp, int n_cpp, int P, int crop_h, int crop_w,
@@ -492,9 +506,9 @@ int lgb_refine_search(const lgb_refine_problem* p, const lgb_ctf_params* ctf, co
     const int nb = (p->n_offsets - o0) < p->offset_batch ? (p->n_offsets - o0) : p->offset_batch;
     const int n_cpp = L.n_cd * nb;
     const int n_c = P * n_cpp;
-    refine_rotations_kernel<<<(P * nb + kRotations - 1) / kRotations, 6 * kRotations, 0, s>>>(
-        euler_angles, euler_offsets, o0, nb, P, rot);
-    if (cudaGetLastError() != cudaSuccess) return LGB_ERR_CUDA;
+    if ((st = launch_chained(refine_rotations_kernel, dim3((P * nb + kRotations - 1) / kRotations),
+                             dim3(6 * kRotations), 0, s, euler_angles, euler_offsets, o0, nb, P, rot)))
+      return st;
     {
       StageScope sc(LGB_STAGE_SLICE, s, prof);
       if ((st = launch_slice(template_dft, d, nullptr, 0, nullptr, P * nb, rot, slices, s))) return st;
@@ -541,9 +555,9 @@ int lgb_refine_search(const lgb_refine_problem* p, const lgb_ctf_params* ctf, co
                                       corr_std, key, cc, s)))
         return st;
     }
-    refine_commit_kernel<<<(P + 127) / 128, 128, 0, s>>>(P, key, cc, o0, nb, best_z, best_cc, best_flat,
-                                                           best_offset_begin, best_batch_len);
-    if (cudaGetLastError() != cudaSuccess) return LGB_ERR_CUDA;
+    if ((st = launch_chained(refine_commit_kernel, dim3((P + 127) / 128), dim3(128), 0, s,
+                             P, key, cc, o0, nb, best_z, best_cc, best_flat, best_offset_begin, best_batch_len)))
+      return st;
   }
   return LGB_OK;
 }
@@ -555,10 +569,10 @@ int lgb_refine_collect(int n_particles, int crop_w, int n_pixel_sizes, int n_def
   if (n_particles < 0 || crop_w < 1 || n_pixel_sizes < 1 || n_defocus < 1 || !raw || !euler_angles || !euler_offsets ||
       !defocus_offsets || !pixel_size_offsets || !packed)
     return LGB_ERR_INVALID_ARGUMENT;
-  refine_collect_kernel<<<(n_particles + 63) / 64, 64, 0, (cudaStream_t)stream>>>(
-      n_particles, crop_w, n_pixel_sizes * n_defocus, n_defocus, static_cast<const unsigned*>(raw), euler_angles,
-      euler_offsets, defocus_offsets, pixel_size_offsets, static_cast<unsigned*>(packed));
-  return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
+  return launch_chained(refine_collect_kernel, dim3((n_particles + 63) / 64), dim3(64), 0, (cudaStream_t)stream,
+                        n_particles, crop_w, n_pixel_sizes * n_defocus, n_defocus, static_cast<const unsigned*>(raw),
+                        euler_angles, euler_offsets, defocus_offsets, pixel_size_offsets,
+                        static_cast<unsigned*>(packed));
 }
 
 int lgb_refine_decode(int n_particles, int crop_h, int crop_w, const void* packed, const double* euler_angles,

@@ -22,6 +22,9 @@ __global__ void __launch_bounds__(NT) rowstore_kernel(const float2* __restrict__
   constexpr int ZS = IdxPad16::pad(WH) + 2;
   __shared__ float2 xr[WH + 4];
   __shared__ float2 z[ZS];
+  chain_wait();
+  LGB_CHAIN_INPUT(Y);
+  LGB_CHAIN_INPUT(offset);
   const int y = blockIdx.x, p = blockIdx.y, t = threadIdx.x;
   const float2* row = Y + ((size_t)p * y_rows + y) * Wcp;
   for (int k = t; k <= WH; k += NT) xr[k] = row[k];
@@ -69,9 +72,8 @@ template <int WH>
 static int rowstore_t(const void* Y, int y_rows, int Wcp, int P, float scale, const float* off, int out_w, float* out,
                       cudaStream_t s) {
   constexpr int NT = row_threads(WH) > FftThreads<WH>::value ? row_threads(WH) : FftThreads<WH>::value;
-  rowstore_kernel<WH, NT><<<dim3(y_rows, P), NT, 0, s>>>(static_cast<const float2*>(Y), y_rows, Wcp, scale, off,
-                                                         out_w, out);
-  return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
+  return launch_chained(rowstore_kernel<WH, NT>, dim3(y_rows, P), dim3(NT), 0, s, static_cast<const float2*>(Y), y_rows,
+                        Wcp, scale, off, out_w, out);
 }
 
 static int launch_rowstore(int W, const void* Y, int y_rows, int Wcp, int P, float scale, const float* off, int out_w,
