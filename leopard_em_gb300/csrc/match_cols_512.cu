@@ -10,8 +10,8 @@ namespace lgb {
 // h 64: 32 correlograms 32.0 -> 26.9, 8: 18.0 -> 16.0, 1: 13.2 -> 13.9;
 // h 256: 32: 35 -> 31, 1: 13.5 -> 16.4; h 384, 80 per image: 320: 233 -> 171.
 // (The split may not depend on the batch: a correlogram's bits would.)
-int launch_colpass_512(const void* A, const void* Ip, int ips, int h, int Wcp, int n_c, int cpi, int y_rows, int waves, void* Y,
-                       cudaStream_t s) {
+int launch_colpass_512(const void* A, const void* Ip, int ips, int h, int Wcp, int n_c, int cpi, int y_rows,
+                        int waves, void* Y, cudaStream_t s) {
   if (h <= 64)
     return colpass_reg_launch<ColReg<8, 4, 2, 8, 32, 8, 2>, true>(A, Ip, ips, h, Wcp, n_c, cpi, y_rows, waves, Y, s);
   return colpass_reg_t<ColReg<2, 8, 4, 8, 16, 8, 4>>(A, Ip, ips, h, Wcp, n_c, cpi, y_rows, waves, Y, s);

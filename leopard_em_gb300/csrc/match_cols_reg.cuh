@@ -25,8 +25,12 @@
 //   4096 x 2049, h 384: 41.6 -> 31.6    3840 x 1921, h 256: 84 -> 33.5
 //   3072 x 1441, h 256: 40 -> 21        2880 x 1441, h 256: 64 -> 23
 //   2048 x 1025, h 256: 18.1 -> 8.5     1024 x 513, h 128: 5.2 -> 2.0
-//   576 x 289, h 128: 2.4 -> 0.7        5760 x 2049, h 256: 177 -> 95
-// (5760 rows leave 200 registers to 80-point transforms and spill.)
+//   576 x 289, h 128: 2.4 -> 0.7        5760 x 2049, h 256: 177 -> 70
+// 5760 rows take ten warps of 168 registers and 150 KB of code in the loop, more
+// than the instruction caches hold.  Their split 80 x 72 (the larger radix where
+// no image and roots are held) spills 460 bytes and measured 70 us, 72 x 80 85;
+// 64 x 90 in eight warps of 255 registers 122 (260 KB of code), three columns a
+// CTA 165 (24-byte row pieces), both directions in one code path 73.
 #pragma once
 
 #include "reg_dft.cuh"
@@ -35,8 +39,8 @@
 
 namespace lgb {
 
-// TWO: w^(r b) as a product of w^(r0 b) and w^(8 r1 b), r = r0 + 8 r1, for the
-// length whose whole table does not fit beside its columns.
+// TWO: w^(r b) as a product of w^(r0 b) and w^(L r1 b), r = r0 + L r1 (L = R1B
+// and R2B), for the length whose whole table does not fit beside its columns.
 template <int R1A_, int R1B_, int R2A_, int R2B_, int NT_, int G_, int MINB_, bool TWO_ = false>
 struct ColReg {
   static constexpr int R1A = R1A_, R1B = R1B_, R2A = R2A_, R2B = R2B_;
@@ -45,18 +49,19 @@ struct ColReg {
   static constexpr bool TWO = TWO_;
   static constexpr int D1 = (R2 + NT - 1) / NT;  // radix-R1 transforms per thread
   static_assert(NT >= R1, "one radix-R2 transform per thread at most");
-  static_assert(!TWO || (D1 == 1 && R1 % 8 == 0 && R2 % 8 == 0), "two-level roots");
   static constexpr int THREADS = (G * NT + 31) / 32 * 32;
   // odd row strides and a column stride of 16 / G (mod 16) float2 keep both
   // transposes conflict free for G columns x consecutive b per half-warp
   static constexpr int S1 = R1 | 1, S2 = R2 | 1;
   static constexpr int CB = R2 * S1 > R1 * S2 ? R2 * S1 : R1 * S2;
   static constexpr int STRIDE = CB + ((16 / G) - CB % 16 + 16) % 16;
-  // root table: [r][b], row stride TS; two-level: [r0 | 8 r1][b < R1], then [q0 | 8 q1][b < R2]
+  // root table: [r][b], row stride TS; two-level: [r0 | R2B r1][b < R1], then [q0 | R1B q1][b < R2]
   static constexpr int TS = R1 | 1;
-  static constexpr int TAB = TWO ? (8 + R2 / 8) * R1 + (8 + R1 / 8) * R2 : R2 * TS;
+  static constexpr int TAB = TWO ? (R2A + R2B) * R1 + (R1A + R1B) * R2 : R2 * TS;
   static constexpr size_t SMEM = sizeof(float2) * ((size_t)G * STRIDE + TAB);
-  static constexpr int WORDS = 2 * R2;   // tensor-memory columns per thread
+  static constexpr int CH = R2 % 16 == 0 ? 16 : (R2 % 4 == 0 && R2 % 8 ? 4 : 8);  // complex values per tensor-memory access
+  static constexpr int SLOTS = (R2 + CH - 1) / CH * CH;
+  static constexpr int WORDS = 2 * SLOTS;  // tensor-memory columns per thread
   static constexpr int WPQ = (THREADS / 32 + 3) / 4;         // warps that share a lane quarter
   static constexpr int COLS_USED = WORDS * WPQ;
   static constexpr int COLS = COLS_USED <= 32    ? 32
@@ -65,34 +70,32 @@ struct ColReg {
                               : COLS_USED <= 256 ? 256
                                                  : 512;
   static_assert(COLS_USED <= 512 && COLS * MINB <= 512, "tensor memory holds every resident CTA's image columns");
-  static constexpr int CH = R2 % 16 == 0 ? 16 : (R2 % 8 == 0 ? 8 : 4);  // complex values per tensor-memory access
-  static_assert(R2 % CH == 0, "whole steps");
 };
 
 // v[r] *= w^(r b) (DIR = -1) or its conjugate, from a whole table's entries
-// tab[r step] or from the two levels lo[r0 step], hi[r1 step].
-template <int R, int DIR, bool TWO>
+// tab[r step] (L = 0) or from the two levels lo[r0 step], hi[r1 step].
+template <int R, int DIR, int L>
 __device__ __forceinline__ void apply_roots(float2* v, const float2* tab, int step) {
-  if constexpr (!TWO) {
+  if constexpr (L == 0) {
 #pragma unroll
     for (int r = 1; r < R; ++r) {
       const float2 w = tab[r * step];
       v[r] = DIR < 0 ? cmul(v[r], w) : cmulc(v[r], w);
     }
   } else {
-    float2 lo[8];
+    float2 lo[L];
 #pragma unroll
-    for (int r = 1; r < 8; ++r) {
+    for (int r = 1; r < L; ++r) {
       lo[r] = tab[r * step];
       v[r] = DIR < 0 ? cmul(v[r], lo[r]) : cmulc(v[r], lo[r]);
     }
 #pragma unroll
-    for (int r1 = 1; r1 < R / 8; ++r1) {
-      const float2 hi = tab[(8 + r1) * step];
+    for (int r1 = 1; r1 < R / L; ++r1) {
+      const float2 hi = tab[(L + r1) * step];
 #pragma unroll
-      for (int r0 = 0; r0 < 8; ++r0) {
+      for (int r0 = 0; r0 < L; ++r0) {
         const float2 w = r0 ? cmul(hi, lo[r0]) : hi;
-        v[8 * r1 + r0] = DIR < 0 ? cmul(v[8 * r1 + r0], w) : cmulc(v[8 * r1 + r0], w);
+        v[L * r1 + r0] = DIR < 0 ? cmul(v[L * r1 + r0], w) : cmulc(v[L * r1 + r0], w);
       }
     }
   }
@@ -103,7 +106,7 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
     colpass_reg_kernel(const float2* __restrict__ A, const float2* __restrict__ Ip, int ips, int h, int Wcp, int n_c,
                        int c_per_block, int c_per_image, int y_rows, float2* __restrict__ Y) {
   constexpr int R1 = C::R1, R2 = C::R2, N = C::N, G = C::G, NT = C::NT, D1 = C::D1, S1 = C::S1, S2 = C::S2;
-  constexpr int CH = C::CH;
+  constexpr int CH = C::CH, SLOTS = C::SLOTS;
   // no thread idles in a pass: its guards are constant, which spares the loads' zero fills
   constexpr bool FULL1 = D1 * NT == R2 && G * NT == C::THREADS, FULL2 = NT == R1 && G * NT == C::THREADS;
   extern __shared__ float2 crsm[];
@@ -134,16 +137,16 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
     }
   };
   if constexpr (C::TWO) {
-    auto fill = [&](float2* dst, int r_hi, int nb) {  // rows 0..7: r, rows 8..: 8 (row - 8)
-      for (int e = threadIdx.x; e < (8 + r_hi) * nb; e += C::THREADS) {
-        const int row = e / nb, b = e - (e / nb) * nb, r = row < 8 ? row : 8 * (row - 8);
+    auto fill = [&](float2* dst, int low, int high, int nb) {  // rows 0..low-1: r, then low (row - low)
+      for (int e = threadIdx.x; e < (low + high) * nb; e += C::THREADS) {
+        const int row = e / nb, b = e - (e / nb) * nb, r = row < low ? row : low * (row - low);
         float sn, cs;
         sincospif(2.0f * (float)(r * b) / (float)N, &sn, &cs);
         dst[e] = make_float2(cs, -sn);
       }
     };
-    fill(tab, R2 / 8, R1);
-    fill(tab + (8 + R2 / 8) * R1, R1 / 8, R2);
+    fill(tab, C::R2B, C::R2A, R1);
+    fill(tab + (C::R2A + C::R2B) * R1, C::R1B, C::R1A, R2);
   } else {
     for (int e = threadIdx.x; e < R2 * R1; e += C::THREADS) {
       const int r = e / R1, b = e - (e / R1) * R1;
@@ -157,13 +160,13 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
   LGB_CHAIN_INPUT(Ip);
   if (SPARSE && c_begin < c_end) fetch(c_begin);
   int image = c_begin / c_per_image;
-  float2 first[R2];
+  float2 first[SLOTS];
   {
     const float2* ip = Ip + (size_t)image * N * ips + kx;
 #pragma unroll
-    for (int s = 0; s < R2; ++s) {
+    for (int s = 0; s < SLOTS; ++s) {
       const int row = t + R1 * DftNT<C::R2A, C::R2B, -1>::out(s);
-      first[s] = (kx < ips && act2 && c_begin < c_end) ? __ldg(ip + (size_t)row * ips) : make_float2(0.f, 0.f);
+      first[s] = (s < R2 && kx < ips && act2 && c_begin < c_end) ? __ldg(ip + (size_t)row * ips) : make_float2(0.f, 0.f);
     }
   }
   tmem_barrier();
@@ -187,7 +190,7 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
 #pragma unroll
         for (int i = 0; i < CH; ++i) {
           const int row = t + R1 * DftNT<C::R2A, C::R2B, -1>::out(s0 + i);
-          w[i] = (kx < ips && act2) ? __ldg(ip + (size_t)row * ips) : make_float2(0.f, 0.f);
+          w[i] = (s0 + i < R2 && kx < ips && act2) ? __ldg(ip + (size_t)row * ips) : make_float2(0.f, 0.f);
         }
         tmem_put<CH>(tm + 2 * s0, w);
       }
@@ -225,7 +228,7 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
       const int tt = act2 ? t : 0;
 #pragma unroll
       for (int r = 0; r < R2; ++r) v[r] = x[r * S1 + tt];
-      apply_roots<R2, -1, C::TWO>(v, tab + tt, C::TWO ? R1 : C::TS);
+      apply_roots<R2, -1, C::TWO ? C::R2B : 0>(v, tab + tt, C::TWO ? R1 : C::TS);
       DftNT<C::R2A, C::R2B, -1>::run(v);
       // ---- cross power, P[0,0] = 0
 #pragma unroll
@@ -233,7 +236,8 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
         float2 w[CH];
         tmem_get<CH>(tm + 2 * s0, w);
 #pragma unroll
-        for (int i = 0; i < CH; ++i) v[s0 + i] = cmulc(w[i], v[s0 + i]);
+        for (int i = 0; i < CH; ++i)
+          if (s0 + i < R2) v[s0 + i] = cmulc(w[i], v[s0 + i]);
       }
       if (t == 0 && kx == 0) v[0] = make_float2(0.f, 0.f);
       // ---- inverse radix R2 on the same elements: output r in slot r
@@ -255,9 +259,9 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
 #pragma unroll
       for (int q = 0; q < R1; ++q) u[q] = x[q * S2 + bb];
       if constexpr (C::TWO)
-        apply_roots<R1, +1, true>(u, tab + (8 + R2 / 8) * R1 + bb, R2);
+        apply_roots<R1, +1, C::R1B>(u, tab + (C::R2A + C::R2B) * R1 + bb, R2);
       else
-        apply_roots<R1, +1, false>(u, tab + bb * C::TS, 1);
+        apply_roots<R1, +1, 0>(u, tab + bb * C::TS, 1);
       FO::run(u);
       if (col_ok && act1) {
         char* yc = reinterpret_cast<char*>(Y + (size_t)c * y_rows * Wcp);  // 32-bit offsets from here: H Wcp 8 B < 2^32
@@ -319,15 +323,21 @@ int colpass_reg_launch(const void* A, const void* Ip, int ips, int h, int Wcp, i
                         y_rows, static_cast<float2*>(Y));
 }
 
-// The sparse form reads inputs q < R1B only: rows h <= R1B R2.  Templates have
-// at most kMaxTemplate rows, so the long columns need no other.
+// The sparse form reads inputs q < R1B only: rows h <= R1B R2.  The first split
+// in Cs (the fastest first) that covers h, else the dense form of the last one;
+// templates have at most kMaxTemplate rows.
 constexpr int kMaxTemplate = 512;
-template <class C>
-int colpass_reg_t(const void* A, const void* Ip, int ips, int h, int Wcp, int n_c, int cpi, int y_rows, int waves, void* Y,
-                  cudaStream_t s) {
+template <class C, class... Cs>
+int colpass_reg_t(const void* A, const void* Ip, int ips, int h, int Wcp, int n_c, int cpi, int y_rows, int waves,
+                  void* Y, cudaStream_t s) {
   if (h > kMaxTemplate) return LGB_ERR_UNSUPPORTED_SIZE;
   if constexpr (C::R1B * C::R2 < kMaxTemplate) {
-    if (h > C::R1B * C::R2) return colpass_reg_launch<C, false>(A, Ip, ips, h, Wcp, n_c, cpi, y_rows, waves, Y, s);
+    if (h > C::R1B * C::R2) {
+      if constexpr (sizeof...(Cs) > 0)
+        return colpass_reg_t<Cs...>(A, Ip, ips, h, Wcp, n_c, cpi, y_rows, waves, Y, s);
+      else
+        return colpass_reg_launch<C, false>(A, Ip, ips, h, Wcp, n_c, cpi, y_rows, waves, Y, s);
+    }
   }
   return colpass_reg_launch<C, true>(A, Ip, ips, h, Wcp, n_c, cpi, y_rows, waves, Y, s);
 }

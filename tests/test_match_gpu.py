@@ -256,6 +256,12 @@ def _padded(H, W):
     return padded_grid(H, W)
 
 
+@pytest.mark.parametrize("H,W,d", [(576, 288, 288), (576, 512, 384), (1024, 512, 512), (2880, 512, 512), (5760, 512, 512)])
+def test_register_column_splits_against_oracle(H, W, d):
+    """Templates that only the second split, or the dense first pass, of a column length covers."""
+    test_register_column_pass_against_oracle(H, W, d, 1)
+
+
 @pytest.mark.parametrize("W", [512, 1024, 2048, 2880, 3072, 3840, 4096, 5760])
 @pytest.mark.parametrize("H,n_o,batch,n_df", [(48, 15, 5, 1), (64, 16, 1, 1), (61, 8, 4, 3)])
 def test_long_row_pass_against_oracle(W, H, n_o, batch, n_df):
