@@ -367,32 +367,33 @@ __global__ void __launch_bounds__(ROWS* R1)
 // (utils.py:106-188) is affine, rfft((p - e) s) = s (A - e U) with
 // U[k] = sum_{px < d} exp(-2 pi i k px / W), and is applied by the column pass.
 //
-// What bounds it: the shared-memory data path, which ran at 85 % with 57 % of
-// it bank conflicts when rows were staged, the real transforms' pre- and
-// post-processing read mirrored elements from shared memory, and all roots
-// came from tables.  Now the three transposes are all that crosses it: both
-// mirrored reads are shuffles between the threads t and -t of a row, the first
-// pass reads T directly, the roots of a thread's position stay in registers
-// over the row groups of a CTA and the others are literals.
-// CTAs of 8 rows, six per SM, wait less at the barriers between passes of
-// unequal width than 16-row ones.  9,216 correlograms: 1,959 -> 1,531 us (16 rows
-// 1,662), 288: 76 -> 66.
+// What bounds it: the shared-memory data path and the issue slots, 70 % each.
+// The passes: radix 16 of the c2r (8 DFTs a row) -> shared transpose -> radix 8,
+// whose thread t then holds the pixel pairs m' = t + 16 q that the rfft's radix-9
+// DFT t takes (q = 8 is the zero padding), so that both run in registers -> shared
+// transpose -> radix 16 (9 DFTs a row).  Both mirrored reads of the real
+// transforms are shuffles between the threads t and -t of a row; roots that
+// depend on the thread come from small tables (in registers they cost the
+// seventh resident CTA or spill), the others are literals.
+// The radix-16 passes have too few DFTs for four warps: warps 0 to 2 finish a row
+// group (three rows each), warps 2 and 3 start the next one, two barriers a group.
+// 38,304 correlograms: 6.35 ms in four passes with a transpose and a barrier
+// between all of them, 5.73 now (five warps, one role each: 7.7).
 template <int ROWS>
-__global__ void __launch_bounds__(ROWS * 16, 48 / ROWS)
+__global__ void __launch_bounds__(ROWS * 16, 7)
     proj_row_rfft_kernel(const float2* __restrict__ T, double* __restrict__ rowstats, int Wcp, int groups,
                          float2* __restrict__ A) {
   constexpr int HT = 256, M = 128, WC = M + 1, NT = 16, S1 = 17;
   constexpr int WH = 144;  // W / 2
   constexpr int C2 = 8;    // c2r: M = 16 x 8
-  constexpr int R2 = 9;    // rfft: WH = 16 x 9
-  // The two radix-16 passes have fewer DFTs per row (8 and 9) than a row has
-  // threads (16): their (row, DFT) tasks are packed densely onto the CTA's
-  // threads.  Row strides of 8 and 9 (mod 16) float2 keep the packed rows'
-  // accesses conflict free, the others are at any stride.
+  constexpr int R2 = 9;    // rfft: WH = 9 x 16
+  static_assert(ROWS == 8, "three warps of three rows (the last of two), then two of four");
+  // row strides of 8 and 9 (mod 16) float2: the radix-16 passes pack 8 and 9
+  // DFTs a row densely onto the lanes without conflicts
   constexpr int SC = C2 * S1, SR = R2 * S1;  // 136 and 153
-  static_assert(SC % 16 == 8 && SR % 16 == 9 && SR >= WH, "conflict-free row strides");
-  __shared__ float2 zb[ROWS * SR];  // c2r transpose (8 x 17 a row), then rfft transpose (9 x 17)
-  __shared__ float2 zr[ROWS * SR];  // rfft input
+  static_assert(SC % 16 == 8 && SR % 16 == 9, "conflict-free row strides");
+  __shared__ float2 zc[ROWS * SC];  // c2r transpose (8 x 17 a row)
+  __shared__ float2 zr[ROWS * SR];  // rfft transpose (9 x 17)
   __shared__ float2 pre[M];         // exp(+i pi k / M)
   __shared__ float2 post[WH + 1];   // exp(-i pi k / WH)
   for (int k = threadIdx.x; k < M; k += blockDim.x) {
@@ -407,63 +408,65 @@ __global__ void __launch_bounds__(ROWS * 16, 48 / ROWS)
   }
   __syncthreads();
   const int c = blockIdx.y;
-  const int g = threadIdx.x / NT, t = threadIdx.x % NT, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x / 32, lane = threadIdx.x & 31;
+  const int g = threadIdx.x / NT, t = threadIdx.x % NT;
   // roots of this thread's position: exp(+2 pi i r t / M) = +-pre[2 r t mod M] and
   // exp(-2 pi i r t / WH) = +-post[2 r t mod WH]
-  float2 rootc[C2], rootr[R2];
-#pragma unroll
-  for (int r = 1; r < C2; ++r) {
-    const int m = 2 * r * t;
+  __shared__ float2 rootc[C2 * NT];
+  {
+    const int m = 2 * (threadIdx.x / NT) * t;
     const float2 v = pre[m & (M - 1)];
-    rootc[r] = m < M ? v : make_float2(-v.x, -v.y);
+    rootc[threadIdx.x] = m < M ? v : make_float2(-v.x, -v.y);
   }
-#pragma unroll
-  for (int r = 1; r < R2; ++r) {
-    const int m = 2 * r * t;
+  __shared__ float2 rootr[R2 * NT];
+  for (int i = threadIdx.x; i < R2 * NT; i += ROWS * NT) {
+    const int m = 2 * (i / NT) * (i % NT);
     const float2 v = post[m <= WH ? m : m - WH];
-    rootr[r] = m <= WH ? v : make_float2(-v.x, -v.y);
+    rootr[i] = m <= WH ? v : make_float2(-v.x, -v.y);
   }
-  const float2 prej = pre[threadIdx.x % C2], postj = post[t];
+  const float2 prej = pre[lane % C2], postj = post[lane % R2];
   chain_wait();
   LGB_CHAIN_INPUT(T);
+  // ---- c2r pass 1 (radix 16) over k = tt + 8q of a group's rows: warps 2 and 3, four rows each
+  auto start = [&](int grp) {
+    const int tt = lane % C2;
+    const int mirror = (lane & ~(C2 - 1)) | ((C2 - tt) & (C2 - 1));  // M - k = (8 - tt) + 8 (15 - q)
+    const int gg = lane / C2 + 4 * (warp - 2);
+    const float2* src = T + ((size_t)c * HT + (blockIdx.x * groups + grp) * ROWS + gg) * WC;
+    float2 x[16], u[16];
+#pragma unroll
+    for (int q = 0; q < 16; ++q) x[q] = __ldg(src + tt + C2 * q);
+    const float2 nyquist = tt == 0 ? __ldg(src + M) : make_float2(0.f, 0.f);
+    static_for<16>([&](auto q_) {
+      constexpr int q = decltype(q_)::value;
+      float2 a = x[q], b;
+      b.x = __shfl_sync(0xffffffffu, x[15 - q].x, mirror);
+      b.y = __shfl_sync(0xffffffffu, x[15 - q].y, mirror);
+      const float2 own = q ? x[(16 - q) % 16] : nyquist;
+      if (tt == 0) b = own;
+      if (q == 0 && tt == 0) a.y = b.y = 0.f;  // DC and Nyquist: real parts only
+      b.y = -b.y;
+      const float2 xo = mul_root<q, 32, +1>(cmul(csub(a, b), prej));
+      u[q] = cadd(cadd(a, b), mul_i<1>(xo));
+    });
+    Dft<16, +1>::run(u);
+#pragma unroll
+    for (int q = 0; q < 16; ++q) zc[gg * SC + tt * S1 + q] = u[q];
+  };
+  if (warp >= 2) start(0);
 #pragma unroll 1
   for (int grp = 0; grp < groups; ++grp) {
     const int row0 = (blockIdx.x * groups + grp) * ROWS;
-    // ---- c2r pass 1 (radix 16) over k = tt + 8q
-    if (threadIdx.x < ROWS * C2) {
-      const int gg = threadIdx.x / C2, tt = threadIdx.x % C2;
-      const float2* src = T + ((size_t)c * HT + row0 + gg) * WC;
-      float2 x[16], u[16];
-#pragma unroll
-      for (int q = 0; q < 16; ++q) x[q] = __ldg(src + tt + C2 * q);
-      const float2 nyquist = tt == 0 ? __ldg(src + M) : make_float2(0.f, 0.f);
-      const int mirror = (lane & ~(C2 - 1)) | ((C2 - tt) & (C2 - 1));  // M - k = (8 - tt) + 8 (15 - q)
-      static_for<16>([&](auto q_) {
-        constexpr int q = decltype(q_)::value;
-        float2 a = x[q], b;
-        b.x = __shfl_sync(0xffffffffu, x[15 - q].x, mirror);
-        b.y = __shfl_sync(0xffffffffu, x[15 - q].y, mirror);
-        const float2 own = q ? x[(16 - q) % 16] : nyquist;
-        if (tt == 0) b = own;
-        if (q == 0 && tt == 0) a.y = b.y = 0.f;  // DC and Nyquist: real parts only
-        b.y = -b.y;
-        const float2 xo = mul_root<q, 32, +1>(cmul(csub(a, b), prej));
-        u[q] = cadd(cadd(a, b), mul_i<1>(xo));
-      });
-      Dft<16, +1>::run(u);
-#pragma unroll
-      for (int q = 0; q < 16; ++q) zb[gg * SC + tt * S1 + q] = u[q];
-    }
-    __syncthreads();
-    // ---- c2r pass 2 (radix 8): pixel pairs m = t + 16r, moments, shifted rfft input
+    __syncthreads();  // this group's c2r rows are there, the last one's rfft rows are read
+    // ---- c2r pass 2 (radix 8): pixel pairs m = t + 16 r, moments, and the rfft's
+    // pass 1 (radix 9) over m' = t + 16 q, q = (r + 4) mod 8 (the ifftshift)
     {
-      const int y = row0 + g;
-      const int py = (y + HT - HT / 2) % HT;
-      float2 w[C2];
+      const int py = (row0 + g + HT - HT / 2) % HT;
+      float2 w[C2], u[R2];
 #pragma unroll
       for (int r = 0; r < C2; ++r) {
-        w[r] = zb[g * SC + r * S1 + t];
-        if (r) w[r] = cmul(w[r], rootc[r]);
+        w[r] = zc[g * SC + r * S1 + t];
+        if (r) w[r] = cmul(w[r], rootc[r * NT + t]);
       }
       Dft<C2, +1>::run(w);
       const float scale = 1.0f / ((float)HT * (float)HT);
@@ -471,10 +474,9 @@ __global__ void __launch_bounds__(ROWS * 16, 48 / ROWS)
       float s1 = 0.f, s2 = 0.f, se = 0.f;
 #pragma unroll
       for (int r = 0; r < C2; ++r) {
-        const int m = t + r * 16;
         const float a = w[r].x * scale, b = w[r].y * scale;
-        const int mp = (m + M / 2) & (M - 1);  // ifftshift: px = 2 mp, 2 mp + 1
-        zr[g * SR + mp] = make_float2(a, b);
+        const int q = (r + C2 / 2) % C2, mp = t + q * 16;  // px = 2 mp, 2 mp + 1
+        u[q] = make_float2(a, b);
         s1 += a + b;
         s2 = fmaf(a, a, fmaf(b, b, s2));
         if (edge_row) {
@@ -484,6 +486,7 @@ __global__ void __launch_bounds__(ROWS * 16, 48 / ROWS)
           if (mp == M - 1) se += b;
         }
       }
+      u[R2 - 1] = make_float2(0.f, 0.f);
 #pragma unroll
       for (int o = 8; o > 0; o >>= 1) {
         s1 += __shfl_xor_sync(0xffffffffu, s1, o);
@@ -496,48 +499,40 @@ __global__ void __launch_bounds__(ROWS * 16, 48 / ROWS)
         rs[1] = (double)s2;
         rs[2] = (double)se;
       }
+      Dft<R2, -1>::run(u);
+#pragma unroll
+      for (int r = 0; r < R2; ++r) zr[g * SR + r * S1 + t] = r ? cmul(u[r], rootr[r * NT + t]) : u[r];
     }
     __syncthreads();
-    // ---- rfft pass 1 (radix 16) over m' = tt + 9q; m' >= 128 is the zero padding
-    if (threadIdx.x < ROWS * R2) {
-      const int gg = threadIdx.x / R2, tt = threadIdx.x - (threadIdx.x / R2) * R2;
+    if (warp < 3) {
+      // ---- rfft pass 2 (radix 16): Z[b + 9 s], then the real post-process with
+      // Z[WH - k] = Z[(9 - b) + 9 (15 - s)]
+      const int b = lane % R2, own_row = 3 * warp + lane / R2;
+      const bool act = lane < 3 * R2 && own_row < ROWS;
+      const int row = act ? own_row : 0;
       float2 v[16];
 #pragma unroll
-      for (int q = 0; q < 16; ++q)
-        v[q] = R2 * q + R2 - 1 < M || tt + R2 * q < M ? zr[gg * SR + tt + R2 * q] : make_float2(0.f, 0.f);
+      for (int q = 0; q < 16; ++q) v[q] = zr[row * SR + b * S1 + q];
       Dft<16, -1>::run(v);
-#pragma unroll
-      for (int q = 0; q < 16; ++q) zb[gg * SR + tt * S1 + q] = v[q];
-    }
-    __syncthreads();
-    // ---- rfft pass 2 (radix 9): Z[t + 16r], then the real post-process with
-    // Z[WH - k] = Z[(16 - t) + 16 (8 - r)]
-    {
-      const int py = (row0 + g + HT - HT / 2) % HT;
-      float2 u[R2];
-#pragma unroll
-      for (int r = 0; r < R2; ++r) {
-        u[r] = zb[g * SR + r * S1 + t];
-        if (r) u[r] = cmul(u[r], rootr[r]);
-      }
-      Dft<R2, -1>::run(u);
-      float2* out = A + ((size_t)c * HT + py) * Wcp;
-      const int mirror = (lane & 16) | ((16 - t) & 15);
-      static_for<R2>([&](auto r_) {
-        constexpr int r = decltype(r_)::value;
+      const int py = (row0 + row + HT - HT / 2) % HT;
+      float2* out = A + ((size_t)c * HT + py) * Wcp + b;
+      const int mirror = b ? lane - b + R2 - b : lane;
+      static_for<16>([&](auto s_) {
+        constexpr int s = decltype(s_)::value;
         float2 zm;
-        zm.x = __shfl_sync(0xffffffffu, u[8 - r].x, mirror);
-        zm.y = __shfl_sync(0xffffffffu, u[8 - r].y, mirror);
-        if (t == 0) zm = u[(9 - r) % 9];
+        zm.x = __shfl_sync(0xffffffffu, v[15 - s].x, mirror);
+        zm.y = __shfl_sync(0xffffffffu, v[15 - s].y, mirror);
+        if (b == 0) zm = v[(16 - s) % 16];
         zm.y = -zm.y;
-        const float2 xe = cscale(cadd(u[r], zm), 0.5f);
-        const float2 xo = mul_i<-1>(cscale(csub(u[r], zm), 0.5f));
-        out[t + 16 * r] = cadd(xe, mul_root<r, 18, -1>(cmul(xo, postj)));
+        const float2 xe = cscale(cadd(v[s], zm), 0.5f);
+        const float2 xo = mul_i<-1>(cscale(csub(v[s], zm), 0.5f));
+        const float2 X = cadd(xe, mul_root<s, 32, -1>(cmul(xo, postj)));
+        if (act) out[R2 * s] = X;
       });
-      if (t == 0) out[WH] = make_float2(u[0].x - u[0].y, 0.f);
-      for (int k = WH + 1 + t; k < Wcp; k += NT) out[k] = make_float2(0.f, 0.f);
+      if (act && b == 0) out[WH] = make_float2(v[0].x - v[0].y, 0.f);
+      if (act && WH + 1 + b < Wcp) out[WH + 1] = make_float2(0.f, 0.f);
     }
-    __syncthreads();  // zb is read
+    if (warp >= 2 && grp + 1 < groups) start(grp + 1);
   }
 }
 

@@ -136,14 +136,13 @@ bool supported_proj_row_rfft(int h, int W) { return h == 256 && W == 288; }
 int launch_proj_row_rfft(int h, int W, const void* T, int n_c, double* rowstats, int Wcp, void* A, cudaStream_t s) {
   if (!supported_proj_row_rfft(h, W) || Wcp < W / 2 + 1) return LGB_ERR_UNSUPPORTED_SIZE;
   // 8-row groups that share a CTA's roots: up to 8 of 32, as long as two rounds
-  // of six CTAs per SM are left (groups of 8 / 4: 9,216 correlograms 1,531 / 1,616
-  // us, 288 correlograms 74 / 66 us)
+  // of seven CTAs per SM are left
   constexpr int ROWS = 8;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   int groups = 8;
-  while (groups > 1 && (long long)n_c * (256 / (ROWS * groups)) < 12LL * sms) groups /= 2;
+  while (groups > 1 && (long long)n_c * (256 / (ROWS * groups)) < 14LL * sms) groups /= 2;
   return launch_chained(proj_row_rfft_kernel<ROWS>, dim3(256 / (ROWS * groups), n_c), dim3(ROWS * 16), 0, s,
                         static_cast<const float2*>(T), rowstats, Wcp, groups, static_cast<float2*>(A));
 }
