@@ -385,18 +385,31 @@ struct EpiLinDx {
   }
 };
 
+template <class Epi, int BN, int ST>
+static int launch_gemm(dim3 grid, const TcGemmArgs& g, const typename Epi::Params& ep, cudaStream_t s) {
+  constexpr int SMEM = TcSmem<BN, false, ST>::BYTES;  // single BF16 term: no lo buffers
+  if (cudaFuncSetAttribute(tc_gemm_kernel<Epi, BN, false, false, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           SMEM) != cudaSuccess)
+    return LGB_ERR_CUDA;
+  tc_gemm_kernel<Epi, BN, false, false, ST><<<grid, kTcThreads, SMEM, s>>>(g, ep);
+  return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
+}
+
+// Stages of K chunks: two where several CTAs share an SM, six (all that fit)
+// where a grid has at most a CTA per SM and each chunk's latency shows: 18 chunks
+// of 128 x 128 in 32 CTAs 22.8 -> 17.9 us.
 template <class Epi, int BN>
 static int run_gemm(int m_tiles, int n_tiles, int k_chunks, int splits, const uint16_t* a, const uint16_t* b,
                     int* status, const typename Epi::Params& ep, cudaStream_t s) {
-  constexpr int SMEM = TcSmem<BN, false>::BYTES;  // single BF16 term: no lo buffers
-  if (cudaFuncSetAttribute(tc_gemm_kernel<Epi, BN, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           SMEM) != cudaSuccess)
-    return LGB_ERR_CUDA;
   const int per = (k_chunks + splits - 1) / splits;
   const int z = (k_chunks + per - 1) / per;
   TcGemmArgs g{a, nullptr, b, nullptr, k_chunks, 1, status, splits > 1 ? per : 0};
-  tc_gemm_kernel<Epi, BN, false, false><<<dim3(n_tiles, m_tiles, z), kTcThreads, SMEM, s>>>(g, ep);
-  return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
+  const dim3 grid(n_tiles, m_tiles, z);
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if ((long long)n_tiles * m_tiles * z <= sms) return launch_gemm<Epi, BN, 6>(grid, g, ep, s);
+  return launch_gemm<Epi, BN, 2>(grid, g, ep, s);
 }
 
 template <class Epi>

@@ -199,30 +199,33 @@ struct TcGemmArgs {
                  // epilogue then adds its partial sums atomically); 0: all chunks
 };
 
-// Shared memory of one CTA: two pipeline stages of [A hi | A lo | B hi | B lo]
+// Shared memory of one CTA: ST pipeline stages of [A hi | A lo | B hi | B lo]
 // K chunks, or [A hi | B hi] when the kernel is built without lo terms (LO =
 // false: half the footprint, so more CTAs fit an SM for single-term GEMMs).
-template <int BN, bool LO = true>
+// Two stages where several CTAs share an SM and hide one another's latency; a
+// grid of a CTA per SM or less wants its chunks in flight itself.
+template <int BN, bool LO = true, int ST = 2>
 struct TcSmem {
   static constexpr int A_BYTES = kTcM * kTcKC * 2;  // 16 KB
   static constexpr int B_BYTES = BN * kTcKC * 2;
   static constexpr int B_OFF = (LO ? 2 : 1) * A_BYTES;  // B hi within a stage
   static constexpr int STAGE = (LO ? 2 : 1) * (A_BYTES + B_BYTES);
-  static constexpr int STAGES = 2;
+  static constexpr int STAGES = ST;
+  static_assert(ST >= 2 && (2 * ST + 1) * 8 + 4 <= 128, "barriers of the stages");
   static constexpr int BYTES = STAGES * STAGE + 1024 /* alignment */ + 128 /* barriers */;
 };
 
-template <class Epi, int BN, bool F16, bool LO = true>
+template <class Epi, int BN, bool F16, bool LO = true, int ST = 2>
 __global__ void __launch_bounds__(kTcThreads, 1)
     tc_gemm_kernel(TcGemmArgs g, typename Epi::Params ep) {
   static_assert(BN % 32 == 0 && BN >= 32 && BN <= 256, "N tile");
-  using S = TcSmem<BN, LO>;
+  using S = TcSmem<BN, LO, ST>;
   extern __shared__ uint8_t tc_raw[];
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(tc_raw) + 1023) & ~(uintptr_t)1023);
   uint64_t* full = reinterpret_cast<uint64_t*>(base + S::STAGES * S::STAGE);
-  uint64_t* empty = full + 2;
-  uint64_t* done = full + 4;
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(full + 6);
+  uint64_t* empty = full + ST;
+  uint64_t* done = full + 2 * ST;
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(full + 2 * ST + 1);
   __shared__ int s_fail;
 
   const int warp = threadIdx.x >> 5;
@@ -233,7 +236,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   const bool lo_terms = LO && g.terms == 3;  // built without lo buffers: hi*hi only
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < ST; ++i) {
       mbar_init(&full[i], 1);
       mbar_init(&empty[i], 1);
     }
@@ -251,28 +254,24 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     const size_t a_blk = tc_block_elems(kTcM), b_blk = tc_block_elems(BN);
     const uint32_t stage_bytes = lo_terms ? (uint32_t)S::STAGE : (uint32_t)(S::A_BYTES + S::B_BYTES);
     auto load = [&](int kc) {
-      uint8_t* st = base + (kc & 1) * S::STAGE;
+      uint8_t* st = base + kc % ST * S::STAGE;
+      uint64_t* bar = &full[kc % ST];
       const size_t ao = ((size_t)m_tile * KC + kc0 + kc) * a_blk, bo = ((size_t)n_tile * KC + kc0 + kc) * b_blk;
-      mbar_expect_tx(&full[kc & 1], stage_bytes);
-      bulk_g2s(st, g.a_hi + ao, S::A_BYTES, &full[kc & 1]);
-      bulk_g2s(st + S::B_OFF, g.b_hi + bo, S::B_BYTES, &full[kc & 1]);
+      mbar_expect_tx(bar, stage_bytes);
+      bulk_g2s(st, g.a_hi + ao, S::A_BYTES, bar);
+      bulk_g2s(st + S::B_OFF, g.b_hi + bo, S::B_BYTES, bar);
       if (lo_terms) {
-        bulk_g2s(st + S::A_BYTES, g.a_lo + ao, S::A_BYTES, &full[kc & 1]);
-        bulk_g2s(st + S::B_OFF + S::B_BYTES, g.b_lo + bo, S::B_BYTES, &full[kc & 1]);
+        bulk_g2s(st + S::A_BYTES, g.a_lo + ao, S::A_BYTES, bar);
+        bulk_g2s(st + S::B_OFF + S::B_BYTES, g.b_lo + bo, S::B_BYTES, bar);
       }
     };
     const uint32_t idesc = mma_idesc(kTcM, BN, F16);
     bool ok = true;
     int issued = 0, landed = 0;  // chunks whose copies were issued / have been waited for
-    load(0);
-    ++issued;
-    if (NK > 1) {
-      load(1);
-      ++issued;
-    }
+    for (; issued < ST && issued < NK; ++issued) load(issued);
     for (int kc = 0; kc < NK && ok; ++kc) {
-      const int s = kc & 1;
-      if (!mbar_wait(&full[s], (kc >> 1) & 1)) {
+      const int s = kc % ST;
+      if (!mbar_wait(&full[s], (kc / ST) & 1)) {
         ok = false;
         break;
       }
@@ -292,14 +291,14 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         }
       }
       mma_commit(&empty[s]);
-      // chunk kc+1 goes into the stage of chunk kc-1 once that chunk's MMAs have
+      // chunk kc-1+ST goes into the stage of chunk kc-1 once that chunk's MMAs have
       // read it; chunk kc's MMAs keep the tensor pipe busy meanwhile
-      if (kc >= 1 && kc + 1 < NK) {
-        if (!mbar_wait(&empty[(kc - 1) & 1], ((kc - 1) >> 1) & 1)) {
+      if (kc >= 1 && issued < NK) {
+        if (!mbar_wait(&empty[(kc - 1) % ST], ((kc - 1) / ST) & 1)) {
           ok = false;
           break;
         }
-        load(kc + 1);
+        load(issued);
         ++issued;
       }
     }
@@ -308,7 +307,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       atomicExch(g.err, LGB_ERR_DEVICE_TIMEOUT);
       // copies still in flight target this CTA's shared memory: wait (bounded)
       // for each before the CTA may exit
-      for (int j = landed; j < issued; ++j) mbar_wait(&full[j & 1], (j >> 1) & 1);
+      for (int j = landed; j < issued; ++j) mbar_wait(&full[j % ST], (j / ST) & 1);
     }
     mma_commit(done);  // tracks every MMA this thread issued
   }
