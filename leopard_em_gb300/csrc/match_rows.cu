@@ -36,7 +36,7 @@ int launch_repack_rows(const void* src, long long rows, int wc, int wcp, void* d
 // takes Re(I00 conj(P00)) scale, P00 = s (sum of the projection - e h^2).
 // The FP64 pipe bounds it (a warp-wide add holds it for 32 cycles), so the
 // warps are CTAs of their own, spread over the SMs: 300 correlograms
-// 10.4 us in CTAs of eight warps, 7.3 in one each, 5.0 without the divisions.
+// 10.4 us in CTAs of eight warps, 7.3 in one each, 5.6 without the divisions.
 __global__ void __launch_bounds__(32)
     norm_constants_kernel(double* __restrict__ rowstats, NormSizes sizes, const float2* __restrict__ dc, size_t dc_stride,
                           float scale, float* __restrict__ offset) {

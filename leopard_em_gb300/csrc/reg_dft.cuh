@@ -1,6 +1,6 @@
 // Composite DFTs held in one thread's registers (R = RA * RB up to 80) with
 // compile-time roots, for the two-pass transforms of match_cols_reg.cuh and
-// match_rows_reg.cuh.
+// match_rows_half.cuh.
 //
 // A long transform in two register passes exchanges its data once through
 // shared memory instead of two or three times; what bounds the passes is then
@@ -157,20 +157,13 @@ struct Dft<12, DIR> {
 // output r = ra + RA rb.  NT: input q = qa RB + qb in slot q, output r in slot
 // ra RB + rb.  TN: input q in slot qb RA + qa, output r in slot r; it takes
 // what an NT of RB * RA left behind.  SPARSE (NT): inputs q >= RB are zero and
-// are not read; the RA-point transforms are then copies.  `hook` runs after
-// each of the RB + RA inner transforms (hook(0) .. hook(RA + RB - 1)): work of
-// another unit that is to be spread over the arithmetic.
-struct NoHook {
-  template <int I>
-  __device__ __forceinline__ void operator()(std::integral_constant<int, I>) const {}
-};
+// are not read; the RA-point transforms are then copies.
 template <int RA, int RB, int DIR, bool SPARSE = false>
 struct DftNT {
   static constexpr int R = RA * RB;
   // output index held by slot s
   __host__ __device__ static constexpr int out(int s) { return s / RB + RA * (s % RB); }
-  template <class H = NoHook>
-  static __device__ __forceinline__ void run(float2* v, H hook = H()) {
+  static __device__ __forceinline__ void run(float2* v) {
     static_for<RB>([&](auto qb_) {
       constexpr int qb = decltype(qb_)::value;
       float2 t[RA];
@@ -186,12 +179,10 @@ struct DftNT {
         constexpr int ra = decltype(ra_)::value;
         v[ra * RB + qb] = mul_root<qb * ra, R, DIR>(t[ra]);
       });
-      hook(std::integral_constant<int, qb>{});
     });
     static_for<RA>([&](auto ra_) {
       constexpr int ra = decltype(ra_)::value;
       Dft<RB, DIR>::run(v + ra * RB);
-      hook(std::integral_constant<int, RB + ra>{});
     });
   }
 };
@@ -199,8 +190,7 @@ struct DftNT {
 template <int RA, int RB, int DIR>
 struct DftTN {
   static constexpr int R = RA * RB;
-  template <class H = NoHook>
-  static __device__ __forceinline__ void run(float2* v, H hook = H()) {
+  static __device__ __forceinline__ void run(float2* v) {
     static_for<RB>([&](auto qb_) {
       constexpr int qb = decltype(qb_)::value;
       Dft<RA, DIR>::run(v + qb * RA);
@@ -208,7 +198,6 @@ struct DftTN {
         constexpr int ra = decltype(ra_)::value;
         v[qb * RA + ra] = mul_root<qb * ra, R, DIR>(v[qb * RA + ra]);
       });
-      hook(std::integral_constant<int, qb>{});
     });
     static_for<RA>([&](auto ra_) {
       constexpr int ra = decltype(ra_)::value;
@@ -218,7 +207,6 @@ struct DftTN {
       Dft<RB, DIR>::run(t);
 #pragma unroll
       for (int b = 0; b < RB; ++b) v[b * RA + ra] = t[b];
-      hook(std::integral_constant<int, RB + ra>{});
     });
   }
 };
