@@ -18,6 +18,8 @@
 // counterpart (Leopard-EM has no learned component).
 #include <cuda_bf16.h>
 
+#include <type_traits>
+
 #include "tc_gemm.cuh"
 
 namespace lgb {
@@ -76,7 +78,8 @@ __device__ __forceinline__ void store8_bits(uint16_t* dst, const uint16_t* v) {
 // rate) unless positions are divided out once for many elements and the stride
 // is a template argument; a run-time stride and per-element divisions cost 256
 // samples of the network's step 1,648 us in gcol and 762 us in im2col, units of
-// eight elements with stepped positions 580 and 390, this 193 and 185.
+// eight elements with stepped positions 580 and 390, this 193 and 185 (gcol of
+// stride-2 layers again: gcol_pairs_kernel).
 //
 // A row's 72 consecutive K elements are the 9 taps of 8 channels: one thread
 // takes them (nine 16-byte units), its taps at compile time, its position and
@@ -243,6 +246,64 @@ __global__ void __launch_bounds__(256) gcol_kernel(ConvShape c, const float* __r
                   return (size_t)img * c.Cout * (c.Ho * c.Wo);
                 },
                 out);
+}
+
+// The same operand of a stride-2 layer of even width, two neighbouring input
+// pixels a thread: of their 18 taps 3 (even image row) or 6 (odd row) meet an
+// output pixel, and which ones is known at compile time, where the general form
+// tests and loads nine a pixel.  Their units are neighbours too: 32-byte stores.
+// 256 samples: 134 -> 77 us for the 64 x 64 layer, 43 -> 25 and 12 -> 8 for the next.
+__global__ void __launch_bounds__(256) gcol_pairs_kernel(ConvShape c, const float* __restrict__ g, int rows_pad,
+                                                         int k_pad, uint16_t* __restrict__ out) {
+  const int pairs = rows_pad / 2, KC = k_pad / kTcKC, units = k_pad / 8, plane_size = c.Ho * c.Wo;
+  const long long n = (long long)pairs * tap_groups(k_pad);
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
+    const int group = (int)(e / pairs), q = 2 * (int)(e - (long long)group * pairs);
+    const unsigned img = (unsigned)q / (unsigned)(c.H * c.W), pix = q - img * (c.H * c.W);
+    const int iy = (int)(pix / (unsigned)c.W), oy = iy / 2, ox = ((int)pix - iy * c.W) / 2;
+    const bool in = q < c.Q, right = ox + 1 < c.Wo, odd = iy & 1, down = odd && oy + 1 < c.Ho;
+    const float* src = g + ((size_t)img * c.Cout + group * 8) * plane_size + oy * c.Wo + ox;
+    // g at (oy, ox), (oy, ox + 1) and, for odd rows, one row down
+    uint16_t at[8][4];
+#pragma unroll
+    for (int ch = 0; ch < 8; ++ch) {
+      const bool ok = in && group * 8 + ch < c.Cout;
+      at[ch][0] = __bfloat16_as_ushort(__float2bfloat16_rn(ok ? src[0] : 0.f));
+      at[ch][1] = __bfloat16_as_ushort(__float2bfloat16_rn(ok && right ? src[1] : 0.f));
+      at[ch][2] = __bfloat16_as_ushort(__float2bfloat16_rn(ok && down ? src[c.Wo] : 0.f));
+      at[ch][3] = __bfloat16_as_ushort(__float2bfloat16_rn(ok && down && right ? src[c.Wo + 1] : 0.f));
+      src += plane_size;
+    }
+    const int tile = q / kTcM, rl = q - tile * kTcM;
+    auto emit = [&](auto odd_row) {
+#pragma unroll
+      for (int u = 0; u < 9; ++u) {
+        const int ku = group * 9 + u;
+        unsigned w[8];  // the even pixel's eight K elements, then the odd pixel's
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const int k = u * 8 + i % 8, ch = k / 9, t = k % 9;
+          int from;  // which of at[ch], -1: none
+          if constexpr (decltype(odd_row)::value)
+            from = i < 8 ? (t == 1 ? 2 : t == 7 ? 0 : -1) : (t == 0 ? 3 : t == 2 ? 2 : t == 6 ? 1 : t == 8 ? 0 : -1);
+          else
+            from = i < 8 ? (t == 4 ? 0 : -1) : (t == 3 ? 1 : t == 5 ? 0 : -1);
+          const unsigned v = from < 0 ? 0u : at[ch][from];
+          w[i / 2] = i % 2 ? w[i / 2] | v << 16 : v;
+        }
+        if (ku < units) {
+          const size_t unit = ((size_t)tile * KC + ku / 8) * (kTcM * 8) + (rl / 8) * 64 + (ku % 8) * 8 + rl % 8;
+          asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(out + unit * 8), "r"(w[0]),
+                       "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                       : "memory");
+        }
+      }
+    };
+    if (odd)
+      emit(std::true_type{});
+    else
+      emit(std::false_type{});
+  }
 }
 
 // B of the weight gradient: gT[co][p] = g[n][co][oy][ox]
@@ -537,8 +598,11 @@ int lgb_nn_conv3x3_backward(int N, int Cin, int H, int W, int Cout, int stride, 
     uint16_t* bm = reinterpret_cast<uint16_t*>(base + ws.dx_a);
     const int bn = bn_for(Cin);
     const int kp = round_up(c.Kt, kTcKC), qp = round_up(c.Q, kTcM), cp = round_up(Cin, bn);
-    (stride == 1 ? gcol_kernel<1> : gcol_kernel<2>)<<<grid256((long long)qp * tap_groups(kp)), 256, 0, s>>>(c, g, qp,
-                                                                                                            kp, a);
+    if (stride == 2 && W % 2 == 0)
+      gcol_pairs_kernel<<<grid256((long long)qp / 2 * tap_groups(kp)), 256, 0, s>>>(c, g, qp, kp, a);
+    else
+      (stride == 1 ? gcol_kernel<1> : gcol_kernel<2>)<<<grid256((long long)qp * tap_groups(kp)), 256, 0, s>>>(c, g, qp,
+                                                                                                              kp, a);
     weights_t_kernel<<<grid256((long long)cp * kp / 8), 256, 0, s>>>(c, static_cast<const bf16t*>(w), cp, kp, bn, bm);
     if (cudaGetLastError() != cudaSuccess) return LGB_ERR_CUDA;
     EpiConvDx::Params ep{dx, Cin, H * W, c.Q};

@@ -213,6 +213,12 @@ def test_linear_layer_odd_shapes_match_torch(N, In, Out):
     assert _rel(db, gq.sum(0)) < 1e-2
 
 
+@pytest.mark.parametrize("N,Cin,H,W,Cout", [(2, 5, 7, 16, 24), (1, 3, 5, 6, 17), (3, 33, 8, 2, 9), (1, 2, 1, 2, 1)])
+def test_conv_stride_two_pixel_pairs(N, Cin, H, W, Cout):
+    """Input gradient of even widths, two pixels a thread: odd heights, a last column and row without a neighbour."""
+    test_conv_gathers_whole_image_rows(N, Cin, H, W, Cout, 2)
+
+
 @pytest.mark.parametrize("N,Cin,H,W,Cout,stride", [(2, 9, 6, 16, 11, 1), (3, 17, 32, 16, 40, 2), (1, 8, 5, 24, 8, 1),
                                                    (2, 1, 16, 48, 3, 2)])
 def test_conv_gathers_whole_image_rows(N, Cin, H, W, Cout, stride):
