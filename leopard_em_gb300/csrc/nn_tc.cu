@@ -456,9 +456,12 @@ static int launch_gemm(dim3 grid, const TcGemmArgs& g, const typename Epi::Param
   return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;
 }
 
-// Stages of K chunks: two where several CTAs share an SM, six (all that fit)
-// where a grid has at most a CTA per SM and each chunk's latency shows: 18 chunks
-// of 128 x 128 in 32 CTAs 22.8 -> 17.9 us.
+// Stages of K chunks.  Six (all that fit) where a grid has at most a CTA per SM
+// and each chunk's latency shows: 18 chunks of 128 x 128 in 32 CTAs 22.8 -> 17.9
+// us.  Larger grids share an SM: three stages leave room for two to three CTAs
+// and suit four chunks or more (512 CTAs of 14 chunks 56 -> 41 us; four stages
+// 57); with fewer, two stages and one CTA more are better (2,048 CTAs of two
+// chunks 26 us, 31 with three stages).
 template <class Epi, int BN>
 static int run_gemm(int m_tiles, int n_tiles, int k_chunks, int splits, const uint16_t* a, const uint16_t* b,
                     int* status, const typename Epi::Params& ep, cudaStream_t s) {
@@ -470,6 +473,7 @@ static int run_gemm(int m_tiles, int n_tiles, int k_chunks, int splits, const ui
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if ((long long)n_tiles * m_tiles * z <= sms) return launch_gemm<Epi, BN, 6>(grid, g, ep, s);
+  if (per >= 4) return launch_gemm<Epi, BN, 3>(grid, g, ep, s);
   return launch_gemm<Epi, BN, 2>(grid, g, ep, s);
 }
 
