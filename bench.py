@@ -950,16 +950,16 @@ def main():
     per_launch_ms = stage_ms[top] / max(1, launches[top])
     ach = alg_bytes.get(top, 0.0) / (per_launch_ms / 1e3) / 1e9 if top in alg_bytes else None
     # DRAM bytes (read + write) of one launch, from ncu captures of this
-    # workload (dram__bytes_read.sum + dram__bytes_write.sum; one launch each,
-    # --set full) at orientation batch 8, 16 and 32.  Batch 64 holds too much
-    # device memory for a multi-pass capture: its figures extend the 16 and 32
-    # captures linearly in the correlograms per launch (colpass 3.657 -> 7.357
-    # GB for 48 -> 96; rowpass 4.042 -> 7.282 GB, of which 0.80 GB is the map
-    # read-modify-write that does not grow).
-    measured_traffic = {("production", 8, "colpass"): 1.875e9, ("production", 8, "rowpass"): 2.390e9,
-                        ("production", 16, "colpass"): 3.657e9, ("production", 16, "rowpass"): 4.042e9,
-                        ("production", 32, "colpass"): 7.357e9, ("production", 32, "rowpass"): 7.282e9,
-                        ("production", 64, "colpass"): 14.757e9, ("production", 64, "rowpass"): 13.762e9}
+    # workload (dram__bytes_read.sum + dram__bytes_write.sum, one launch each)
+    # at orientation batch 16 and 32.  Batch 64 holds too much device memory for
+    # a multi-pass capture: its figures, and batch 8's, extend these linearly in
+    # the correlograms per launch (48 -> 96: colpass 3.619 -> 7.163 GB, rowpass
+    # 4.085 -> 7.319 GB, of which 0.85 GB is the map read-modify-write that does
+    # not grow).
+    measured_traffic = {("production", 8, "colpass"): 1.847e9, ("production", 8, "rowpass"): 2.468e9,
+                        ("production", 16, "colpass"): 3.619e9, ("production", 16, "rowpass"): 4.085e9,
+                        ("production", 32, "colpass"): 7.163e9, ("production", 32, "rowpass"): 7.319e9,
+                        ("production", 64, "colpass"): 14.251e9, ("production", 64, "rowpass"): 13.787e9}
     roofline = {
         "bound": "hbm", "kernel": top, "achieved": ach, "peak": peaks["hbm_gbs"], "unit": "GB/s",
         "frac": (ach / peaks["hbm_gbs"]) if ach else None,
