@@ -42,6 +42,13 @@ int launch_norm_constants(double* rowstats, int n_c, int h, int norm_h, int norm
 // norm_ready: rowstats already holds the constants of launch_norm_constants.
 int launch_pad_rfft(int W, const float* proj, const double* rowstats, int h, int norm_h, int norm_w, int Wcp,
                     int n_c, void* A, cudaStream_t s, bool norm_ready = false);
+// Its longer rows (match_pad_reg.cuh).
+#define LGB_PAD_REG_SIZES(X) X(512) X(1024) X(2048) X(2880) X(3072) X(3840) X(4096) X(5760)
+#define X(n)                                                                                                          \
+  int launch_pad_rfft_##n(const float* proj, const double* rowstats, int h, int norm_h, int norm_w, int Wcp, int n_c, \
+                          void* A, cudaStream_t s, bool norm_ready);
+LGB_PAD_REG_SIZES(X)
+#undef X
 // Ip holds one spectrum per image, H rows of ips columns (W/2 + 1 <= ips <= Wcp,
 // Wcp = W/2 + 1 rounded up to 4); correlogram c uses image c / c_per_image.
 // Only rows y < y_rows of each inverse column transform are stored (Y is [n_c][y_rows][Wcp]).

@@ -86,39 +86,24 @@ template <int WH>
 static int pad_rfft_t(const float* proj, const double* rowstats, int h, int norm_h, int norm_w, int Wcp, int n_c,
                       void* A, cudaStream_t s, bool norm_ready) {
   constexpr int NT = FftThreads<WH>::value;
-  if constexpr (WH >= 1024) {
-    // long rows: tables in dynamic shared memory, 32 rows per CTA, constants precomputed
-    constexpr int ROWS = 2, RPC = 32;
-    using PR = PadRows<WH, ROWS>;
-    if (!norm_ready) {
-      const int st = launch_norm_constants(const_cast<double*>(rowstats), n_c, h, norm_h, norm_w, s);
-      if (st) return st;
-    }
-    if (cudaFuncSetAttribute(pad_rfft_rows_kernel<WH, ROWS, RPC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)PR::SMEM) != cudaSuccess)
-      return LGB_ERR_CUDA;
-    return launch_chained(pad_rfft_rows_kernel<WH, ROWS, RPC>, dim3((h + RPC - 1) / RPC, n_c), dim3(ROWS * NT), PR::SMEM,
-                          s, proj, rowstats, h, Wcp, static_cast<float2*>(A));
-  } else {
-    // at least one full warp: the normalisation reduction shuffles across warp 0
-    constexpr int ROWS0 = NT >= 128 ? 2 : (NT >= 32 ? 4 : (NT >= 16 ? 8 : 16));
-    constexpr int ROWS1 = ROWS0 * NT >= 32 ? ROWS0 : (32 + NT - 1) / NT;
-    // static shared memory (ROWS rows of the padded transform) stays under 40 KB
-    constexpr int ROWS = ROWS1 * (IdxPad16::pad(WH) + 2) * 8 <= 40960 ? ROWS1 : 1;
-    static_assert(ROWS * NT >= 32, "pad_rfft CTA must hold a full warp");
-    const int ctas = (h + ROWS - 1) / ROWS;
-    // precompute the constants when many CTAs share a correlogram (each would
-    // otherwise reduce all h rows in FP64); a few CTAs do it themselves
-    const int ready = norm_ready || ctas >= 16;
-    if (ready && !norm_ready) {
-      const int st = launch_norm_constants(const_cast<double*>(rowstats), n_c, h, norm_h, norm_w, s);
-      if (st) return st;
-    }
-    dim3 grid(ctas, n_c);
-    // shared twiddle tables where a CTA transforms >= 4 rows
-    return launch_chained(pad_rfft_kernel<WH, ROWS, (ROWS >= 4)>, grid, dim3(ROWS * NT), 0, s, proj, rowstats, h,
-                          NormSizes(h, norm_h, norm_w), Wcp, ready, static_cast<float2*>(A));
+  // at least one full warp: the normalisation reduction shuffles across warp 0
+  constexpr int ROWS0 = NT >= 128 ? 2 : (NT >= 32 ? 4 : (NT >= 16 ? 8 : 16));
+  constexpr int ROWS1 = ROWS0 * NT >= 32 ? ROWS0 : (32 + NT - 1) / NT;
+  // static shared memory (ROWS rows of the padded transform) stays under 40 KB
+  constexpr int ROWS = ROWS1 * (IdxPad16::pad(WH) + 2) * 8 <= 40960 ? ROWS1 : 1;
+  static_assert(ROWS * NT >= 32, "pad_rfft CTA must hold a full warp");
+  const int ctas = (h + ROWS - 1) / ROWS;
+  // precompute the constants when many CTAs share a correlogram (each would
+  // otherwise reduce all h rows in FP64); a few CTAs do it themselves
+  const int ready = norm_ready || ctas >= 16;
+  if (ready && !norm_ready) {
+    const int st = launch_norm_constants(const_cast<double*>(rowstats), n_c, h, norm_h, norm_w, s);
+    if (st) return st;
   }
+  dim3 grid(ctas, n_c);
+  // shared twiddle tables where a CTA transforms >= 4 rows
+  return launch_chained(pad_rfft_kernel<WH, ROWS, (ROWS >= 4)>, grid, dim3(ROWS * NT), 0, s, proj, rowstats, h,
+                        NormSizes(h, norm_h, norm_w), Wcp, ready, static_cast<float2*>(A));
 }
 
 template <int WH>
@@ -138,11 +123,17 @@ int launch_pad_rfft(int W, const float* proj, const double* rowstats, int h, int
                     int n_c, void* A, cudaStream_t s, bool norm_ready) {
   if (W % 2 || norm_w > W || norm_w < h || norm_h < h) return LGB_ERR_UNSUPPORTED_SIZE;
   if (!supported_row(W)) return LGB_ERR_UNSUPPORTED_SIZE;
+  if (h % 2) return LGB_ERR_UNSUPPORTED_SIZE;
   switch (W / 2) {
+#define X(n)  \
+  case n / 2: \
+    return launch_pad_rfft_##n(proj, rowstats, h, norm_h, norm_w, Wcp, n_c, A, s, norm_ready);
+    LGB_PAD_REG_SIZES(X)
+#undef X
 #define X(n) \
   case n:    \
     return pad_rfft_t<n>(proj, rowstats, h, norm_h, norm_w, Wcp, n_c, A, s, norm_ready);
-    LGB_ROW_SIZES(X)
+    LGB_ROW_GENERIC_SIZES(X)
 #undef X
     default:
       return LGB_ERR_UNSUPPORTED_SIZE;

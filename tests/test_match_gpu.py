@@ -278,6 +278,18 @@ def test_long_row_pass_against_oracle(W, H, n_o, batch, n_df):
     _assert_parity(gpu, ref, second=ref["second_best"])
 
 
+@pytest.mark.parametrize("W,d,batch", [(512, 384, 3), (1024, 384, 3), (2048, 288, 3), (2880, 288, 3), (3072, 96, 40),
+                                       (3840, 288, 3), (4096, 384, 3), (5760, 288, 3), (512, 48, 40)])
+def test_padded_rows_against_oracle(W, d, batch):
+    """Padded row transforms: templates that fill most of the first pass, odd row shares,
+    normalisation constants reduced in place (few correlograms) and precomputed (many)."""
+    kw = _small_workload(512, W, d, batch + 2, 1)
+    gpu = _gpu_search(kw, batch)
+    ref = orc.core_match_template_cpu(**kw, orientation_batch_size=batch, track_second_best=True,
+                                      stat_dtype=torch.float64, compute_dtype=torch.float64, device="cuda:0")
+    _assert_parity(gpu, ref, second=ref["second_best"])
+
+
 @pytest.mark.parametrize("W,batch", [(512, 17), (512, 9), (1024, 13), (1024, 7), (2048, 7)])
 @pytest.mark.parametrize("H", [48, 64])
 def test_split_row_pass_against_oracle(W, batch, H):
