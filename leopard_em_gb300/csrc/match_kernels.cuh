@@ -101,14 +101,15 @@ __global__ void __launch_bounds__(COLS* FftThreads<HT>::value)
   }
 }
 
-// proj_col for HT = R1*R2 (256 = 16*16) in two register passes: radix R1
+// proj_col for HT = R1*R2 (ProjSplit, match_proj.cu) in two register passes: radix R1
 // over rows t + R2*q of slice x filter straight from global memory ->
 // shared transpose M1[t][q] (odd stride R1+1; column stride 2 mod 16) ->
 // radix R2 with twiddles w^(r*t), w = exp(+2 pi i / HT) -> rows t + R1*r of T.
 // G columns per CTA (lane bits 0-2), one thread per butterfly.
-template <int R1, int R2>
+// R2 = R2A R2B: above 18 points a composite transform in registers.
+template <int R1, int R2A, int R2B>
 struct ProjColPair {
-  static constexpr int HT = R1 * R2;
+  static constexpr int R2 = R2A * R2B, HT = R1 * R2;
   static constexpr int NT = R1 > R2 ? R1 : R2;
   static constexpr int G = 8;
   static constexpr int S1 = R1 + 1;
@@ -117,12 +118,12 @@ struct ProjColPair {
   static constexpr int NROOT = (R1 - 1) * (R2 - 1) + 1;
 };
 
-template <int R1, int R2>
-__global__ void __launch_bounds__(ProjColPair<R1, R2>::G* ProjColPair<R1, R2>::NT)
+template <int R1, int R2A, int R2B>
+__global__ void __launch_bounds__(ProjColPair<R1, R2A, R2B>::G* ProjColPair<R1, R2A, R2B>::NT)
     proj_col_pair_kernel(const float2* __restrict__ slices, const float* __restrict__ pf, int nb, int n_cd,
                          float2* __restrict__ T) {
-  using PC = ProjColPair<R1, R2>;
-  constexpr int HT = PC::HT, WC = HT / 2 + 1, G = PC::G, S1 = PC::S1;
+  using PC = ProjColPair<R1, R2A, R2B>;
+  constexpr int R2 = PC::R2, HT = PC::HT, WC = HT / 2 + 1, G = PC::G, S1 = PC::S1;
   __shared__ float2 buf[G * PC::STRIDE];
   __shared__ float2 root[PC::NROOT];  // exp(+2 pi i m / HT)
   for (int m = threadIdx.x; m < PC::NROOT; m += blockDim.x) {
@@ -164,11 +165,14 @@ __global__ void __launch_bounds__(ProjColPair<R1, R2>::G* ProjColPair<R1, R2>::N
     float2 w[R2];
 #pragma unroll
     for (int r = 0; r < R2; ++r) w[r] = cmul(x[r * S1 + t], root[r * t]);
-    Dft<R2, +1>::run(w);
+    if constexpr (R2A == 1)
+      Dft<R2, +1>::run(w);
+    else
+      DftNT<R2A, R2B, +1>::run(w);
     if (col_ok) {
       float2* out = T + (size_t)c * HT * WC + (size_t)t * WC + kx;
 #pragma unroll
-      for (int r = 0; r < R2; ++r) out[(size_t)r * R1 * WC] = w[r];
+      for (int s = 0; s < R2; ++s) out[(size_t)(R2A == 1 ? s : DftNT<R2A, R2B, +1>::out(s)) * R1 * WC] = w[s];
     }
   }
 }
@@ -253,7 +257,7 @@ __global__ void __launch_bounds__(ROWS* FftThreads<HT / 2>::value)
   }
 }
 
-// proj_row for HT/2 = R1*R2 (128 = 16*8) in two register passes: the c2r
+// proj_row for HT/2 = R1*R2 (ProjSplit) in two register passes: the c2r
 // pre-twiddle is applied while loading the radix-R1 inputs k = t + R2*q from
 // the staged row; shared transpose M1[t][q]; radix R2 with twiddles w^(r*t)
 // leaves pixel pairs m = t + R1*r in thread t.  Same outputs, ifftshift and

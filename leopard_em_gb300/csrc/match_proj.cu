@@ -101,34 +101,60 @@ int launch_slice(const void* vol, int d, const float* euler, int o0, const int* 
 }
 
 constexpr int kProjCols = 8;
-constexpr int kProjRows = 8;
+
+// Splits of the template sizes for the two-pass kernels: d = R1 R2 of the column
+// pass (R2 = A x B), d / 2 = R1 R2 of the row pass; 0: the generic kernel
+// (d / 2 = 96 has no split whose rows are lane aligned).  Against three to
+// five passes through shared memory, microseconds for 96 correlograms, columns
+// and rows: 64 4.8 + 4.2 -> 3.3 + 4.2, 128 6.9 + 6.9 -> 5.2 + 5.6, 192 12.8 -> 8.3
+// (columns), 288 32 + 40 -> 16 + 20, 384 38 + 54 -> 23 + 34, 512 59 + 70 -> 40 + 60;
+// for two correlograms 288 7.5 + 7.4 -> 3.9 + 4.6.
+template <int HT>
+struct ProjSplit {
+  static constexpr int COL1 = 0, COL2A = 0, COL2B = 0, ROW1 = 0, ROW2 = 0, ROWS = 8;
+};
+#define LGB_PROJ_SPLIT(n, c1, c2a, c2b, r1, r2, rows)                                                      \
+  template <>                                                                                              \
+  struct ProjSplit<n> {                                                                                    \
+    static constexpr int COL1 = c1, COL2A = c2a, COL2B = c2b, ROW1 = r1, ROW2 = r2, ROWS = rows;           \
+  };
+LGB_PROJ_SPLIT(64, 8, 1, 8, 8, 4, 16)
+LGB_PROJ_SPLIT(96, 12, 1, 8, 16, 3, 8)
+LGB_PROJ_SPLIT(128, 16, 1, 8, 8, 8, 16)
+LGB_PROJ_SPLIT(192, 16, 1, 12, 0, 0, 8)
+LGB_PROJ_SPLIT(256, 16, 1, 16, 16, 8, 8)
+LGB_PROJ_SPLIT(288, 16, 1, 18, 16, 9, 8)
+LGB_PROJ_SPLIT(384, 16, 3, 8, 16, 12, 8)
+LGB_PROJ_SPLIT(512, 16, 4, 8, 16, 16, 8)
+#undef LGB_PROJ_SPLIT
 
 template <int HT>
 static int proj_col_t(const void* slices, const float* pf, int nb, int n_cd, int n_c, void* T, cudaStream_t s) {
   constexpr int WC = HT / 2 + 1;
-  if constexpr (HT == 256) {
-    // two register passes (16 x 16), 8 columns per CTA
-    using PC = ProjColPair<16, 16>;
+  using PS = ProjSplit<HT>;
+  if constexpr (PS::COL1 > 0) {
+    using PC = ProjColPair<PS::COL1, PS::COL2A, PS::COL2B>;
     dim3 pgrid((WC + PC::G - 1) / PC::G, n_c);
-    return launch_chained(proj_col_pair_kernel<16, 16>, pgrid, dim3(PC::G * PC::NT), 0, s,
+    return launch_chained(proj_col_pair_kernel<PS::COL1, PS::COL2A, PS::COL2B>, pgrid, dim3(PC::G * PC::NT), 0, s,
+                          static_cast<const float2*>(slices), pf, nb, n_cd, static_cast<float2*>(T));
+  } else {
+    dim3 grid((WC + kProjCols - 1) / kProjCols, n_c);
+    return launch_chained(proj_col_kernel<HT, kProjCols>, grid, dim3(kProjCols * FftThreads<HT>::value), 0, s,
                           static_cast<const float2*>(slices), pf, nb, n_cd, static_cast<float2*>(T));
   }
-  dim3 grid((WC + kProjCols - 1) / kProjCols, n_c);
-  return launch_chained(proj_col_kernel<HT, kProjCols>, grid, dim3(kProjCols * FftThreads<HT>::value), 0, s,
-                        static_cast<const float2*>(slices), pf, nb, n_cd, static_cast<float2*>(T));
 }
 
 template <int HT>
 static int proj_row_t(const void* T, int n_c, float* proj, double* rowstats, cudaStream_t s) {
-  static_assert(HT % kProjRows == 0, "rows per CTA must divide the template size");
-  dim3 grid(HT / kProjRows, n_c);
-  if constexpr (HT == 256) {
-    // two register passes (16 x 8) of the 128-point c2r, 16 threads per row
-    return launch_chained(proj_row_pair_kernel<16, 8, kProjRows>, grid, dim3(kProjRows * 16), 0, s,
+  using PS = ProjSplit<HT>;
+  static_assert(HT % PS::ROWS == 0, "rows per CTA must divide the template size");
+  dim3 grid(HT / PS::ROWS, n_c);
+  if constexpr (PS::ROW1 > 0)
+    return launch_chained(proj_row_pair_kernel<PS::ROW1, PS::ROW2, PS::ROWS>, grid, dim3(PS::ROWS * PS::ROW1), 0, s,
                           static_cast<const float2*>(T), proj, rowstats);
-  }
-  return launch_chained(proj_row_kernel<HT, kProjRows>, grid, dim3(kProjRows * FftThreads<HT / 2>::value), 0, s,
-                        static_cast<const float2*>(T), proj, rowstats);
+  else
+    return launch_chained(proj_row_kernel<HT, PS::ROWS>, grid, dim3(PS::ROWS * FftThreads<HT / 2>::value), 0, s,
+                          static_cast<const float2*>(T), proj, rowstats);
 }
 
 bool supported_proj_row_rfft(int h, int W) { return h == 256 && W == 288; }

@@ -290,6 +290,16 @@ def test_padded_rows_against_oracle(W, d, batch):
     _assert_parity(gpu, ref, second=ref["second_best"])
 
 
+@pytest.mark.parametrize("d", [16, 32, 48, 64, 96, 128, 192, 256, 288, 384])
+def test_projection_passes_against_oracle(d):
+    """Projection columns and rows of every template size, several filter planes a slice."""
+    kw = _small_workload(512, 512, d, 9, 3)
+    gpu = _gpu_search(kw, 4)
+    ref = orc.core_match_template_cpu(**kw, orientation_batch_size=4, track_second_best=True,
+                                      stat_dtype=torch.float64, compute_dtype=torch.float64, device="cuda:0")
+    _assert_parity(gpu, ref, second=ref["second_best"])
+
+
 @pytest.mark.parametrize("W,batch", [(512, 17), (512, 9), (1024, 13), (1024, 7), (2048, 7)])
 @pytest.mark.parametrize("H", [48, 64])
 def test_split_row_pass_against_oracle(W, batch, H):
