@@ -8,6 +8,8 @@ or a call fails, a RuntimeError (ValueError for bad arguments) is raised.
 from __future__ import annotations
 
 import ctypes
+import functools
+import hashlib
 import os
 import threading
 
@@ -162,6 +164,18 @@ class StageProfile:
 
 def library_path() -> str:
     return _build.LIB_PATH
+
+
+@functools.cache
+def _file_digest(path: str) -> str:
+    with open(path, "rb") as f:
+        return hashlib.file_digest(f, "sha256").hexdigest()[:16]
+
+
+def library_digest() -> str:
+    """Digest of the library file: one build's measurements do not stand for
+    another's (the version number does not change with every kernel)."""
+    return _file_digest(library_path())
 
 
 def lib():

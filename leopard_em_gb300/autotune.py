@@ -13,7 +13,7 @@ the cost of a larger intermediate) and the column pass's grid split
 (``col_waves``: how many waves of CTAs the correlogram loop is split into).
 ``tune_search`` times candidates on the caller's own inputs with CUDA events,
 by coordinate descent (grid at B = 8, then B on the best grid, then the split),
-and caches the winner per device and search shape in a JSON file
+and caches the winner per device, library build and search shape in a JSON file
 (``$LEOPARD_EM_GB300_TUNE_CACHE``, default
 ``~/.cache/leopard_em_gb300/autotune.json``).  The reference has no
 counterpart: its orientation batch is a user setting
@@ -29,7 +29,7 @@ from dataclasses import asdict, dataclass
 
 import torch
 
-from ._native import lib
+from ._native import lib, library_digest
 
 CACHE_ENV = "LEOPARD_EM_GB300_TUNE_CACHE"
 DEFAULT_BATCHES = (2, 4, 8, 12, 16, 24, 32, 48, 64)
@@ -90,7 +90,7 @@ def _store_cache(path: str, key: str, value: dict) -> None:
 def tuning_key(device: torch.device, grid: tuple[int, int], micrograph: tuple[int, int], template_size: int,
                n_pixel_sizes: int, n_defocus: int) -> str:
     name = torch.cuda.get_device_name(device).replace(" ", "_")
-    return (f"{name}/v{lib().lgb_version()}/grid{grid[0]}x{grid[1]}/mic{micrograph[0]}x{micrograph[1]}"
+    return (f"{name}/v{lib().lgb_version()}-{library_digest()}/grid{grid[0]}x{grid[1]}/mic{micrograph[0]}x{micrograph[1]}"
             f"/d{template_size}/C{n_pixel_sizes}/D{n_defocus}")
 
 

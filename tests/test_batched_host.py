@@ -55,6 +55,22 @@ def test_tuning_cache_round_trip(tmp_path, monkeypatch):
     assert autotune._load_cache(str(path)) == {}
 
 
+def test_tunings_of_another_build_are_not_used(tmp_path, monkeypatch):
+    """The cache key follows the library file: kernels change without the version number."""
+    import torch
+
+    from leopard_em_gb300 import _native
+
+    monkeypatch.setattr(torch.cuda, "get_device_name", lambda device=None: "GPU")
+    shape = (torch.device("cuda:0"), (512, 512), (512, 512), 64, 1, 1)
+    mine = autotune.tuning_key(*shape)
+    assert autotune.tuning_key(*shape) == mine
+    other = tmp_path / "lib.so"
+    other.write_bytes(b"another build")
+    monkeypatch.setattr(_native, "library_path", lambda: str(other))
+    assert autotune.tuning_key(*shape) != mine
+
+
 def test_graph_batches_heuristic():
     assert autotune.SearchTuning.graph_batches_for(8) == 16
     assert autotune.SearchTuning.graph_batches_for(200) == 1
