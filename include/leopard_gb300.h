@@ -61,8 +61,9 @@ typedef struct lgb_match_problem {
   int micrograph_h;
   int micrograph_w;
   /* Column-pass launch shape: split correlograms over CTAs until the grid
-   * covers about col_waves x the SM count (0 = 4).  Results do not depend on
-   * it. */
+   * covers about col_waves x the SM count.  0: the library's choice (the
+   * cheapest split by its cost model where the column length has one, else 4).
+   * Results do not depend on it. */
   int col_waves;
 } lgb_match_problem;
 

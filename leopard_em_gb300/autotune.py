@@ -6,13 +6,15 @@ transposed micrograph puts its width on the column transform, which pays when
 the height has only a slow column kernel, e.g. 5760 rows), the correlation
 grid (the FFT lengths; a micrograph may be
 zero padded past the smallest compiled grid to a power of two, whose
-transforms have the register-fused kernels), the orientation batch B
+transforms can still be faster), the orientation batch B
 (correlograms per statistics update: larger batches amortise the
 image-spectrum read and the map read-modify-write over more correlograms, at
 the cost of a larger intermediate) and the column pass's grid split
-(``col_waves``: how many waves of CTAs the correlogram loop is split into).
+(``col_waves``: 0 for the library's own choice, else how many waves of CTAs the
+correlogram loop is split into).
 ``tune_search`` times candidates on the caller's own inputs with CUDA events,
-by coordinate descent (grid at B = 8, then B on the best grid, then the split),
+by coordinate descent (grid at B = 8, then B on the best grid, both with the
+library's own split, then the split),
 and caches the winner per device, library build and search shape in a JSON file
 (``$LEOPARD_EM_GB300_TUNE_CACHE``, default
 ``~/.cache/leopard_em_gb300/autotune.json``).  The reference has no
@@ -34,7 +36,7 @@ from ._native import lib, library_digest
 CACHE_ENV = "LEOPARD_EM_GB300_TUNE_CACHE"
 DEFAULT_BATCHES = (2, 4, 8, 12, 16, 24, 32, 48, 64)
 MAX_BATCH_CORRELOGRAMS = 1024  # C * D * B cap: larger batches gain little and hold a big intermediate
-DEFAULT_WAVES = (2, 4, 8)
+DEFAULT_WAVES = (0, 2, 4, 8)
 TRANSPOSE_GAIN = 0.9  # a transposed grid must time at most this fraction of the best direct one
 _lock = threading.Lock()
 
@@ -177,7 +179,7 @@ def tune_search(image_dft, template_dft, ctf_filters, whitening_filter_template,
                 timings[cand] = _time_candidate(make_search, cand, n_probe, repeats)
             return timings[cand]
 
-        w0 = 4 if 4 in waves else waves[0]
+        w0 = next((w for w in (0, 4) if w in waves), waves[0])
         b0 = 8 if 8 in batches else batches[0]
         grid_cands = [g for g in grids if fits(g, b0)] or grids[:1]
         direct = [g for g in grid_cands if not g[1]] or grid_cands[:1]

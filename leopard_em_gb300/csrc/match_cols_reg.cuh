@@ -285,14 +285,15 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
 // the split whose rounds are cheapest, a CTA costing its correlograms plus
 // about one more for its roots and image columns (4096 rows, 48 correlograms:
 // 48 / 24 / 12 per CTA measured 33.8 / 31.9 / 32.4 us per correlogram).  A
-// caller's `waves` asks for about that many rounds instead.
-inline int colpass_per_block(int groups, int n_c, int slots, int waves) {
+// caller's `waves` asks for about waves x the SM count CTAs instead.
+inline int colpass_per_block(int groups, int n_c, int sms, int per_sm, int waves) {
   if (waves > 0) {
     int split = 1;
-    while (split < n_c && groups * split < waves * slots) split *= 2;
+    while (split < n_c && (long long)groups * split < (long long)waves * sms) split *= 2;
     if (split > n_c) split = n_c;
     return (n_c + split - 1) / split;
   }
+  const int slots = sms * per_sm;
   int best = n_c;
   long long best_cost = -1;
   for (int split = 1; split <= n_c && split <= 64; ++split) {
@@ -317,7 +318,7 @@ int colpass_reg_launch(const void* A, const void* Ip, int ips, int h, int Wcp, i
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int groups = (Wcp + C::G - 1) / C::G;
-  const int per = colpass_per_block(groups, n_c, sms * C::MINB, waves);
+  const int per = colpass_per_block(groups, n_c, sms, C::MINB, waves);
   return launch_chained(colpass_reg_kernel<C, SPARSE>, dim3(groups, (n_c + per - 1) / per), dim3(C::THREADS), C::SMEM, s,
                         static_cast<const float2*>(A), static_cast<const float2*>(Ip), ips, h, Wcp, n_c, per, cpi,
                         y_rows, static_cast<float2*>(Y));

@@ -53,7 +53,8 @@ LGB_PAD_REG_SIZES(X)
 // Wcp = W/2 + 1 rounded up to 4); correlogram c uses image c / c_per_image.
 // Only rows y < y_rows of each inverse column transform are stored (Y is [n_c][y_rows][Wcp]).
 // waves: the correlogram range is split until the grid covers about waves x
-// the SM count (0 = 4).
+// the SM count (0 = colpass_per_block's cheapest split for LGB_COL_REG_SIZES, 4
+// for the others).
 // norm (H = 288 only; null otherwise): A holds un-normalised row spectra of
 // length norm_w rows and correlogram c is normalised on load as
 // s (A - e U[kx]), (e, s) = norm[c * norm_stride], U[k] = sum_{x < h} exp(-2 pi i k x / norm_w).

@@ -144,6 +144,17 @@ def test_col_waves_do_not_change_results():
         assert torch.equal(v, b["_maps"][k]), k
 
 
+@pytest.mark.parametrize("H,W", [(512, 64), (576, 64), (1024, 48), (2048, 48), (4096, 48), (5760, 48)])
+def test_col_waves_of_the_register_passes(H, W):
+    """Every split of the correlograms, the library's own (0) among them, gives the same maps."""
+    kw = _workload(H, W, 32, 12, n_df=2)
+    ref = _search(kw, 6)
+    for waves in (1, 2, 3, 8, 1000000):
+        got = _search(kw, 6, col_waves=waves)
+        for k, v in ref["_maps"].items():
+            assert torch.equal(v, got["_maps"][k]), (waves, k)
+
+
 def test_autotuner_picks_valid_parameters_and_caches(tmp_path, monkeypatch):
     monkeypatch.setenv(autotune.CACHE_ENV, str(tmp_path / "tune.json"))
     kw = _workload(512, 512, 64, 24, n_df=2)

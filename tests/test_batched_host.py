@@ -71,6 +71,11 @@ def test_tunings_of_another_build_are_not_used(tmp_path, monkeypatch):
     assert autotune.tuning_key(*shape) != mine
 
 
+def test_tuner_can_choose_the_librarys_own_column_split():
+    """col_waves 0 is a choice of its own (no power of two reaches it)."""
+    assert 0 in autotune.DEFAULT_WAVES
+
+
 def test_graph_batches_heuristic():
     assert autotune.SearchTuning.graph_batches_for(8) == 16
     assert autotune.SearchTuning.graph_batches_for(200) == 1
