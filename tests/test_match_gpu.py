@@ -359,3 +359,34 @@ def test_finalize_against_64_bits(H, W):
     assert torch.isnan(res["correlation_mean"][0, 5]) and res["scaled_mip"][0, 5] == 0
     assert torch.equal(res["best_phi"], kw["euler_angles"][idx % 12, 0][:H, :W])
     assert torch.equal(res["best_defocus"], kw["defocus_values"][idx // 12][:H, :W])
+
+
+@pytest.mark.parametrize("W", [512, 1024, 2048, 2880, 3072, 3840, 4096, 5760])
+@pytest.mark.parametrize("batch", [5, 17])
+def test_large_magnitudes_scale_exactly(W, batch):
+    """An image times a power of two: every map scales by it, bit for bit, as
+    long as a correlogram's own square fits FP32 (not H W times as much)."""
+    kw = _small_workload(64, W, 32, 17, 1)
+    f = 2.0**50
+    a, b = (MatchTemplateSearch(**k, device=torch.device("cuda:0"), orientation_batch_size=batch)
+            for k in (kw, dict(kw, image_dft=kw["image_dft"] * f)))
+    a.run()
+    b.run()
+    ma, mb = a.maps(), b.maps()
+    assert torch.equal(mb["correlation_squared_sum"], ma["correlation_squared_sum"] * f * f)
+    assert torch.equal(mb["correlation_sum"], ma["correlation_sum"] * f)
+    assert torch.equal(mb["mip"], ma["mip"] * f)
+    assert torch.equal(mb["best_global_index"], ma["best_global_index"])
+
+
+@pytest.mark.parametrize("W", [512, 1024, 2048, 2880, 3072, 3840, 4096, 5760])
+def test_ties_do_not_depend_on_the_batch(W):
+    """Orientations that differ by rounding only: many pixels tie, and the first
+    index wins whether the tie falls within a batch or between two."""
+    kw = _small_workload(64, W, 32, 18, 1)
+    kw["euler_angles"] = kw["euler_angles"][:1] + 1e-5 * torch.arange(18)[:, None] * torch.tensor([[1.0, 0.0, 0.5]])
+    one, many = (MatchTemplateSearch(**kw, device=torch.device("cuda:0"), orientation_batch_size=b) for b in (1, 18))
+    one.run()
+    many.run()
+    assert torch.equal(one.mip, many.mip)
+    assert torch.equal(one.best_index, many.best_index)
