@@ -31,10 +31,14 @@ __global__ void filters_kernel(const float* __restrict__ ctf, const float* __res
 // What bounds it: the maps' traffic (56 B a pixel), now that the FP64 pipe (one
 // operation per SM per clock) is left with the mean and the variance: the
 // standard deviation and z are carried in pairs of floats (48 bits), split from
-// the doubles by integer operations.  24 M pixels: 1,731 us with FP64 division
-// and square root, 793 us with an FP64 Newton step, 365 us now.
+// the doubles by integer operations, and ranges are compared by exponents.  24 M
+// pixels: 1,731 us with FP64 division and square root, 793 us with an FP64
+// Newton step, 369 us with FP64 comparisons, 250 us now.
+// The count's reciprocal is rounded: where the variance is below 2^-24 of the
+// mean's square (never in a search of noise) both are divided out instead, so
+// that a small spread keeps its digits and equal correlograms have none.
 __global__ void __launch_bounds__(256)
-    finalize_kernel(int out_h, int out_w, int W, double inv_total, unsigned stride_cs, unsigned n_orient,
+    finalize_kernel(int out_h, int out_w, int W, double total, double inv_total, unsigned stride_cs, unsigned n_orient,
                     const float* __restrict__ mip, const int* __restrict__ best, const double* __restrict__ s1,
                     const double* __restrict__ s2, const float* __restrict__ euler, const float* __restrict__ defocus,
                     float* __restrict__ mip_out, float* __restrict__ scaled, float* __restrict__ phi,
@@ -45,30 +49,36 @@ __global__ void __launch_bounds__(256)
       const size_t i = (size_t)y * W + x, o = (size_t)y * out_w + x;
       const float m = mip[i];
       const int g = best[i];
-      const double mean = s1[i] * inv_total;
-      const double var = fma(-mean, mean, s2[i] * inv_total);
+      double mean = s1[i] * inv_total;
+      double var = fma(-mean, mean, s2[i] * inv_total);
+      // (exponents as integers: a double comparison takes the FP64 pipe, too)
+      const int em = (__double2hiint(mean) >> 20) & 0x7ff;
+      int ev = __double2hiint(var) >> 20;  // negative with var
+      if (ev < 1 || ev < 2 * em - 1023 - 24) {
+        mean = s1[i] / total;
+        var = fma(-mean, mean, s2[i] / total);
+        ev = __double2hiint(var) >> 20;
+      }
       float z = 0.f, sd = 0.f;  // also where var is not a number
-      if (var > 0.0) {
-        if (var > 1e-20 && var < 1e20 && fabs(mean) < 1e20 && fabsf(m) < 1e20f) {
-          const float2 v = d2f_split(var), mu = d2f_split(mean);
-          // 1/sd = y + dy: a float reciprocal square root and its first-order
-          // correction from the exact residual e = 1 - var y^2 (e^2 is below 48 bits)
-          const float y = rsqrtf(v.x);
-          const float p = y * y, pe = fmaf(y, y, -p);
-          const float e = fmaf(-v.x, p, 1.f) - fmaf(v.x, pe, v.y * p);
-          const float dy = 0.5f * y * e;
-          const float s = v.x * y;
-          sd = s + (fmaf(v.x, y, -s) + fmaf(v.y, y, v.x * dy));
-          // m - mean as a sum of two floats
-          const float d = m - mu.x, back = m - d;
-          const float dl = ((m - (d + back)) + (back - mu.x)) - mu.y;
-          const float q = d * y;
-          z = q + (fmaf(d, y, -q) + fmaf(dl, y, d * dy));
-        } else {
-          const double s = sqrt(var);
-          sd = (float)s;
-          z = (float)(((double)m - mean) / s);
-        }
+      if (ev > 1023 - 66 && ev < 1023 + 66 && em < 1023 + 66 && fabsf(m) < 1e20f) {
+        const float2 v = d2f_split(var), mu = d2f_split(mean);
+        // 1/sd = y + dy: a float reciprocal square root and its first-order
+        // correction from the exact residual e = 1 - var y^2 (e^2 is below 48 bits)
+        const float y = rsqrtf(v.x);
+        const float p = y * y, pe = fmaf(y, y, -p);
+        const float e = fmaf(-v.x, p, 1.f) - fmaf(v.x, pe, v.y * p);
+        const float dy = 0.5f * y * e;
+        const float s = v.x * y;
+        sd = s + (fmaf(v.x, y, -s) + fmaf(v.y, y, v.x * dy));
+        // m - mean as a sum of two floats
+        const float d = m - mu.x, back = m - d;
+        const float dl = ((m - (d + back)) + (back - mu.x)) - mu.y;
+        const float q = d * y;
+        z = q + (fmaf(d, y, -q) + fmaf(dl, y, d * dy));
+      } else if (var > 0.0) {
+        const double s = sqrt(var);
+        sd = (float)s;
+        z = (float)(((double)m - mean) / s);
       }
       if (mip_out) mip_out[o] = m;
       scaled[o] = z;
@@ -406,7 +416,7 @@ static int finalize_maps(const lgb_match_problem* p, int out_h, int out_w, long 
   const unsigned stride_cs = stride > 0xffffffffLL ? 0xffffffffu : (unsigned)stride;
   const int gx = (out_w + 255) / 256, gy = out_h < 65535 ? out_h : 65535;
   finalize_kernel<<<dim3(gx, gy), 256, 0, (cudaStream_t)stream>>>(
-      out_h, out_w, p->image_w, 1.0 / (double)total_positions, stride_cs, (unsigned)p->n_orientations, mip, best_index,
+      out_h, out_w, p->image_w, (double)total_positions, 1.0 / (double)total_positions, stride_cs, (unsigned)p->n_orientations, mip, best_index,
       corr_sum, corr_sq_sum, euler_angles, defocus_values, mip_out, scaled_mip, best_phi, best_theta, best_psi,
       best_defocus, corr_mean, corr_std);
   return cudaGetLastError() == cudaSuccess ? LGB_OK : LGB_ERR_CUDA;

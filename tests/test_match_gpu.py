@@ -390,3 +390,25 @@ def test_ties_do_not_depend_on_the_batch(W):
     many.run()
     assert torch.equal(one.mip, many.mip)
     assert torch.equal(one.best_index, many.best_index)
+
+
+@pytest.mark.parametrize("n_o,n_df", [(7, 7), (1, 3), (41, 3), (36, 11)])
+def test_finalize_of_constant_pixels(n_o, n_df):
+    """Equal correlograms with exact sums have no spread: std 0 and z 0.  Small
+    and large spreads about a zero mean hold every digit (outputs are rounded
+    once to float32: 1e-6 relative)."""
+    kw = _small_workload(48, 64, 32, n_o, n_df)
+    s = MatchTemplateSearch(**kw, device=torch.device("cuda:0"), orientation_batch_size=4)
+    n, g = s.total_projections, torch.Generator().manual_seed(n_o)
+    a = torch.randint(-4000, 4000, s.mip.shape, generator=g).double() / 1024
+    sd = torch.zeros_like(a)
+    spread = torch.tensor([1e-25, 1e-20, 1e-15, 1e-9, 1e-3, 1.0, 1e3, 1e15], dtype=torch.float64)
+    a[0, :8], sd[0, :8] = 0.0, spread
+    s.load_maps({"mip": a.float().cuda(), "best_global_index": torch.zeros(a.shape, dtype=torch.int32).cuda(),
+                 "correlation_sum": (a * n).cuda(), "correlation_squared_sum": ((a * a + sd * sd) * n).cuda()})
+    res = s.result()
+    got = res["correlation_variance"].double()
+    assert torch.equal(got[1:], torch.zeros_like(got[1:])) and torch.equal(got[0, 8:], torch.zeros_like(got[0, 8:]))
+    assert torch.equal(res["scaled_mip"], torch.zeros_like(res["scaled_mip"]))
+    assert ((got[0, :8] - spread).abs() <= 1e-6 * spread).all()
+    assert torch.equal(res["correlation_mean"].double(), a)
