@@ -23,16 +23,18 @@ namespace lgb {
 
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// After chain_wait(), for each const __restrict__ input: read-only loads carry no
-// order of their own and could otherwise move above the wait.  (Through the
-// global address, or the compiler would no longer know the address space.)
+// After chain_wait(), for each __restrict__ pointer, read or written: the compiler
+// need not order accesses through one against an asm that has not seen it, and
+// read-only loads carry no order of their own; both could move above the wait.
+// (Through the global address, or the compiler would no longer know the address
+// space.)
 template <class T>
-__device__ __forceinline__ const T* chain_input(const T* p) {
+__device__ __forceinline__ T* chain_pointer(T* p) {
   size_t g = __cvta_generic_to_global(p);
   asm volatile("" : "+l"(g)::"memory");
-  return static_cast<const T*>(__cvta_global_to_generic(g));
+  return static_cast<T*>(__cvta_global_to_generic(g));
 }
-#define LGB_CHAIN_INPUT(p) p = chain_input(p)
+#define LGB_CHAIN_POINTER(p) p = chain_pointer(p)
 
 template <class... P, class... A>
 inline int launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {

@@ -156,8 +156,9 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
     }
   }
   chain_wait();
-  LGB_CHAIN_INPUT(A);
-  LGB_CHAIN_INPUT(Ip);
+  LGB_CHAIN_POINTER(A);
+  LGB_CHAIN_POINTER(Ip);
+  LGB_CHAIN_POINTER(Y);
   if (SPARSE && c_begin < c_end) fetch(c_begin);
   int image = c_begin / c_per_image;
   float2 first[SLOTS];

@@ -96,8 +96,9 @@ __global__ void __launch_bounds__(ColFused<R, P>::THREADS, 1)
   // first-pass sparse form: at most two non-zero inputs per butterfly when h <= 2*NB
   const bool sparse = h <= 2 * NB;
   chain_wait();
-  LGB_CHAIN_INPUT(A);
-  LGB_CHAIN_INPUT(Ip);
+  LGB_CHAIN_POINTER(A);
+  LGB_CHAIN_POINTER(Ip);
+  LGB_CHAIN_POINTER(Y);
   __syncthreads();
 
   const int fj = IdxPad16::f(j);
@@ -212,8 +213,9 @@ __global__ void __launch_bounds__(ColTab<HN>::G* ColTab<HN>::NT)
   const int g = threadIdx.x / NT, t = threadIdx.x - (threadIdx.x / NT) * NT;
   float2* x = ctsm + g * STRIDE;
   chain_wait();
-  LGB_CHAIN_INPUT(A);
-  LGB_CHAIN_INPUT(Ip);
+  LGB_CHAIN_POINTER(A);
+  LGB_CHAIN_POINTER(Ip);
+  LGB_CHAIN_POINTER(Y);
   __syncthreads();
 #pragma unroll 1
   for (int c = c_begin; c < c_end; ++c) {
@@ -313,9 +315,10 @@ __global__ void __launch_bounds__(ColPair<R1, R2>::THREADS, 4)
     }
   }
   chain_wait();
-  LGB_CHAIN_INPUT(A);
-  LGB_CHAIN_INPUT(Ip);
-  LGB_CHAIN_INPUT(norm);
+  LGB_CHAIN_POINTER(A);
+  LGB_CHAIN_POINTER(Ip);
+  LGB_CHAIN_POINTER(Y);
+  LGB_CHAIN_POINTER(norm);
   __syncthreads();
 #pragma unroll 1
   for (int c = c_begin; c < c_end; ++c) {

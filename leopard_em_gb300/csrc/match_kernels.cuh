@@ -71,8 +71,9 @@ __global__ void __launch_bounds__(COLS* FftThreads<HT>::value)
   constexpr int STRIDE = IdxPad16::pad(HT) + 2;
   __shared__ float2 buf[COLS * STRIDE];
   chain_wait();
-  LGB_CHAIN_INPUT(slices);
-  LGB_CHAIN_INPUT(pf);
+  LGB_CHAIN_POINTER(slices);
+  LGB_CHAIN_POINTER(pf);
+  LGB_CHAIN_POINTER(T);
   // c = (p*n_cd + cd)*nb + b: slices are per (p, b), filters per (p, cd)
   const int c = blockIdx.y;
   const int pc = c / nb, b = c - (c / nb) * nb;
@@ -132,8 +133,9 @@ __global__ void __launch_bounds__(ProjColPair<R1, R2A, R2B>::G* ProjColPair<R1, 
     root[m] = make_float2(cs, sn);
   }
   chain_wait();
-  LGB_CHAIN_INPUT(slices);
-  LGB_CHAIN_INPUT(pf);
+  LGB_CHAIN_POINTER(slices);
+  LGB_CHAIN_POINTER(pf);
+  LGB_CHAIN_POINTER(T);
   // c = (p*n_cd + cd)*nb + b: slices are per (p, b), filters per (p, cd)
   const int c = blockIdx.y;
   const int pc = c / nb, b = c - (c / nb) * nb;
@@ -194,7 +196,9 @@ __global__ void __launch_bounds__(ROWS* FftThreads<HT / 2>::value)
   __shared__ float2 z[ROWS][ZS];
   __shared__ float part[ROWS * NT][3];
   chain_wait();
-  LGB_CHAIN_INPUT(T);
+  LGB_CHAIN_POINTER(T);
+  LGB_CHAIN_POINTER(proj);
+  LGB_CHAIN_POINTER(rowstats);
   const int c = blockIdx.y;
   const int g = threadIdx.x / NT, t = threadIdx.x - (threadIdx.x / NT) * NT;
   const int row0 = blockIdx.x * ROWS;
@@ -293,7 +297,9 @@ __global__ void __launch_bounds__(ROWS* R1)
     root[m] = make_float2(cs, sn);
   }
   chain_wait();
-  LGB_CHAIN_INPUT(T);
+  LGB_CHAIN_POINTER(T);
+  LGB_CHAIN_POINTER(proj);
+  LGB_CHAIN_POINTER(rowstats);
   const int c = blockIdx.y;
   const int g = threadIdx.x / NT, t = threadIdx.x - (threadIdx.x / NT) * NT;
   const int row0 = blockIdx.x * ROWS;
@@ -430,7 +436,9 @@ __global__ void __launch_bounds__(ROWS * 16, 7)
   }
   const float2 prej = pre[lane % C2], postj = post[lane % R2];
   chain_wait();
-  LGB_CHAIN_INPUT(T);
+  LGB_CHAIN_POINTER(T);
+  LGB_CHAIN_POINTER(rowstats);
+  LGB_CHAIN_POINTER(A);
   // ---- c2r pass 1 (radix 16) over k = tt + 8q of a group's rows: warps 2 and 3, four rows each
   auto start = [&](int grp) {
     const int tt = lane % C2;
@@ -617,8 +625,9 @@ __global__ void __launch_bounds__(ROWS* FftThreads<WH>::value)
   }
   const int c = blockIdx.y;
   chain_wait();
-  LGB_CHAIN_INPUT(proj);
-  LGB_CHAIN_INPUT(rowstats);
+  LGB_CHAIN_POINTER(proj);
+  LGB_CHAIN_POINTER(rowstats);
+  LGB_CHAIN_POINTER(A);
   // norm_ready: constants (e, s) precomputed by norm_constants_kernel as a
   // float2 over rowstats[c][0][0]; otherwise warp 0 reduces the row moments here
   __shared__ float norm[2];
@@ -715,7 +724,12 @@ __global__ void __launch_bounds__(NT, 2)
     pre[k] = make_float2(cs, sn);
   }
   chain_wait();
-  LGB_CHAIN_INPUT(Y);
+  LGB_CHAIN_POINTER(Y);
+  LGB_CHAIN_POINTER(o0_dev);
+  LGB_CHAIN_POINTER(mip);
+  LGB_CHAIN_POINTER(best);
+  LGB_CHAIN_POINTER(s1);
+  LGB_CHAIN_POINTER(s2);
   float bmax[2 * PIX], bs[2 * PIX], bss[2 * PIX];
   int barg[2 * PIX];
 #pragma unroll

@@ -54,8 +54,9 @@ __global__ void __launch_bounds__(C::THREADS)
     post[p] = make_float2(cs, -sn);
   }
   chain_wait();
-  LGB_CHAIN_INPUT(proj);
-  LGB_CHAIN_INPUT(rowstats);
+  LGB_CHAIN_POINTER(proj);
+  LGB_CHAIN_POINTER(rowstats);
+  LGB_CHAIN_POINTER(A);
   const int c = blockIdx.y;
   // the constants (e, s): precomputed over rowstats[c][0][0], or reduced here by warp 0
   if (norm_ready) {

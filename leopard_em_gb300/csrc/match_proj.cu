@@ -21,9 +21,11 @@ __global__ void __launch_bounds__(256)
                  const int* __restrict__ o0_dev, const float* __restrict__ rotations, int tiles,
                  float2* __restrict__ slices) {
   chain_wait();
-  LGB_CHAIN_INPUT(vol);
-  LGB_CHAIN_INPUT(euler);
-  LGB_CHAIN_INPUT(rotations);
+  LGB_CHAIN_POINTER(vol);
+  LGB_CHAIN_POINTER(euler);
+  LGB_CHAIN_POINTER(o0_dev);
+  LGB_CHAIN_POINTER(rotations);
+  LGB_CHAIN_POINTER(slices);
   const int b = blockIdx.y;
   __shared__ float R[9];
   __shared__ SinCos angle[3];

@@ -41,7 +41,9 @@ __global__ void __launch_bounds__(32)
     norm_constants_kernel(double* __restrict__ rowstats, NormSizes sizes, const float2* __restrict__ dc, size_t dc_stride,
                           float scale, float* __restrict__ offset) {
   chain_wait();
-  LGB_CHAIN_INPUT(dc);
+  LGB_CHAIN_POINTER(rowstats);
+  LGB_CHAIN_POINTER(dc);
+  LGB_CHAIN_POINTER(offset);
   const int c = blockIdx.x, h = sizes.h;
   double* rs = rowstats + (size_t)c * h * 3;
   float e = 0.f, s = 0.f;

@@ -88,7 +88,12 @@ __global__ void __launch_bounds__(C::THREADS, C::MINB)
   }
   const float2* tab_last = tab + TableSize<1, typename DropLast<RL>::type>::value;
   chain_wait();
-  LGB_CHAIN_INPUT(Y);
+  LGB_CHAIN_POINTER(Y);
+  LGB_CHAIN_POINTER(o0_dev);
+  LGB_CHAIN_POINTER(mip);
+  LGB_CHAIN_POINTER(best);
+  LGB_CHAIN_POINTER(s1);
+  LGB_CHAIN_POINTER(s2);
   stage(blockIdx.x * ROWS + g, c0);
   if (o0_dev) o0 += *o0_dev;
 #pragma unroll 1

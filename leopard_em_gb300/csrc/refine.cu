@@ -31,8 +31,9 @@ __global__ void __launch_bounds__(6 * kRotations)
                             int n_particles, float* __restrict__ rot) {
   __shared__ SinCos angle[kRotations][6];
   chain_wait();
-  LGB_CHAIN_INPUT(euler);
-  LGB_CHAIN_INPUT(offsets);
+  LGB_CHAIN_POINTER(euler);
+  LGB_CHAIN_POINTER(offsets);
+  LGB_CHAIN_POINTER(rot);
   const int n = n_particles * nb, first = blockIdx.x * kRotations;
   {
     const int item = threadIdx.x / 6, k = threadIdx.x % 6, i = first + item;
@@ -158,9 +159,11 @@ __global__ void __launch_bounds__(ROWS* R1, 3)
     red_cc[0] = 0u;
   }
   chain_wait();
-  LGB_CHAIN_INPUT(Y);
-  LGB_CHAIN_INPUT(corr_mean);
-  LGB_CHAIN_INPUT(corr_std);
+  LGB_CHAIN_POINTER(Y);
+  LGB_CHAIN_POINTER(corr_mean);
+  LGB_CHAIN_POINTER(corr_std);
+  LGB_CHAIN_POINTER(slot_key);
+  LGB_CHAIN_POINTER(slot_cc);
   const int y = blockIdx.x, p = blockIdx.y;
   const int g = threadIdx.x / NT, t = threadIdx.x - (threadIdx.x / NT) * NT;
   unsigned long long best_key = 0ull;
@@ -266,11 +269,12 @@ __global__ void refine_collect_kernel(int P, int crop_w, int n_cd, int D, const 
                                       const float* __restrict__ defocus, const float* __restrict__ pixel,
                                       unsigned* __restrict__ packed) {
   chain_wait();
-  LGB_CHAIN_INPUT(raw);
-  LGB_CHAIN_INPUT(euler);
-  LGB_CHAIN_INPUT(offsets);
-  LGB_CHAIN_INPUT(defocus);
-  LGB_CHAIN_INPUT(pixel);
+  LGB_CHAIN_POINTER(raw);
+  LGB_CHAIN_POINTER(euler);
+  LGB_CHAIN_POINTER(offsets);
+  LGB_CHAIN_POINTER(defocus);
+  LGB_CHAIN_POINTER(pixel);
+  LGB_CHAIN_POINTER(packed);
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= P) return;
   const int flat = (int)raw[2 * (size_t)P + p], o0 = (int)raw[3 * (size_t)P + p];

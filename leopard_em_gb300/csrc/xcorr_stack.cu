@@ -23,8 +23,9 @@ __global__ void __launch_bounds__(NT) rowstore_kernel(const float2* __restrict__
   __shared__ float2 xr[WH + 4];
   __shared__ float2 z[ZS];
   chain_wait();
-  LGB_CHAIN_INPUT(Y);
-  LGB_CHAIN_INPUT(offset);
+  LGB_CHAIN_POINTER(Y);
+  LGB_CHAIN_POINTER(offset);
+  LGB_CHAIN_POINTER(out);
   const int y = blockIdx.x, p = blockIdx.y, t = threadIdx.x;
   const float2* row = Y + ((size_t)p * y_rows + y) * Wcp;
   for (int k = t; k <= WH; k += NT) xr[k] = row[k];
