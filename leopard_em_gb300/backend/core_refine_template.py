@@ -64,6 +64,14 @@ def _search(particle_stack_dft, template_dft, euler_angles, euler_angle_offsets,
         raise ValueError(f"corr_mean / corr_std must be (N, {crop_h}, {crop_w})")
     if tuple(projective_filters.shape) != (N, d, d // 2 + 1):
         raise ValueError("projective_filters must be (N, d, d//2+1)")
+    # the kernels read N and K rows of three and N defoci
+    if euler_angles.shape[-1:] != (3,) or euler_angles.numel() < 3 * N:
+        raise ValueError(f"euler_angles must be (N, 3) for N = {N} particles, got {tuple(euler_angles.shape)}")
+    if euler_angle_offsets.dim() != 2 or euler_angle_offsets.shape[1] != 3:
+        raise ValueError(f"euler_angle_offsets must be (K, 3), got {tuple(euler_angle_offsets.shape)}")
+    for name, t in (("defocus_u", defocus_u), ("defocus_v", defocus_v), ("defocus_angle", defocus_angle)):
+        if t.numel() < N:
+            raise ValueError(f"{name} must hold one value for each of N = {N} particles, got {tuple(t.shape)}")
     prm = _ctf_params(ctf_kwargs)
     per_call = max(1, min(N, max_correlograms_per_call // max(1, C * D * B)))
     L = lib()
@@ -144,6 +152,9 @@ def core_refine_template(
         raise ValueError("anisotropic magnification (mag_matrix) is not supported by leopard_em_gb300")
     if num_cuda_streams > 1:
         warnings.warn("num_cuda_streams is ignored: one fused kernel sequence per particle group", stacklevel=2)
+    if euler_angles.numel() != 3 * particle_stack_dft.shape[0]:  # a pose for each particle to compose with
+        raise ValueError(f"euler_angles must be (N, 3) for N = {particle_stack_dft.shape[0]} particles, got "
+                         f"{tuple(euler_angles.shape)}")
     raw, eul, offs, dfo, pxo = _search(particle_stack_dft, template_dft, euler_angles, euler_angle_offsets,
                                        defocus_offsets, defocus_u, defocus_v, defocus_angle, pixel_size_offsets,
                                        corr_mean, corr_std, ctf_kwargs, projective_filters, device, batch_size)

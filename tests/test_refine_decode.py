@@ -54,3 +54,22 @@ def test_decode_at_the_poles(theta):
     e = rot.combine_euler_angles(f[:, 7:10].double(), f[:, 10:13].double()).float()
     e = torch.where(e < 0, e + torch.tensor([360.0, 180.0, 360.0]), e)
     assert torch.equal(decode_refine_results(words, None, 33, 33)["refined_euler_angles"], e)
+
+
+@pytest.mark.parametrize("change", [{"euler_angles": (3, 3)}, {"euler_angles": (1, 3)}, {"euler_angles": (2, 2)},
+                                    {"euler_angle_offsets": (5, 1)}, {"euler_angle_offsets": (5,)},
+                                    {"defocus_u": (1,)}, {"defocus_angle": (0,)}])
+def test_poses_and_offsets_of_another_shape_are_refused(change):
+    """Before any device work: the decoding no longer runs through torch operations that refuse them."""
+    from leopard_em_gb300.backend import core_refine_template
+
+    shapes = {"euler_angles": (2, 3), "euler_angle_offsets": (5, 3), "defocus_offsets": (1,), "defocus_u": (2,),
+              "defocus_v": (2,), "defocus_angle": (2,), "pixel_size_offsets": (1,), "corr_mean": (2, 17, 17),
+              "corr_std": (2, 17, 17), "projective_filters": (2, 48, 25)}
+    kw = {k: torch.zeros(change.get(k, s)) for k, s in shapes.items()}
+    kw["particle_stack_dft"] = torch.zeros((2, 64, 33), dtype=torch.complex64)
+    kw["template_dft"] = torch.zeros((48, 48, 25), dtype=torch.complex64)
+    ctf = {"voltage": 300.0, "spherical_aberration": 2.7, "amplitude_contrast_ratio": 0.07, "ctf_B_factor": 0.0,
+           "phase_shift": 0.0, "pixel_size": 1.0}
+    with pytest.raises(ValueError, match=next(iter(change))):
+        core_refine_template(**kw, ctf_kwargs=ctf, device=torch.device("cuda:0"))
