@@ -384,13 +384,9 @@ template <int N, int NT, int DIR, class IDX = IdxPlain>
 __device__ __noinline__ void block_fft_outline(float2* x, int t) {
   Passes<N, NT, DIR, IDX, 1, false, typename Plan<N>::type>::run(x, t, N);
 }
+// (pruned: inputs at index >= nz are known to be zero, the first pass skips them)
 template <int N, int NT, int DIR, class IDX = IdxPlain>
 __device__ __noinline__ void block_fft_pruned_outline(float2* x, int t, int nz) {
-  Passes<N, NT, DIR, IDX, 1, true, typename Plan<N>::type>::run(x, t, nz);
-}
-// Same, with inputs at index >= nz known to be zero (first pass skips them).
-template <int N, int NT, int DIR, class IDX = IdxPlain>
-__device__ __forceinline__ void block_fft_pruned(float2* x, int t, int nz) {
   Passes<N, NT, DIR, IDX, 1, true, typename Plan<N>::type>::run(x, t, nz);
 }
 

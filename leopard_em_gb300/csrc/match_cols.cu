@@ -53,18 +53,18 @@ static int colpass_tab_t(const void* A, const void* Ip, int ips, int h, int Wcp,
                         y_rows, static_cast<float2*>(Y));
 }
 
-template <int R, int P>
+template <int R>
 static int colpass_fused_t(const void* A, const void* Ip, int ips, int h, int Wcp, int n_c, int cpi, int y_rows, int waves,
                            void* Y, cudaStream_t s) {
-  using CF = ColFused<R, P>;
-  if (cudaFuncSetAttribute(colpass_fused_kernel<R, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CF::SMEM) !=
+  using CF = ColFused<R>;
+  if (cudaFuncSetAttribute(colpass_fused_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CF::SMEM) !=
       cudaSuccess)
     return LGB_ERR_CUDA;
   int per = 1;
   const int groups = Wcp / kColGroup;
   const int split = colpass_split(groups, n_c, waves, &per);
   dim3 grid(groups, split);
-  return launch_chained(colpass_fused_kernel<R, P>, grid, dim3(CF::THREADS), CF::SMEM, s,
+  return launch_chained(colpass_fused_kernel<R>, grid, dim3(CF::THREADS), CF::SMEM, s,
                         static_cast<const float2*>(A), static_cast<const float2*>(Ip), ips, h, Wcp, n_c, per, cpi,
                         y_rows, static_cast<float2*>(Y));
 }
@@ -91,9 +91,9 @@ int launch_colpass(int H, const void* A, const void* Ip, int ips, int h, int Wcp
   if (norm && (H != 288 || norm_w < 2 || norm_w / 2 + 1 > Wcp || norm_stride < 1)) return LGB_ERR_UNSUPPORTED_SIZE;
   switch (H) {
     case 256:
-      return colpass_fused_t<16, 2>(A, Ip, ips, h, Wcp, n_c, cpi, y_rows, waves, Y, s);
+      return colpass_fused_t<16>(A, Ip, ips, h, Wcp, n_c, cpi, y_rows, waves, Y, s);
     case 64:
-      return colpass_fused_t<8, 2>(A, Ip, ips, h, Wcp, n_c, cpi, y_rows, waves, Y, s);
+      return colpass_fused_t<8>(A, Ip, ips, h, Wcp, n_c, cpi, y_rows, waves, Y, s);
     case 288:
       return colpass_pair_t<16, 18>(A, Ip, ips, h, Wcp, n_c, cpi, y_rows, waves, Y, s, norm, norm_stride, norm_w);
 #define X(n) \

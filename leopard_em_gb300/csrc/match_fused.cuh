@@ -1,6 +1,6 @@
 // Register-fused column passes of the plain FP32 search.
 //
-// colpass_fused_kernel<R, P>  (H = R^P = 64, 256, one butterfly per thread per pass)
+// colpass_fused_kernel<R>  (H = R^2 = 64, 256, one butterfly per thread per pass)
 //   The forward FFT's last Stockham pass leaves element j + q*H/R of the
 //   column in thread j, and the inverse FFT's first pass consumes exactly those
 //   elements in the same thread: forward-last -> cross power -> inverse-first
@@ -51,40 +51,29 @@ __device__ __forceinline__ int opaque(int v) {
 }
 
 // ---------------------------------------------------------------------------
-// Fused column pass for H = R^P.
+// Fused column pass for H = R^2.
 // ---------------------------------------------------------------------------
-template <int R, int P>
-struct UniformPlan;
 template <int R>
-struct UniformPlan<R, 2> {
-  using type = Radices<R, R>;
-  static constexpr int N = R * R;
-};
-template <int R, int P>
 struct ColFused {
-  using RL = typename UniformPlan<R, P>::type;
-  static constexpr int N = UniformPlan<R, P>::N;
-  static constexpr int NB = N / R;                    // butterflies per pass = threads per column
+  using RL = Radices<R, R>;
+  static constexpr int N = R * R;
+  static constexpr int NB = R;                        // butterflies per pass = threads per column
   static constexpr int THREADS = kColGroup * NB;
   static constexpr int STRIDE = IdxPad16::pad(N) + 4; // column stride in shared memory (float2)
-  static constexpr int TAB = TableSize<1, RL>::value; // twiddle entries of passes 2..P
+  static constexpr int TAB = TableSize<1, RL>::value; // twiddle entries of the second pass
   static constexpr size_t SMEM = sizeof(float2) * (size_t)(kColGroup * STRIDE + TAB);
 };
 
-template <int R, int P>
-__global__ void __launch_bounds__(ColFused<R, P>::THREADS, 1)
+template <int R>
+__global__ void __launch_bounds__(ColFused<R>::THREADS, 1)
     colpass_fused_kernel(const float2* __restrict__ A, const float2* __restrict__ Ip, int ips, int h, int Wcp, int n_c,
                          int c_per_block, int c_per_image, int y_rows, float2* __restrict__ Y) {
-  using CF = ColFused<R, P>;
+  using CF = ColFused<R>;
   using RL = typename CF::RL;
   constexpr int N = CF::N, NB = CF::NB, STRIDE = CF::STRIDE;
-  constexpr int NS_LAST = N / R;
   extern __shared__ float2 csm[];
   float2* tab = csm + kColGroup * STRIDE;
   FillTables<N, 1, RL>::run(tab, threadIdx.x, CF::THREADS);
-  // twiddle sub-table of the last pass (stride NS_LAST)
-  const float2* tab_last = tab + TableSize<1, typename DropLast<RL>::type>::value;
-  const float2* tab_mid = tab;  // middle passes start at stride R (first pass has none)
 
   const int lane = threadIdx.x & 31;
   const int g = lane & 3;                             // column within the group
@@ -104,7 +93,7 @@ __global__ void __launch_bounds__(ColFused<R, P>::THREADS, 1)
   const int fj = IdxPad16::f(j);
   const int f1 = padded_first<R>(j);
   // sparse inputs of the first correlogram; later ones are prefetched one
-  // correlogram ahead, while the current one runs its middle passes
+  // correlogram ahead, while the current one is transformed
   float2 nx0 = make_float2(0.f, 0.f), nx1 = make_float2(0.f, 0.f);
   if (sparse && c_begin < c_end) {
     const float2* a = A + (size_t)c_begin * h * Wcp + kx;
@@ -140,12 +129,10 @@ __global__ void __launch_bounds__(ColFused<R, P>::THREADS, 1)
 #pragma unroll
     for (int q = 0; q < R; ++q) x[f1 + q] = v[q];
     __syncthreads();
-    // ---- forward middle passes
-    TablePasses<N, NB, -1, IdxPad16, R, typename Middle<RL>::type>::run(x, tab_mid, j);
-    // ---- forward last pass -> registers
+    // ---- forward pass 2 -> registers
 #pragma unroll
     for (int q = 0; q < R; ++q) v[q] = x[padded_at<IdxPad16, NB>(fj, j, q)];
-    twiddle_from_table<R, -1, NS_LAST>(v, tab_last, j);
+    twiddle_from_table<R, -1, R>(v, tab, j);
     Dft<R, -1>::run(v);
     // v[q] = P[row j + q*NB]; cross power with the image spectrum, P[0,0] = 0
     {
@@ -159,15 +146,14 @@ __global__ void __launch_bounds__(ColFused<R, P>::THREADS, 1)
     }
     // ---- inverse pass 1 in registers (stride 1, no twiddles)
     Dft<R, +1>::run(v);
-    __syncthreads();  // everyone has read the forward last pass inputs
+    __syncthreads();  // everyone has read the forward pass 2 inputs
 #pragma unroll
     for (int q = 0; q < R; ++q) x[f1 + q] = v[q];
     __syncthreads();
-    TablePasses<N, NB, +1, IdxPad16, R, typename Middle<RL>::type>::run(x, tab_mid, j);
-    // ---- inverse last pass -> global
+    // ---- inverse pass 2 -> global
 #pragma unroll
     for (int q = 0; q < R; ++q) v[q] = x[padded_at<IdxPad16, NB>(fj, j, q)];
-    twiddle_from_table<R, +1, NS_LAST>(v, tab_last, j);
+    twiddle_from_table<R, +1, R>(v, tab, j);
     Dft<R, +1>::run(v);
     float2* yo = Y + (size_t)c * y_rows * ws + (size_t)j * ws + kx;
 #pragma unroll

@@ -557,7 +557,6 @@ struct NormSizes {
   double mean;       // rel^2 / n, rel = n / (H W)
   double border;     // (H - h) (W - h)
   double root;       // sqrt(H W)
-  NormSizes() = default;
   NormSizes(int h_, int H, int W)
       : h(h_), inv_edge(1.0 / (4.0 * h_ - 4.0)), n((double)h_ * h_), mean(n / ((double)H * W) / ((double)H * W)),
         border((double)(H - h_) * (double)(W - h_)), root(sqrt((double)H * (double)W)) {}
@@ -602,26 +601,24 @@ __device__ inline double projection_norm_constants(const double* rs, const NormS
 // for k = 0..W/2, zeros up to Wcp.  The normalisation is that of a
 // norm_h x norm_w micrograph (W may exceed norm_w when the micrograph was
 // zero padded to a supported FFT length).  Real FFT of length W = 2*WH through a
-// WH-point complex FFT (first pass pruned to the ceil(h/2) non-zero inputs).
+// WH-point complex FFT (first pass pruned to the h/2 non-zero inputs; templates
+// are even).  The short rows: a CTA holds many and fills the shared tables of
+// twiddles and post-twiddles once for them.
 // ---------------------------------------------------------------------------
-// TAB: twiddles and post-twiddles from shared tables filled once per CTA (for
-// small transforms, where a CTA holds many rows to amortise the fill).
-template <int WH, int ROWS, bool TAB>
+template <int WH, int ROWS>
 __global__ void __launch_bounds__(ROWS* FftThreads<WH>::value)
     pad_rfft_kernel(const float* __restrict__ proj, const double* __restrict__ rowstats, int h, NormSizes sizes,
                     int Wcp, int norm_ready, float2* __restrict__ A) {
   constexpr int NT = FftThreads<WH>::value;
   constexpr int ZS = IdxPad16::pad(WH) + 2;
   __shared__ float2 z[ROWS][ZS];
-  __shared__ float2 post[TAB ? WH + 1 : 1];  // exp(-i pi k / WH)
-  __shared__ float2 tab[TAB ? FftTable<WH>::SIZE + 1 : 1];
-  if (TAB) {
-    fill_fft_table<WH>(tab, threadIdx.x, blockDim.x);
-    for (int k = threadIdx.x; k <= WH; k += blockDim.x) {
-      float sn, cs;
-      sincospif((float)k / (float)WH, &sn, &cs);
-      post[k] = make_float2(cs, -sn);
-    }
+  __shared__ float2 post[WH + 1];  // exp(-i pi k / WH)
+  __shared__ float2 tab[FftTable<WH>::SIZE + 1];
+  fill_fft_table<WH>(tab, threadIdx.x, blockDim.x);
+  for (int k = threadIdx.x; k <= WH; k += blockDim.x) {
+    float sn, cs;
+    sincospif((float)k / (float)WH, &sn, &cs);
+    post[k] = make_float2(cs, -sn);
   }
   const int c = blockIdx.y;
   chain_wait();
@@ -645,20 +642,13 @@ __global__ void __launch_bounds__(ROWS* FftThreads<WH>::value)
   const int g = threadIdx.x / NT, t = threadIdx.x - (threadIdx.x / NT) * NT;
   const int y = blockIdx.x * ROWS + g;
   const bool active = y < h;
-  const int nz = (h + 1) / 2;
+  const int nz = h / 2;
   if (active) {
     const float* p = proj + ((size_t)c * h + y) * h;
-    for (int m = t; m < nz; m += NT) {
-      const float a = (p[2 * m] - e) * s;
-      const float b = (2 * m + 1 < h) ? (p[2 * m + 1] - e) * s : 0.f;
-      z[g][IdxPad16::f(m)] = make_float2(a, b);
-    }
+    for (int m = t; m < nz; m += NT) z[g][IdxPad16::f(m)] = make_float2((p[2 * m] - e) * s, (p[2 * m + 1] - e) * s);
   }
   __syncthreads();
-  if (TAB)
-    block_fft_pruned_tab<WH, NT, -1, IdxPad16>(z[g], tab, t, nz);
-  else
-    block_fft_pruned<WH, NT, -1, IdxPad16>(z[g], t, nz);
+  block_fft_pruned_tab<WH, NT, -1, IdxPad16>(z[g], tab, t, nz);
   if (!active) return;
   float2* out = A + ((size_t)c * h + y) * Wcp;
   for (int k = t; k <= WH; k += NT) {
@@ -666,15 +656,7 @@ __global__ void __launch_bounds__(ROWS* FftThreads<WH>::value)
     const float2 Zm = cconj(z[g][IdxPad16::f(k == 0 ? 0 : WH - k)]);
     const float2 xe = cscale(cadd(Zk, Zm), 0.5f);
     const float2 xo = mul_i<-1>(cscale(csub(Zk, Zm), 0.5f));
-    float2 w;
-    if (TAB) {
-      w = post[k];
-    } else {
-      float sn, cs;
-      sincospif((float)k / (float)WH, &sn, &cs);
-      w = make_float2(cs, -sn);
-    }
-    out[k] = cadd(xe, cmul(w, xo));
+    out[k] = cadd(xe, cmul(post[k], xo));
   }
   for (int k = WH + 1 + t; k < Wcp; k += NT) out[k] = make_float2(0.f, 0.f);
 }

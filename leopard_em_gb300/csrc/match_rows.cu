@@ -103,8 +103,7 @@ static int pad_rfft_t(const float* proj, const double* rowstats, int h, int norm
     if (st) return st;
   }
   dim3 grid(ctas, n_c);
-  // shared twiddle tables where a CTA transforms >= 4 rows
-  return launch_chained(pad_rfft_kernel<WH, ROWS, (ROWS >= 4)>, grid, dim3(ROWS * NT), 0, s, proj, rowstats, h,
+  return launch_chained(pad_rfft_kernel<WH, ROWS>, grid, dim3(ROWS * NT), 0, s, proj, rowstats, h,
                         NormSizes(h, norm_h, norm_w), Wcp, ready, static_cast<float2*>(A));
 }
 

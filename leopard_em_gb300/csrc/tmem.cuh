@@ -25,16 +25,6 @@ __device__ __forceinline__ void tmem_barrier() {
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // N complex values, 2 N columns; a load is complete when its statement is.
-__device__ __forceinline__ void tmem_put2(unsigned addr, const float2* v) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "f"(v[0].x), "f"(v[0].y), "f"(v[1].x), "f"(v[1].y)
-               : "memory");
-}
-__device__ __forceinline__ void tmem_get2(unsigned addr, float2* v) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];\n tcgen05.wait::ld.sync.aligned;"
-               : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[1].x), "=f"(v[1].y)
-               : "r"(addr)
-               : "memory");
-}
 __device__ __forceinline__ void tmem_put4(unsigned addr, const float2* v) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(addr), "f"(v[0].x), "f"(v[0].y), "f"(v[1].x), "f"(v[1].y), "f"(v[2].x), "f"(v[2].y), "f"(v[3].x), "f"(v[3].y)
                : "memory");
@@ -76,8 +66,7 @@ __device__ __forceinline__ void tmem_put(unsigned addr, const float2* v) {
 }
 template <int N>
 __device__ __forceinline__ void tmem_get(unsigned addr, float2* v) {
-  static_assert(N == 2 || N == 4 || N == 8 || N == 16, "one access");
-  if constexpr (N == 2) tmem_get2(addr, v);
+  static_assert(N == 4 || N == 8 || N == 16, "one access");
   if constexpr (N == 4) tmem_get4(addr, v);
   if constexpr (N == 8) tmem_get8(addr, v);
   if constexpr (N == 16) tmem_get16(addr, v);
