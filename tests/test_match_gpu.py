@@ -412,3 +412,30 @@ def test_finalize_of_constant_pixels(n_o, n_df):
     assert torch.equal(res["scaled_mip"], torch.zeros_like(res["scaled_mip"]))
     assert ((got[0, :8] - spread).abs() <= 1e-6 * spread).all()
     assert torch.equal(res["correlation_mean"].double(), a)
+
+
+def test_searches_on_two_streams_at_once():
+    """Chained kernels and column passes in tensor memory, interleaved on two
+    streams (column lengths that hold all of an SM's tensor memory and a part
+    of it): the maps of each search alone, bit for bit."""
+    shapes = [(4096, 128, 64), (512, 512, 64), (1024, 96, 48), (576, 288, 96)]
+    kws = [_small_workload(*s, 12, 2, seed=i) for i, s in enumerate(shapes)]
+    dev = torch.device("cuda:0")
+
+    def search(i, graph):
+        return MatchTemplateSearch(**kws[i], device=dev, orientation_batch_size=3, graph_batches=graph)
+
+    alone = [search(i, 0) for i in range(len(shapes))]
+    for s in alone:
+        s.run()
+    both = [search(i, i % 2 * 2) for i in range(len(shapes))]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    for a in range(0, 12, 3):
+        for i, s in enumerate(both):
+            with torch.cuda.stream(streams[i % 2]):
+                s.run(a, a + 3)
+    torch.cuda.synchronize()
+    for x, y in zip(alone, both):
+        for k, v in x.maps().items():
+            assert torch.equal(v, y.maps()[k]), (x.shape, k)

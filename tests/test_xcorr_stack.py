@@ -98,3 +98,20 @@ def test_device_matches_oracle_register_column_lengths(H, W, d, mode):
     got = cross_correlate_particle_stack(ps, vol, rot, pf, mode=mode)
     ref = orr.cross_correlate_particle_stack_cpu(ps, vol, rot, pf, mode=mode)
     _close(got.numpy(), ref.numpy())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("H,d", [(64, 48), (128, 96), (256, 192), (288, 256), (512, 96)])
+def test_particles_at_an_odd_storage_offset(H, d):
+    """The column passes read the caller's rows: a stack that starts 8 bytes off a 16-byte line gives the same bits."""
+    from leopard_em_gb300.backend import cross_correlate_particle_stack
+
+    g = torch.Generator().manual_seed(H)
+    ps = torch.fft.rfft2(torch.randn((3, H, H), generator=g)).cuda()
+    vol = torch.fft.fftshift(torch.fft.rfftn(torch.randn((d, d, d), generator=g)), dim=(0, 1)).cuda()
+    rot = torch.linalg.qr(torch.randn((3, 3, 3), generator=g, dtype=torch.float64))[0].float().cuda()
+    pf = (torch.rand((3, d, d // 2 + 1), generator=g) + 0.5).cuda()
+    buf = torch.empty(ps.numel() + 1, dtype=ps.dtype, device=ps.device)
+    odd = buf[1:].view(ps.shape).copy_(ps)
+    assert odd.data_ptr() % 16 == 8 and odd.is_contiguous()
+    assert torch.equal(cross_correlate_particle_stack(odd, vol, rot, pf), cross_correlate_particle_stack(ps, vol, rot, pf))
