@@ -42,8 +42,21 @@ def _without_lambdas(text):
     return text
 
 
-def test_chained_kernels_are_found():
-    assert len(_chained_kernels()) >= 15
+def test_every_kernel_launched_as_a_link_waits():
+    """A link without the wait would let the one after it run ahead of everything before."""
+    waiting = {name for _, name, _, _ in _chained_kernels()}
+    launched = set()
+    for f in sorted(os.listdir(CSRC)):
+        if f.endswith((".cu", ".cuh")) and f != "chain.cuh":
+            with open(os.path.join(CSRC, f)) as src:
+                text = src.read()
+            for m in re.finditer(r"launch_chained\(\s*(\w+)", text):
+                # a variable holds one of the kernels named where it is set
+                names = {m[1]} if m[1].endswith("_kernel") else set(
+                    re.findall(r"\w+_kernel", re.search(rf"auto\*? {m[1]} = ([^;]*);", text)[1]))
+                assert names
+                launched |= names
+    assert len(launched) >= 15 and launched <= waiting
 
 
 @pytest.mark.parametrize("kernel", _chained_kernels(), ids=lambda k: k[1])
@@ -55,6 +68,7 @@ def test_restrict_pointers_are_passed_on_after_the_wait(kernel):
     names = [re.search(r"(\w+)\s*$", p)[1] for p in params.split(",") if "__restrict__" in p]
     before, after = body.split("chain_wait()", 1)
     before = _without_lambdas(before)
+    assert "return" not in before  # every thread waits
     for n in names:
         assert f"LGB_CHAIN_POINTER({n})" in after, n
         for use in re.finditer(rf"\b{n}\b", before):  # (whether it is null may be asked)

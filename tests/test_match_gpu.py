@@ -439,3 +439,34 @@ def test_searches_on_two_streams_at_once():
     for x, y in zip(alone, both):
         for k, v in x.maps().items():
             assert torch.equal(v, y.maps()[k]), (x.shape, k)
+
+
+@pytest.mark.parametrize("H,W,d", [(512, 512, 64), (64, 128, 32)])
+def test_search_inside_a_callers_capture(H, W, d):
+    """A caller's graph that holds a search: behind a copy, behind work of
+    another stream, and twice in a row."""
+    kw = _small_workload(H, W, d, 8, 2)
+    dev = torch.device("cuda:0")
+    s = MatchTemplateSearch(**kw, device=dev, orientation_batch_size=4)
+    fresh = {k: v.clone() for k, v in s.maps().items()}
+    s.run()
+    want = {k: v.clone() for k, v in s.maps().items()}
+    a, b, c = (torch.randn(1 << 16, device=dev) for _ in range(3))
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        s.load_maps(fresh)
+        s.run(0, 4)
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            c.copy_(a + b)
+        b.copy_(a)
+        torch.cuda.current_stream().wait_stream(side)
+        s.run(4, 8)
+    for _ in range(2):
+        for v in s.maps().values():
+            v.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        for k, v in s.maps().items():
+            assert torch.equal(v, want[k]), k
