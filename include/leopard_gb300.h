@@ -197,7 +197,8 @@ int lgb_match_search_static_scratch(const lgb_match_problem* problem, const void
                                     void* stream);
 
 /* Decode the best index and turn the sums into mean, standard deviation and
- * z-score (FP64 arithmetic, FP32 outputs; all maps device, H x W):
+ * z-score (mean and variance in FP64, std and z from them to 48 bits, FP32
+ * outputs; all maps device, H x W):
  *   corr_mean = S/total, corr_std = sqrt(max(S2/total - mean^2, 0)),
  *   scaled_mip = (mip - mean)/std, or 0 where std == 0.
  * `total_positions` is N*D*C of the whole search. */

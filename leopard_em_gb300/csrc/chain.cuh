@@ -6,10 +6,10 @@
 //
 // What it is for: batches whose kernels take a few microseconds each.  One
 // particle refined: 363 -> 329 us; 24 orientations of 512 x 512: 336 -> 311;
-// 1,908: 4.44 -> 4.29 ms; stacks of 1 to 16 crops: 74 -> 65 us.  Letting the successor in as soon as the last CTA of
-// a grid has started (an explicit trigger) made them slower: its CTAs take
-// slots, shared memory and issue slots that the running ones still use
-// (1,908 orientations of 512 x 512 4.46 -> 5.15 ms).
+// 1,908: 4.44 -> 4.29 ms; stacks of 1 to 16 crops: 74 -> 65 us.  Letting the
+// successor in as soon as the last CTA of a grid has started (an explicit
+// trigger) made them slower: its CTAs take slots, shared memory and issue slots
+// that the running ones still use (1,908 orientations of 512 x 512 4.46 -> 5.15 ms).
 //
 // Order: a grid completes only when all its CTAs have waited, so a finished
 // predecessor means that everything before it is finished too.  chain_wait()

@@ -17,10 +17,11 @@
 //                     (rowpass_half_kernel, short rows rowpass_kernel)
 //                     statistics update (utils.py:191-255): max over the
 //                     batch, strict '>' MIP update, global index, FP64 sums
-// Two-register-pass forms for the refinement crops (288^2, d = 256):
-// proj_col_pair_kernel (256 = 16 x 16) and proj_row_rfft_kernel (row c2r
-// 16 x 8 and the padded rfft 16 x 9 in one kernel; the normalisation moves to
-// the column pass, colpass_pair_kernel in match_fused.cuh).
+// Templates from 64 run their projection passes in two register passes
+// (proj_col_pair_kernel, proj_row_pair_kernel).  Refinement crops (288^2, d = 256)
+// take proj_row_rfft_kernel instead of the row pass and pad_rfft: the row c2r
+// 16 x 8 and the padded rfft 9 x 16 in one kernel; the normalisation moves to
+// the column pass (colpass_pair_kernel in match_fused.cuh).
 #pragma once
 
 #include "chain.cuh"

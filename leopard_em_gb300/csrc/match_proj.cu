@@ -12,9 +12,9 @@ namespace lgb {
 // What bounds it: the sectors that a warp's gathers touch.  A warp samples a
 // patch of 8 columns x 4 rows: whatever the orientation, its points share
 // volume rows, where 32 columns of one row, as before, lie in up to 32 of them.
-// 300 slices of 256: 128 -> 118 us; 32 slices of 64 a batch: 7.0 -> 6.7,
-// 5.0 with a thread for each FP64 sincos.  Loading
-// the 16 B that hold both x neighbours where they are aligned: 130.
+// 300 slices of 256: 128 -> 118 us; 32 slices of 64 a batch: 10.3 -> 6.6,
+// 5.0 with a thread for each FP64 sincos.  Loading the 16 B that hold both x
+// neighbours where they are aligned: 130 us for the 300.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
     slice_kernel(const float2* __restrict__ vol, int d, const float* __restrict__ euler, int o0,

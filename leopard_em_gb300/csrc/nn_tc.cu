@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(256) gcol_kernel(ConvShape c, const float* __r
 // pixels a thread: of their 18 taps 3 (even image row) or 6 (odd row) meet an
 // output pixel, and which ones is known at compile time, where the general form
 // tests and loads nine a pixel.  Their units are neighbours too: 32-byte stores.
-// 256 samples: 134 -> 77 us for the 64 x 64 layer, 43 -> 25 and 12 -> 8 for the next.
+// 256 samples: 134 -> 77 us for the layer of 32 x 32 inputs, 43 -> 25 and 12 -> 8 for the next.
 __global__ void __launch_bounds__(256) gcol_pairs_kernel(ConvShape c, const float* __restrict__ g, int rows_pad,
                                                          int k_pad, uint16_t* __restrict__ out) {
   const int pairs = rows_pad / 2, KC = k_pad / kTcKC, units = k_pad / 8, plane_size = c.Ho * c.Wo;

@@ -7,8 +7,8 @@
 // utils/cross_correlation.py:8-40).  Unlike the search, the DC bin of the
 // projection is not zeroed here; the column pass (shared with the search)
 // zeroes it, and the row kernel adds the DC term back:
-// Re(I[0,0] conj(P[0,0])) / (H W), with P[0,0] = sum over the projection rows
-// of their rfft DC bins.
+// Re(I[0,0] conj(P[0,0])) / (H W), with P[0,0] = s (sum of the projection - e d^2)
+// from the row moments (norm_constants_kernel).
 #include "match_kernels.cuh"
 #include "match_launch.h"
 
